@@ -579,7 +579,7 @@ def main():
             "gpu_launches": launches,
             "stages_ms": {k: v / args.steps for k, v in stage_acc.items()},
             "corr_tile": {"chosen": tile_chosen, "trials": tile_trials},
-            "roofline": {"kernel": "correlator path: stream_tma (values + monitors), monitor_finalize, block, "
+            "roofline": {"kernel": "correlator path: stream_box (values + monitors), monitor_finalize, block, "
                                    "block_finalize, c2_pair x2, c2_tail, c2_finalize",
                          "bound": "hbm", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,

@@ -162,15 +162,16 @@ void legendre_projection(int order, int nopit, int ave, double frametime, double
 }
 
 // Basis values at the correction times t = frametime (f + 1.5) of frames
-// f = 0..num-1 (java:9747: x + 0.5 with 1-based x).
+// f = 0..num-1 (java:9747: x + 0.5 with 1-based x), basis_stride(order) floats
+// per frame.
 void legendre_basis_table(int order, int num, double frametime, double uscale, double uoff,
                           float *table)
 {
-    const int k = order + 1;
+    const int st = basis_stride(order);
     double lb[kMaxPoly + 1];
     for (int f = 0; f < num; f++) {
         legendre_d(frametime * (f + 1.5) * uscale + uoff, order, lb);
-        for (int i = 0; i < k; i++) table[(size_t)f * k + i] = (float)lb[i];
+        for (int i = 0; i < st; i++) table[(size_t)f * st + i] = i <= order ? (float)lb[i] : 0.f;
     }
 }
 
@@ -467,7 +468,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     AL(pl->dev_err, 1);
     if (j.bleach == IMFCS_BLEACH_POLYNOMIAL) {
         AL(pl->proj, (size_t)(j.poly_order + 1) * j.nopit);
-        AL(pl->basis, (size_t)(j.poly_order + 1) * j.num);
+        AL(pl->basis, (size_t)basis_stride(j.poly_order) * j.num);
     }
     if (cfg->gls) {
         AS(pl->bprod, np * (chanum - 1) * (size_t)pl->pnum_max);
@@ -520,7 +521,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     if (e == cudaSuccess && j.bleach == IMFCS_BLEACH_POLYNOMIAL) {
         std::vector<double> proj((size_t)(j.poly_order + 1) * j.nopit);
         legendre_projection(j.poly_order, j.nopit, j.ave, cfg->frametime, proj.data(), pl->uscale, pl->uoff);
-        std::vector<float> table((size_t)(j.poly_order + 1) * j.num);
+        std::vector<float> table((size_t)basis_stride(j.poly_order) * j.num);
         legendre_basis_table(j.poly_order, j.num, cfg->frametime, pl->uscale, pl->uoff, table.data());
         e = cudaMemcpy(pl->proj, proj.data(), proj.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(pl->basis, table.data(), table.size() * sizeof(float), cudaMemcpyHostToDevice);

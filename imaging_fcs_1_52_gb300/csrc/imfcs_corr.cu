@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kCorrThreads) corr_kernel(Job j, const LagInfo
     // basis table of chunk 0
     if (j.bleach == IMFCS_BLEACH_POLYNOMIAL)
         for (int i = tid; i < kChunk * order1; i += kCorrThreads)
-            sh_basis[i] = (i / order1) < j.num ? __ldg(&basis[i]) : 0.f;
+            sh_basis[i] = (i / order1) < j.num ? __ldg(&basis[(size_t)(i / order1) * basis_stride(j.poly_order) + i % order1]) : 0.f;
     __syncthreads();
 
     for (int c = 0; c < nchunks; c++) {
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kCorrThreads) corr_kernel(Job j, const LagInfo
         }
         if (j.bleach == IMFCS_BLEACH_POLYNOMIAL && f0 + kChunk < j.num)
             for (int i = tid; i < kChunk * order1; i += kCorrThreads)
-                sh_basis[i] = (f0 + kChunk + i / order1) < j.num ? __ldg(&basis[(size_t)(f0 + kChunk) * order1 + i]) : 0.f;
+                sh_basis[i] = (f0 + kChunk + i / order1) < j.num ? __ldg(&basis[(size_t)(f0 + kChunk + i / order1) * basis_stride(j.poly_order) + i % order1]) : 0.f;
         __syncthreads();
     }
 

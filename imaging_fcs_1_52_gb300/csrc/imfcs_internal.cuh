@@ -230,6 +230,10 @@ __device__ __forceinline__ float bleach_correct(float v, float f, float f0, floa
 // 1-based frame number x = t + 1 (java:9747).
 __device__ __forceinline__ float frame_time(const Job &j, int t) { return j.frametime * ((float)t + 1.5f); }
 
+// Floats between the frames of the polynomial basis table (order + 1 values,
+// padded with zeros to whole float4s).
+__host__ __device__ __forceinline__ int basis_stride(int order) { return (order + 4) & ~3; }
+
 // Legendre polynomials P_0..P_order at u.
 __device__ __forceinline__ void legendre(float u, int order, float *out)
 {
