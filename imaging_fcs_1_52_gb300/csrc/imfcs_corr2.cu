@@ -574,147 +574,243 @@ __global__ void __launch_bounds__(NT, 512 / NT) c2_tail_kernel(C2Args a, const f
 }
 
 // ---------------------------------------------------------------------------
-// Generic-P level kernel (the plugin's P = 32, java:1022-1024): one (pixel,
-// level k, group of up to 8 delays) per thread over the whole frame range
-// (one segment).  Level 0 has delays 0..P, level k >= 1 delays P/2+1..P
-// (java:7391-7424).  The thread builds its level-k samples from the level-0
-// stream (sums of 2^k samples, pairwise within groups of 8), keeps a ring of
-// its last 2P samples in shared memory and its delays' block sums and block
-// statistics in registers, like the tail kernel.
+// P = 32 (java:1022-1024): level 0 has delays 0..32, every upper level delays
+// 17..32 (java:7391-7424), more than the pair kernels' rings hold.  Pixels go
+// in chunks whose scratch stays bounded; per chunk
+//   cg_levels_kernel    the binned sample streams of levels 1..Q-1 from s0;
+//   cg_blocks_kernel    one (pixel, frame segment, level, up to 17 delays) per
+//                       thread: the blocked products P_z of every block and
+//                       the segment's product totals;
+//   cg_finalize_kernel  per (pixel, lag) the block statistics over all blocks
+//                       in order, the totals, the outputs.
+// Blocks are independent of each other, so the frame segments run in
+// parallel; only the statistics, a few operations per block, follow the order
+// of the blocks.  48x48x20,000: 10.4 ms with one thread per (pixel, level,
+// 8 delays) over the whole recording -- two warps an SM at work, each summing
+// its samples from s0 again -- to 0.56 ms (blocks) + 0.06 (levels) + 0.08
+// (finalise).  A chunk's scratch (level streams and products, some 400 KB a
+// pixel at 50,000 frames) stays below 512 MB, less than the level-0 stream.
 // ---------------------------------------------------------------------------
-template <bool CCF, int P>
-__global__ void __launch_bounds__(64) cg_kernel(C2Args a, const float *inA, const float *inB)
+constexpr int kCgDelays = 17;                 // delays per thread: 0..16 and 17..32
+constexpr int kCgStep = 16;                   // samples per step of a thread
+constexpr size_t kCgChunkBytes = (size_t)512 << 20;   // scratch of a pixel chunk
+
+struct CgArgs {
+    CorrOut o;
+    const float4 *mon;        // [pix][chanum]
+    const int *blk_ind;       // [pix]
+    const LagInfo *li;
+    int npix, p0, np, cs;     // all pixels; the chunk's first pixel, pixels and stride
+    int chanum, p, q, num, nseg, pnum_max;
+    int numbin[kMaxLevels], seg_log[kMaxLevels];
+    const float *s0a, *s0b;   // [frame][npix]
+    float *lva, *lvb;         // levels 1..Q-1 of the chunk: [sample][cs] at lv_off
+    size_t lv_off[kMaxLevels];
+    float *pz;                // [lag][pnum_max][cs] blocked products
+    float2 *tot;              // [segment][lag][cs] product totals
+};
+
+// Level-k samples (k = 1..3 pairwise, java:9467-9476; above, the level-3
+// samples of a sample added in order) of 2^(Q-1) frames per thread.
+template <bool CCF>
+__global__ void __launch_bounds__(128) cg_levels_kernel(CgArgs a)
 {
-    constexpr int NT = 64;
-    constexpr int RS = 2 * P;                       // ring (power of two, > the largest delay)
-    constexpr int G0 = (P + 1 + 7) / 8;             // level-0 groups: delays 0..P
-    constexpr int GK = P / 2 / 8;                   // groups of an upper level
-    __shared__ float ring_sm[(CCF ? 2 : 1) * RS * NT];
-    const int tid = threadIdx.x;
-    const int pix = blockIdx.x * NT + tid;
-    const int gy = blockIdx.y;
-    int k, dlo, nd;
-    if (gy < G0) { k = 0; dlo = 8 * gy; nd = min(8, P + 1 - dlo); }
-    else { k = 1 + (gy - G0) / GK; dlo = P / 2 + 1 + 8 * ((gy - G0) % GK); nd = 8; }
-    if (pix >= a.npix || k >= a.q) return;          // no block-wide synchronisation below
-    float *rb = ring_sm + tid;
-    float *ra = CCF ? ring_sm + RS * NT + tid : rb;
-    if (!CCF) inA = inB;
-    C2Ctx c;
-    c2_ctx(c, a, pix, 0, k);
-    const int nkk = a.numbin[k], nk0 = a.numbin[0];
-    const int m = 1 << k;
-    const int lag0 = k == 0 ? dlo : (P + 1) + (k - 1) * (P / 2) + (dlo - (P / 2 + 1));
-    const int dmax = dlo + nd - 1;
-    const int lk = c.ind - k;
-    const int L = lk > 0 ? (1 << lk) : 1;
-
-    float ma[8], mb[8];
+    const int pc = blockIdx.x * 128 + threadIdx.x;
+    if (pc >= a.np) return;
+    const int span = 1 << max(a.q - 1, 3);
+    const int f0 = blockIdx.y * span;
+    for (int tr = 0; tr < (CCF ? 2 : 1); tr++) {
+        const float *in = (tr ? a.s0b : a.s0a) + a.p0 + pc;
+        float *lv = (tr ? a.lvb : a.lva) + pc;
+        float up[kMaxLevels];                 // running sums of levels 4..Q-1
 #pragma unroll
-    for (int l = 0; l < 8; l++) {
-        const float4 mm = __ldg(&c.mon[lag0 + min(l, nd - 1)]);
-        ma[l] = mm.x;
-        mb[l] = mm.y;
+        for (int k = 4; k < 8; k++) up[k] = 0.f;
+        for (int f = f0; f < f0 + span && f < a.num; f += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = f + i < a.num ? __ldg(&in[(size_t)(f + i) * a.npix]) : 0.f;
+#pragma unroll
+            for (int k = 1; k <= 3; k++) {
+#pragma unroll
+                for (int i = 0; i < (8 >> k); i++) {
+                    v[i] = v[2 * i] + v[2 * i + 1];
+                    const int n = (f >> k) + i;
+                    if (k < a.q && n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = v[i];
+                }
+            }
+#pragma unroll
+            for (int k = 4; k < 8; k++) {
+                if (k >= a.q) break;
+                up[k] += v[0];
+                if (((f + 8) & ((1 << k) - 1)) == 0) {
+                    const int n = f >> k;
+                    if (n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = up[k];
+                    up[k] = 0.f;
+                }
+            }
+        }
     }
-    float acc[8], head[8], thi[8], tlo[8], S1[8], S2[8], rr[8];
-#pragma unroll
-    for (int l = 0; l < 8; l++) acc[l] = head[l] = thi[l] = tlo[l] = S1[l] = S2[l] = rr[l] = 0.f;
-    float b0 = 0.f, b1 = 0.f;
+}
 
-    // samples 0 .. nkk - 1 + dmax (samples from nkk on are zero)
-    const int nend = nkk + dmax;
-#pragma unroll 1
-    for (int n = 0; n < nend; n++) {
-        float vb = 0.f, va = 0.f;
-        if (n < nkk) {
-            for (int q0 = n * m; q0 < n * m + m; q0 += 8) {
-                float wb[8], wa[8];
+// One level's samples of one pixel.
+struct CgStream {
+    const float *p;
+    int n, stride;
+    __device__ __forceinline__ float at(int i) const { return i < n ? __ldg(&p[(size_t)i * stride]) : 0.f; }
+};
+
+// State of one thread: block sums of its delays dlo .. dlo + nd - 1.  What
+// only block ends touch -- the heads and the product totals -- is in shared
+// memory (this thread's column of [field][delay][thread]).
+constexpr int kCgThreads = 64;
+struct CgThread {
+    float acc[kCgDelays];
+    float b0, b1;
+    float *sm;
+    int dlo, nd, lag0, L, pnum, pc;
+    __device__ __forceinline__ float &head(int l) { return sm[l * kCgThreads]; }
+    __device__ __forceinline__ float &thi(int l) { return sm[(kCgDelays + l) * kCgThreads]; }
+    __device__ __forceinline__ float &tlo(int l) { return sm[(2 * kCgDelays + l) * kCgThreads]; }
+    // sums of the d samples after sample y, for every delay d of the thread
+    __device__ __forceinline__ void heads(const CgStream &b, int y, float (&h)[kCgDelays]) const
+    {
+        float v[kCgDelays], s = 0.f;
+        if (dlo) {                        // all loads before their sums: one latency, not one each
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int q = q0 + i;
-                    const bool in = i < m && q < nk0;
-                    wb[i] = in ? __ldg(&inB[(size_t)q * a.npix + pix]) : 0.f;
-                    wa[i] = (CCF && in) ? __ldg(&inA[(size_t)q * a.npix + pix]) : 0.f;
-                }
+            for (int i = 1; i < kCgDelays; i++) v[i] = b.at(y + i);
 #pragma unroll
-                for (int w = 1; w < 8; w *= 2)
-#pragma unroll
-                    for (int i = 0; i < 8; i += 2 * w) {
-                        wb[i] += wb[i + w];
-                        wa[i] += wa[i + w];
-                    }
-                vb += wb[0];
-                va += wa[0];
-            }
+            for (int i = 1; i < kCgDelays; i++) s += v[i];
         }
-        rb[(n & (RS - 1)) * NT] = vb;
-        if (CCF) ra[(n & (RS - 1)) * NT] = va;
-        const int y = n - dmax;
-        if (y < 0) continue;
-        if (y == 0) {
-            // heads of the first block: sums of the delayed samples 0 .. d-1
-            float h = 0.f;
 #pragma unroll
-            for (int l = 0; l < 8; l++) head[l] = 0.f;
-            for (int i = 0; i < dmax; i++) {
-                h += rb[(i & (RS - 1)) * NT];
+        for (int l = 0; l < kCgDelays; l++) v[l] = l < nd && dlo + l > 0 ? b.at(y + dlo + l) : 0.f;
 #pragma unroll
-                for (int l = 0; l < 8; l++)
-                    if (dlo + l == i + 1) head[l] = h;
-            }
+        for (int l = 0; l < kCgDelays; l++) {
+            s += v[l];
+            h[l] = s;
         }
-        const float x0 = ra[(y & (RS - 1)) * NT];
+    }
+    // the block ending at direct sample y
+    __device__ __forceinline__ void block_end(const CgArgs &a, const CgStream &b, const float4 *mon, int y)
+    {
+        float nh[kCgDelays];
+        heads(b, y, nh);
+        const int z = y / L;
+        float2 mw[kCgDelays];
 #pragma unroll
-        for (int l = 0; l < 8; l++) acc[l] = fmaf(x0, rb[((y + dlo + l) & (RS - 1)) * NT], acc[l]);
-        b0 += x0;
-        b1 += rb[(y & (RS - 1)) * NT];
-        if (((y + 1) & (L - 1)) == 0) {
-            // heads of the next block: sums of the delayed samples y+1 .. y+d
-            float nh[8], h = 0.f;
+        for (int l = 0; l < kCgDelays; l++) mw[l] = __ldg((const float2 *)&mon[lag0 + min(l, nd - 1)]);
 #pragma unroll
-            for (int l = 0; l < 8; l++) nh[l] = 0.f;
-            for (int i = 1; i <= dmax; i++) {
-                h += rb[((y + i) & (RS - 1)) * NT];
-#pragma unroll
-                for (int l = 0; l < 8; l++)
-                    if (dlo + l == i) nh[l] = h;
-            }
-            const int z = y / L;
-            const bool stat = z < c.pnum;
-#pragma unroll
-            for (int l = 0; l < 8; l++) {
-                const float D = b1 - head[l] + nh[l];
-                const float Pz = (acc[l] - mb[l] * b0 - ma[l] * D + (float)L * ma[l] * mb[l]) / (float)L;
-                ff t = {thi[l], tlo[l]};
+        for (int l = 0; l < kCgDelays; l++) {
+            if (l < nd) {
+                const float2 mm = mw[l];
+                const float D = b1 - head(l) + nh[l];
+                const float Pz = (acc[l] - mm.y * b0 - mm.x * D + (float)L * mm.x * mm.y) / (float)L;
+                ff t = {thi(l), tlo(l)};
                 ff_add(t, acc[l]);
-                thi[l] = t.hi;
-                tlo[l] = t.lo;
-                if (stat && l < nd) {
-                    if (z == 0) rr[l] = Pz;
-                    const float dv = Pz - rr[l];
-                    S1[l] += dv;
-                    S2[l] = fmaf(dv, dv, S2[l]);
-                    if (c.gls && lag0 + l >= 1)
-                        c.bprod[((size_t)pix * (c.chanum - 1) + (lag0 + l - 1)) * c.pnum_stride + z] = Pz;
-                }
-                head[l] = nh[l];
+                thi(l) = t.hi;
+                tlo(l) = t.lo;
+                if (z < pnum) a.pz[((size_t)(lag0 + l) * a.pnum_max + z) * a.cs + pc] = Pz;
+                head(l) = nh[l];
                 acc[l] = 0.f;
             }
-            b0 = 0.f;
-            b1 = 0.f;
         }
+        b0 = 0.f;
+        b1 = 0.f;
+    }
+};
+
+// Grid (pixel blocks, level items, frame segments).  Item 0, 1: level 0,
+// delays 0..16 and 17..32; item 1 + k: level k.  Sixteen samples at a time
+// with the delayed samples in registers where no block ends inside them
+// (blocks of 16 samples and more); shorter blocks, at the upper levels, take
+// their samples one by one.  Issue-bound: 17 FMAs and 3 loads a sample.
+template <bool CCF>
+__global__ void __launch_bounds__(kCgThreads, 6) cg_blocks_kernel(CgArgs a)
+{
+    __shared__ float sm[3 * kCgDelays * kCgThreads];
+    const int pc = blockIdx.x * kCgThreads + threadIdx.x;
+    const int item = blockIdx.y, seg = blockIdx.z;
+    const int k = item < 2 ? 0 : item - 1;
+    const int s0 = seg << a.seg_log[k];
+    if (pc >= a.np || s0 >= a.num) return;
+    const int pix = a.p0 + pc;
+    const int s1 = min(s0 + (1 << a.seg_log[k]), a.num);
+    const int nk = a.numbin[k];
+    const int ys0 = s0 >> k, ys1 = (s1 >= a.num) ? nk : (s1 >> k);
+    CgStream sb, sa;
+    if (k == 0) {
+        sb = {a.s0b + pix, nk, a.npix};
+        sa = {a.s0a + pix, nk, a.npix};
+    } else {
+        sb = {a.lvb + a.lv_off[k] + pc, nk, a.cs};
+        sa = {a.lva + a.lv_off[k] + pc, nk, a.cs};
+    }
+    const int ind = a.blk_ind[pix];
+    CgThread t;
+    t.sm = sm + threadIdx.x;
+    t.pc = pc;
+    t.dlo = item == 0 ? 0 : a.p / 2 + 1;
+    t.nd = item == 0 ? a.p / 2 + 1 : a.p / 2;
+    t.lag0 = item < 2 ? t.dlo : (a.p + 1) + (k - 1) * (a.p / 2);
+    t.L = ind > k ? 1 << (ind - k) : 1;
+    t.pnum = a.li->pnum_by_ind[ind];
+    t.b0 = t.b1 = 0.f;
+#pragma unroll
+    for (int l = 0; l < kCgDelays; l++) t.acc[l] = t.thi(l) = t.tlo(l) = 0.f;
+    {
+        float h[kCgDelays];
+        t.heads(sb, ys0 - 1, h);
+#pragma unroll
+        for (int l = 0; l < kCgDelays; l++) t.head(l) = h[l];
+    }
+    const float4 *mon = a.mon + (size_t)pix * a.chanum;
+
+    float w[kCgDelays - 1 + kCgStep];      // delayed samples y + dlo ...
+#pragma unroll
+    for (int i = 0; i < kCgDelays - 1; i++) w[i] = sb.at(ys0 + t.dlo + i);
+#pragma unroll 1
+    for (int y = ys0; y < ys1; y += kCgStep) {
+#pragma unroll
+        for (int j = 0; j < kCgStep; j++) w[kCgDelays - 1 + j] = sb.at(y + t.dlo + kCgDelays - 1 + j);
+        if (t.L >= kCgStep && y + kCgStep <= ys1) {
+            float x[kCgStep], v[kCgStep];
+#pragma unroll
+            for (int j = 0; j < kCgStep; j++) {
+                v[j] = sb.at(y + j);
+                x[j] = CCF ? sa.at(y + j) : v[j];
+            }
+#pragma unroll
+            for (int j = 0; j < kCgStep; j++) {
+#pragma unroll
+                for (int l = 0; l < kCgDelays; l++) t.acc[l] = fmaf(x[j], w[j + l], t.acc[l]);
+                t.b0 += x[j];
+                t.b1 += v[j];
+            }
+            if (((y + kCgStep) & (t.L - 1)) == 0) t.block_end(a, sb, mon, y + kCgStep - 1);
+        } else {
+            const int ye = min(y + kCgStep, ys1);
+#pragma unroll 1
+            for (int yy = y; yy < ye; yy++) {
+                float d[kCgDelays];
+                const float x = sa.at(yy), v = sb.at(yy);
+#pragma unroll
+                for (int l = 0; l < kCgDelays; l++) d[l] = sb.at(yy + t.dlo + l);
+#pragma unroll
+                for (int l = 0; l < kCgDelays; l++) t.acc[l] = fmaf(x, d[l], t.acc[l]);
+                t.b0 += x;
+                t.b1 += v;
+                if (((yy + 1) & (t.L - 1)) == 0) t.block_end(a, sb, mon, yy);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kCgDelays - 1; i++) w[i] = w[i + kCgStep];
     }
 #pragma unroll
-    for (int l = 0; l < 8; l++) {
-        if (l >= nd) break;
-        ff t = {thi[l], tlo[l]};
-        ff_add(t, acc[l]);
-        stat_ref(c.stats, c.npix, lag0 + l, 0, pix) = t.hi;
-        stat_ref(c.stats, c.npix, lag0 + l, 1, pix) = t.lo;
-        stat_ref(c.stats, c.npix, lag0 + l, 2, pix) = S1[l];
-        stat_ref(c.stats, c.npix, lag0 + l, 3, pix) = S2[l];
-        stat_ref(c.stats, c.npix, lag0 + l, 4, pix) = rr[l];
-    }
+    for (int l = 0; l < kCgDelays; l++)
+        if (l < t.nd) {
+            ff u = {t.thi(l), t.tlo(l)};
+            ff_add(u, t.acc[l]);                 // the partial block at the end
+            a.tot[((size_t)seg * a.chanum + t.lag0 + l) * a.cs + pc] = make_float2(u.hi, u.lo);
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -722,6 +818,29 @@ __global__ void __launch_bounds__(64) cg_kernel(C2Args a, const float *inA, cons
 // statistics brought to one shift (FP64), outputs as calculateCF
 // (java:9491-9531).
 // ---------------------------------------------------------------------------
+// Outputs of one (pixel, lag) from its product total A and the statistics of
+// its pnum blocked products (sums S1, S2 shifted by r).
+__device__ __forceinline__ void write_lag(const CorrOut &o, const float4 *mon, const LagInfo *li, int chanum, int pix,
+                                          int lag, int pnum, double A, double S1, double S2, double r)
+{
+    const float4 m = mon[(size_t)pix * chanum + lag];
+    const double n = li->prodnum[lag];
+    const double dmDm = (double)m.z * (double)m.w;
+    const double sumprod = A - n * (double)m.x * (double)m.y;
+    const double corav = sumprod / (n * dmDm);
+    const double pn = pnum;
+    const double bv = (S2 / pn - (S1 / pn) * (S1 / pn)) / ((pn - 1) * dmDm * dmDm);
+    double acf = corav;
+    if (o.gls) acf = (lag == 0) ? 0.0 : (S1 + pn * r) / (pn * dmDm);   // mcov (java:9526-9531)
+    if (o.acf) o.acf[(size_t)pix * chanum + lag] = acf;
+    if (o.var) o.var[(size_t)pix * chanum + lag] = bv;
+    if (o.sd) o.sd[(size_t)pix * chanum + lag] = sqrt(bv);
+    if (lag == 1) {
+        if (o.nb_mean) o.nb_mean[pix] = m.z;
+        if (o.nb_cov) o.nb_cov[pix] = sumprod / n;
+    }
+}
+
 __global__ void c2_finalize_kernel(C2Args a)
 {
     // lag-major threads: the segment statistics [lag][stat][pixel] are read
@@ -750,22 +869,40 @@ __global__ void c2_finalize_kernel(C2Args a)
         S1 += s1s + cnt * dr;
         S2 += s2s + 2.0 * dr * s1s + cnt * dr * dr;
     }
-    const float4 m = a.mon[(size_t)pix * a.chanum + lag];
-    const double n = a.li->prodnum[lag];
-    const double dmDm = (double)m.z * (double)m.w;
-    const double sumprod = A - n * (double)m.x * (double)m.y;
-    const double corav = sumprod / (n * dmDm);
-    const double pn = pnum;
-    const double bv = (S2 / pn - (S1 / pn) * (S1 / pn)) / ((pn - 1) * dmDm * dmDm);
-    double acf = corav;
-    if (a.o.gls) acf = (lag == 0) ? 0.0 : (S1 + pn * r) / (pn * dmDm);   // mcov (java:9526-9531)
-    if (a.o.acf) a.o.acf[(size_t)pix * a.chanum + lag] = acf;
-    if (a.o.var) a.o.var[(size_t)pix * a.chanum + lag] = bv;
-    if (a.o.sd) a.o.sd[(size_t)pix * a.chanum + lag] = sqrt(bv);
-    if (lag == 1) {
-        if (a.o.nb_mean) a.o.nb_mean[pix] = m.z;
-        if (a.o.nb_cov) a.o.nb_cov[pix] = sumprod / n;
+    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, pnum, A, S1, S2, r);
+}
+
+// P = 32: the block statistics of one (pixel, lag) over its blocks in order
+// (FP32, shifted by the first block), the segments' totals in FP64.
+__global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
+{
+    const int pc = blockIdx.x * 128 + threadIdx.x, lag = blockIdx.y;
+    if (pc >= a.np) return;
+    const int pix = a.p0 + pc;
+    const int pnum = a.li->pnum_by_ind[a.blk_ind[pix]];
+    const float *pz = a.pz + (size_t)lag * a.pnum_max * a.cs + pc;
+    const float r = pnum > 0 ? pz[0] : 0.f;
+    float S1 = 0.f, S2 = 0.f;
+    for (int z = 0; z < pnum; z += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = z + u < pnum ? pz[(size_t)(z + u) * a.cs] : r;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (z + u < pnum) {
+                const float dv = v[u] - r;
+                S1 += dv;
+                S2 = fmaf(dv, dv, S2);
+            }
     }
+    const int sl = a.seg_log[lag <= a.p ? 0 : 1 + (lag - (a.p + 1)) / (a.p / 2)];
+    const int nseg = (a.num + (1 << sl) - 1) >> sl;
+    double A = 0.0;
+    for (int sg = 0; sg < nseg; sg++) {
+        const float2 t = a.tot[((size_t)sg * a.chanum + lag) * a.cs + pc];
+        A += (double)t.x + (double)t.y;
+    }
+    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, pnum, A, S1, S2, r);
 }
 
 // ---------------------------------------------------------------------------
@@ -774,7 +911,7 @@ __global__ void c2_finalize_kernel(C2Args a)
 // The chain needs blocks of at least 16 level-0 and 8 level-1 samples
 // (ind >= Q-1 >= 4).
 bool corr2_supported(const Job &j) { return j.p == kP && j.q >= 5; }
-// P = 32: the generic level kernel (any Q)
+// P = 32 (any Q)
 bool corrg_supported(const Job &j) { return j.p == 32; }
 
 namespace {
@@ -815,9 +952,40 @@ Plan2 plan2(const Job &j)
 
 int corr2_nseg(const Job &j) { return plan2(j).nseg_max; }
 
+// The P = 32 path's scratch: bytes per pixel, and the pixels of a chunk.
+struct CgPlan {
+    int chunk, nseg, pnum_max, seg_log[kMaxLevels], numbin[kMaxLevels];
+    size_t lv, pz, tot;                   // floats per pixel: level streams, products, totals
+};
+static CgPlan cg_plan(const Job &j)
+{
+    CgPlan p;
+    p.pnum_max = max((j.num - (j.p << (j.q - 1))) >> (j.q - 1), 1);
+    const int base = max(j.blocknum - 1, j.q - 1);     // every pixel's block length divides 2^base frames
+    p.lv = 0;
+    int nb = j.num;
+    p.nseg = 1;
+    for (int k = 0; k < j.q; k++, nb /= 2) {
+        p.numbin[k] = nb;
+        if (k) p.lv += nb;
+        p.seg_log[k] = max(base, k + 4);               // whole steps of 16 samples
+        p.nseg = max(p.nseg, (j.num + (1 << p.seg_log[k]) - 1) >> p.seg_log[k]);
+    }
+    p.lv *= j.is_ccf ? 2 : 1;
+    p.pz = (size_t)j.chanum * p.pnum_max;
+    p.tot = (size_t)2 * j.chanum * p.nseg;
+    size_t c = kCgChunkBytes / ((p.lv + p.pz + p.tot) * sizeof(float));
+    c = c < 64 ? 64 : c & ~(size_t)63;
+    p.chunk = (int)(c < (size_t)j.npix ? c : (size_t)j.npix);
+    return p;
+}
+
 int corr_kernel_count(const Job &j)
 {
-    if (corrg_supported(j)) return 2;
+    if (corrg_supported(j)) {
+        const int c = cg_plan(j).chunk;
+        return 3 * ((j.npix + c - 1) / c);
+    }
     if (!corr2_supported(j)) return 1;
     const Plan2 p = plan2(j);
     return p.npair + (p.k_tail < j.q ? 1 : 0) + 1;   // pair kernels, tail, finalise
@@ -825,6 +993,10 @@ int corr_kernel_count(const Job &j)
 
 size_t corr_stats_floats(const Job &j)
 {
+    if (corrg_supported(j)) {
+        const CgPlan p = cg_plan(j);
+        return (p.pz + p.tot) * p.chunk;
+    }
     const size_t one = (size_t)j.chanum * kStatN * j.npix;
     return corr2_supported(j) ? one * corr2_nseg(j) : one;
 }
@@ -833,6 +1005,10 @@ size_t corr_stats_floats(const Job &j)
 // npix), written by the pair kernels for the next level pair.
 size_t corr_stream_floats(const Job &j)
 {
+    if (corrg_supported(j)) {
+        const CgPlan p = cg_plan(j);
+        return p.lv * p.chunk;
+    }
     if (!corr2_supported(j)) return 1;
     const size_t tr = j.is_ccf ? 2 : 1;
     return tr * (size_t)j.npix * ((size_t)(j.num >> 2) + (size_t)(j.num >> 4) + 3);
@@ -858,39 +1034,57 @@ static void launch_pair(bool ccf, int variant, dim3 grid, cudaStream_t stream, c
     }
 }
 
-// The generic-P correlator: level kernel over the whole frame range, then
-// the finalise kernel (one segment).
-
+// The P = 32 correlator, one pixel chunk after the other.
 cudaError_t launch_corrg(const Job &j, const LagInfo *li, const float *s0, const float4 *mon, const int *blk_ind,
-                         const CorrOut &o, cudaStream_t stream)
+                         const CorrOut &o, float *streams, cudaStream_t stream)
 {
-    C2Args a;
+    const CgPlan p = cg_plan(j);
+    CgArgs a;
     memset(&a, 0, sizeof(a));
     a.o = o;
     a.mon = mon;
     a.blk_ind = blk_ind;
     a.li = li;
     a.npix = j.npix;
+    a.cs = p.chunk;
     a.chanum = j.chanum;
     a.p = j.p;
     a.q = j.q;
     a.num = j.num;
-    {
-        int nb = j.num;
-        for (int k = 0; k < j.q; k++) { a.numbin[k] = nb; nb /= 2; }
+    a.nseg = p.nseg;
+    a.pnum_max = p.pnum_max;
+    size_t off = 0;
+    for (int k = 0; k < j.q; k++) {
+        a.numbin[k] = p.numbin[k];
+        a.seg_log[k] = p.seg_log[k];
+        if (k) {
+            a.lv_off[k] = off;
+            off += (size_t)p.numbin[k] * p.chunk;
+        }
     }
-    for (int k = 0; k < kMaxLevels; k++) a.seg_log[k] = 30;   // one segment
-    a.stat_stride = (size_t)j.chanum * kStatN * j.npix;
-    const float *s0a = s0, *s0b = j.is_ccf ? s0 + (size_t)j.npix * j.num : s0;
-    constexpr int P = 32;
-    const dim3 grid((j.npix + 63) / 64, (P + 1 + 7) / 8 + (j.q - 1) * (P / 16));
-    if (j.is_ccf) cg_kernel<true, P><<<grid, 64, 0, stream>>>(a, s0a, s0b);
-    else cg_kernel<false, P><<<grid, 64, 0, stream>>>(a, s0a, s0b);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const int n = j.npix * j.chanum;
-    c2_finalize_kernel<<<(n + 255) / 256, 256, 0, stream>>>(a);
-    return cudaGetLastError();
+    a.s0a = s0;
+    a.s0b = j.is_ccf ? s0 + (size_t)j.npix * j.num : s0;
+    a.lva = streams;
+    a.lvb = j.is_ccf ? streams + off : streams;
+    a.tot = (float2 *)o.stats;
+    a.pz = o.stats + p.tot * p.chunk;
+    const int span = 1 << max(j.q - 1, 3);
+    for (a.p0 = 0; a.p0 < j.npix; a.p0 += p.chunk) {
+        a.np = min(p.chunk, j.npix - a.p0);
+        const dim3 gl((a.np + 127) / 128, (j.num + span - 1) / span);
+        const dim3 gb((a.np + kCgThreads - 1) / kCgThreads, j.q + 1, p.nseg);
+        if (j.is_ccf) {
+            cg_levels_kernel<true><<<gl, 128, 0, stream>>>(a);
+            cg_blocks_kernel<true><<<gb, kCgThreads, 0, stream>>>(a);
+        } else {
+            cg_levels_kernel<false><<<gl, 128, 0, stream>>>(a);
+            cg_blocks_kernel<false><<<gb, kCgThreads, 0, stream>>>(a);
+        }
+        cg_finalize_kernel<<<dim3((a.np + 127) / 128, j.chanum), 128, 0, stream>>>(a);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_corr2(const Job &j, const LagInfo *li, const float *s0, const float4 *mon, const int *blk_ind,
