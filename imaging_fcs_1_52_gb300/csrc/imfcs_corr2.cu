@@ -35,7 +35,6 @@ namespace imfcs {
 
 constexpr int kC2Threads = 64;       // pixels per CTA unless the tile says 32
 constexpr int kMaxSegExtra = 4;
-constexpr int kHeadFields = (kP + 1) + 8;                   // first-level heads d = 0..16, second-level d = 9..16
 
 // Arguments shared by the pair, tail and finalise kernels.
 struct C2Args {
@@ -49,511 +48,382 @@ struct C2Args {
     size_t stat_stride;       // floats per segment in o.stats
 };
 
-// Per-thread context.
-struct C2Ctx {
-    float *stats;             // this segment's statistics
-    const float4 *mon;        // this pixel's monitors
-    float *bprod;
-    int npix, pix, chanum, pnum_stride, gls;
-    int ind, pnum, zfirst;
-    bool valid;               // false: a lane without a pixel (computes, writes nothing)
-    // where the block statistics of this (pixel, segment) live: the global
-    // array (stride npix) or a shared-memory copy (stride = threads) that the
-    // caller writes back; and (optional) the lags' monitors (a, b) in shared
-    // memory with stride smon_stride, both from lag lag0 on
-    float *sst;
-    int sst_stride;
-    const float2 *smon;
-    int smon_stride;
-    int lag0;
-    __device__ __forceinline__ float &stat(int lag, int s) const
-    {
-        return sst[(size_t)((lag - lag0) * kStatN + s) * sst_stride];
-    }
-    __device__ __forceinline__ float2 monitor(int lag) const
-    {
-        if (smon) return smon[(lag - lag0) * smon_stride];
-        const float4 m = __ldg(&mon[lag]);
-        return make_float2(m.x, m.y);
-    }
-};
-
-// One block end of one lag: total, blocked product and its statistics.
-__device__ __forceinline__ void c2_block_stat(const C2Ctx &c, int lag, float A, float B0, float D, int L, int z)
+// The blocked product of one block of one lag, (A - b B - a D + L a b) / L,
+// with L a power of two (iL = 1/L and L a are exact).
+__device__ __forceinline__ float block_product(float A, float B, float D, float a, float b, float L, float iL)
 {
-    if (!c.valid) return;
-    const float2 m = c.monitor(lag);
-    const float a = m.x, b = m.y;
-    const float P = (A - b * B0 - a * D + (float)L * a * b) / (float)L;
-    float &ahi = c.stat(lag, 0);
-    float &alo = c.stat(lag, 1);
-    ff t = {ahi, alo};
-    ff_add(t, A);
-    ahi = t.hi;
-    alo = t.lo;
-    if (z < c.pnum) {
-        float &r = c.stat(lag, 4);
-        if (z == c.zfirst) r = P;      // per-segment shift of the block statistics
-        const float dv = P - r;
-        c.stat(lag, 2) += dv;
-        c.stat(lag, 3) += dv * dv;
-        if (c.gls && lag >= 1) c.bprod[((size_t)c.pix * (c.chanum - 1) + (lag - 1)) * c.pnum_stride + z] = P;
-    }
-}
-
-__device__ __forceinline__ void c2_add_total(const C2Ctx &c, int lag, float A)
-{
-    if (!c.valid) return;
-    float &ahi = c.stat(lag, 0);
-    float &alo = c.stat(lag, 1);
-    ff t = {ahi, alo};
-    ff_add(t, A);
-    ahi = t.hi;
-    alo = t.lo;
-}
-
-__device__ __forceinline__ void c2_ctx(C2Ctx &c, const C2Args &a, int pix, int seg, int k)
-{
-    c.valid = pix < a.npix;
-    if (!c.valid) pix = a.npix - 1;   // reads stay in bounds; writes are masked
-    c.stats = a.o.stats + (size_t)seg * a.stat_stride;
-    c.mon = a.mon + (size_t)pix * a.chanum;
-    c.bprod = a.o.bprod;
-    c.npix = a.npix;
-    c.pix = pix;
-    c.chanum = a.chanum;
-    c.pnum_stride = a.o.pnum_stride;
-    c.gls = a.o.gls;
-    c.ind = a.blk_ind[pix];
-    c.pnum = a.li->pnum_by_ind[c.ind];
-    c.zfirst = (seg << a.seg_log[k]) >> c.ind;
-    c.sst = c.stats + pix;
-    c.sst_stride = a.npix;
-    c.smon = nullptr;
-    c.smon_stride = 0;
-    c.lag0 = 0;
+    return fmaf(L * a, b, fmaf(-a, D, fmaf(-b, B, A))) * iL;
 }
 
 // ---------------------------------------------------------------------------
 // Pair kernel: levels k (first) and k+1 (second) of one (pixel, segment).
 // FIRST17: the first level is level 0 (lags 0..16); otherwise its lags are
 // delays 9..16.  TWO: the second level exists (k+1 < Q).
+//
+// A step takes the 16 first-level direct samples from y0 on with the 32
+// samples from y0 on in registers (the next 16 already loading), and the
+// eight second-level direct samples of the step before, whose delayed samples
+// are then complete.  Both windows move by register copies, so one step's
+// code, 336 FMAs for levels 0-1, serves every step and block ends are in it
+// once.  What only block ends touch -- totals, statistics, heads -- is in
+// shared memory, the monitors and the statistics' shift in the L1.
 // ---------------------------------------------------------------------------
-template <bool FIRST17>
-struct PairReg {
-    static constexpr int NF = FIRST17 ? kP + 1 : 8;   // first-level lags
-    static constexpr int DF = FIRST17 ? 0 : 9;        // first-level delay of lag 0
-    float wB[32], wA[32];      // first-level rings (delayed / direct trace), index n & 31
-    float rB[32], rA[32];      // second-level rings, index n & 31
-    float accF[NF], accS[8];
-    float bF0, bF1, bS0, bS1;
-    float curB[16], curA[16];  // samples n .. n+15 in flight (slot n & 15)
-};
+constexpr int kPairFields = 5;    // per lag in shared memory: Ahi, Alo, S1, S2, head
 
-struct PairGeo {
-    const float *inA, *inB;    // level-k samples [n][npix]
-    float *outA, *outB;        // level-(k+2) samples [n][npix] or nullptr
-    int k, nk, nk1, nk2;       // level and sample counts of levels k, k+1, k+2
-    int sk0, sk1;              // direct samples [sk0, sk1) of level k
-    int LF, LS;                // block lengths (samples) of levels k and k+1
-    int lagF, lagS;            // first lag index of the two levels
-};
+// Fields of one thread: lag l of the pass, field f at sm[(l * kPairFields + f) * NT].
+template <int NT>
+struct PairBlocks {
+    float *sm;
+    const float4 *mon;        // this pixel's monitors from the pass's first lag on
+    float *rst;               // this (segment, pixel)'s shift of the first lag's statistics
+    float *bprod;             // this pixel's products of the first lag, or nullptr
+    int npix, pnum_stride, pnum, zfirst;
+    bool skip0;               // the pass's first lag is lag 0 (no product kept)
+    __device__ __forceinline__ float &at(int l, int f) { return sm[(l * kPairFields + f) * NT]; }
 
-__device__ __forceinline__ float c2_load(const float *in, int n, int nk, int npix, int pix)
-{
-    return n < nk ? __ldg(&in[(size_t)n * npix + pix]) : 0.f;
-}
-
-// Sample source of a pair kernel: level-k samples of the direct (a) and
-// delayed (b) traces from the materialised FP32 streams.  prep(g) precedes
-// the reads of group g's 16 samples (in order, jj = 0..15); acquire/release
-// bracket the groups (hooks for a source that stages its data).
-struct GlobalSrc {
-    const float *inA, *inB;
-    int nk, npix, pix;
-    __device__ __forceinline__ void prep(int) {}
-    __device__ __forceinline__ float a(int n, int) { return c2_load(inA, n, nk, npix, pix); }
-    __device__ __forceinline__ float b(int n, int) { return c2_load(inB, n, nk, npix, pix); }
-    __device__ __forceinline__ bool acquire(int) { return true; }
-    __device__ __forceinline__ void release(int) {}
-};
-
-template <bool CCF, bool FIRST17, bool TWO, int QP, class Src>
-__device__ __forceinline__ void c2_pair_group(const C2Ctx &c, const PairGeo &p, float *heads, int nt,
-                                              PairReg<FIRST17> &R, int g, Src &src)
-{
-    constexpr int NF = PairReg<FIRST17>::NF, DF = PairReg<FIRST17>::DF;
-    constexpr int PH0 = 16 * (QP & 1);
-    constexpr int PH1 = 8 * QP;
-    const int n0 = 16 * g;
-    const bool dirF = (n0 - 16 >= p.sk0) && (n0 - 16 < p.sk1);          // direct samples n0-16 .. n0-1
-    const bool dirS = TWO && (n0 - 32 >= p.sk0) && (n0 - 32 < p.sk1);   // second-level 8g-16 .. 8g-9
-    src.prep(g + 1);
+    // The block z of N lags from lag l0 of the pass on: acc the products' sums
+    // (cleared), B and Bd the sums of the direct and undelayed samples, nh the
+    // sums of the first d samples of the next block per lag.
+    template <int N>
+    __device__ __forceinline__ void end(int l0, float (&acc)[N], float B, float Bd, const float (&nh)[N], int L, int z)
+    {
+        const float fL = (float)L, iL = 1.f / fL;
+        const bool stat = z < pnum, first = z == zfirst;
+        constexpr int kBatch = 6;          // lags whose monitors and shifts load together
 #pragma unroll
-    for (int jj = 0; jj < 16; jj++) {
-        const int n = n0 + jj;
-        const float vB = R.curB[jj];
-        R.wB[(PH0 + jj) & 31] = vB;
-        if (CCF) {
-            R.wA[(PH0 + jj) & 31] = R.curA[jj];
-            R.curA[jj] = src.a(n + 16, jj);
-        }
-        R.curB[jj] = src.b(n + 16, jj);
-        if (dirF) {
-            // direct sample y = n - 16 with delayed samples y + DF .. y + 16 = n
-            const float x0 = CCF ? R.wA[(PH0 + 16 + jj) & 31] : R.wB[(PH0 + 16 + jj) & 31];
+        for (int lb = 0; lb < N; lb += kBatch) {
+            float2 m[kBatch];
+            float r[kBatch];
 #pragma unroll
-            for (int d = 0; d < NF; d++) R.accF[d] = fmaf(x0, R.wB[(PH0 + 16 + jj + DF + d) & 31], R.accF[d]);
-            R.bF0 += x0;
-            R.bF1 += R.wB[(PH0 + 16 + jj) & 31];
-        }
-        if (TWO && (jj & 1)) {
-            // second-level sample m = 8g + jj/2 from first-level samples n-1, n
-            const int i1 = jj >> 1;
-            const int m = 8 * g + i1;
-            const bool ok = m < p.nk1;
-            const float sB = ok ? R.wB[(PH0 + jj - 1) & 31] + R.wB[(PH0 + jj) & 31] : 0.f;
-            R.rB[(PH1 + i1) & 31] = sB;
-            if (CCF) R.rA[(PH1 + i1) & 31] = ok ? R.wA[(PH0 + jj - 1) & 31] + R.wA[(PH0 + jj) & 31] : 0.f;
-            if (dirS) {
-                // direct sample y1 = m - 16, delayed samples y1 + 9 .. y1 + 16 = m
-                const float x1 = CCF ? R.rA[(PH1 + i1 + 16) & 31] : R.rB[(PH1 + i1 + 16) & 31];
+            for (int u = 0; u < kBatch; u++) {
+                if (lb + u >= N) break;
+                m[u] = __ldg((const float2 *)&mon[l0 + lb + u]);
+                r[u] = stat && !first ? rst[(size_t)(l0 + lb + u) * kStatN * npix] : 0.f;
+            }
 #pragma unroll
-                for (int l = 0; l < 8; l++) R.accS[l] = fmaf(x1, R.rB[(PH1 + i1 + 16 + 9 + l) & 31], R.accS[l]);
-                R.bS0 += x1;
-                R.bS1 += R.rB[(PH1 + i1 + 16) & 31];
+            for (int u = 0; u < kBatch; u++) {
+                if (lb + u >= N) break;
+                const int l = lb + u, s = l0 + l;
+                const float P = block_product(acc[l], B, Bd - at(s, 4) + nh[l], m[u].x, m[u].y, fL, iL);
+                ff t = {at(s, 0), at(s, 1)};
+                ff_add(t, acc[l]);
+                at(s, 0) = t.hi;
+                at(s, 1) = t.lo;
+                at(s, 4) = nh[l];
+                acc[l] = 0.f;
+                if (stat) {
+                    if (first) {                    // the segment's shift of the block statistics
+                        rst[(size_t)s * kStatN * npix] = P;
+                    } else {
+                        const float dv = P - r[u];
+                        at(s, 2) += dv;
+                        at(s, 3) = fmaf(dv, dv, at(s, 3));
+                    }
+                    if (bprod && !(skip0 && s == 0)) bprod[(size_t)s * pnum_stride + z] = P;
+                }
             }
         }
     }
-    // level-(k+2) samples 4g .. 4g+3 from second-level samples 8g .. 8g+7
-    if (TWO && p.outB && c.valid) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int m2 = 4 * g + i;
-            if (m2 >= (p.sk0 >> 2) && m2 < (p.sk1 >> 2) && m2 < p.nk2) {
-                p.outB[(size_t)m2 * c.npix + c.pix] = R.rB[(PH1 + 2 * i) & 31] + R.rB[(PH1 + 2 * i + 1) & 31];
-                if (CCF)
-                    p.outA[(size_t)m2 * c.npix + c.pix] = R.rA[(PH1 + 2 * i) & 31] + R.rA[(PH1 + 2 * i + 1) & 31];
-            }
-        }
-    }
-    // heads of the segment's first blocks (its first 16 samples of either
-    // level sit at ring positions 0..15)
-    if (QP == 1 && n0 == p.sk0 + 16) {
-        float h = 0.f;
-        heads[0] = 0.f;
-#pragma unroll
-        for (int d = 1; d <= kP; d++) { h += R.wB[(d - 1) & 31]; heads[d * nt] = h; }
-    }
-    if (TWO && QP == 2 && n0 == p.sk0 + 32) {
-        float h = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            h += R.rB[i & 31];
-            if (i + 1 >= 9) heads[(kP + 1 + i + 1 - 9) * nt] = h;
-        }
-    }
-    // first-level block end: last direct sample y = n0 - 1; heads of the next
-    // block are samples n0 .. n0 + d - 1 (this group)
-    if (dirF && (n0 & (p.LF - 1)) == 0) {
-        const int z = n0 / p.LF - 1;
-#pragma unroll 1
-        for (int l = 0; l < NF; l++) {
-            const int d = DF + l;
-            float nh = 0.f;
-#pragma unroll
-            for (int i = 0; i < kP; i++)
-                if (i < d) nh += R.wB[(PH0 + i) & 31];
-            float A = 0.f;
-#pragma unroll
-            for (int ll = 0; ll < NF; ll++)
-                if (ll == l) A = R.accF[ll];
-            float *hd = heads + d * nt;
-            c2_block_stat(c, p.lagF + l, A, R.bF0, R.bF1 - hd[0] + nh, p.LF, z);
-            hd[0] = nh;
-        }
-#pragma unroll
-        for (int l = 0; l < NF; l++) R.accF[l] = 0.f;
-        R.bF0 = 0.f;
-        R.bF1 = 0.f;
-    }
-    // second-level block end: last direct sample y1 = 8g - 9; heads of the
-    // next block are second-level samples 8g - 8 .. 8g - 9 + d
-    if (dirS && ((8 * g - 8) & (p.LS - 1)) == 0) {
-        const int z = (8 * g - 8) / p.LS - 1;
-#pragma unroll 1
-        for (int l = 0; l < 8; l++) {
-            const int d = 9 + l;
-            float nh = 0.f;
-#pragma unroll
-            for (int i = 1; i <= kP; i++)
-                if (i <= d) nh += R.rB[(PH1 - 9 + i + 32) & 31];
-            float A = 0.f;
-#pragma unroll
-            for (int ll = 0; ll < 8; ll++)
-                if (ll == l) A = R.accS[ll];
-            float *hd = heads + (kP + 1 + l) * nt;
-            c2_block_stat(c, p.lagS + l, A, R.bS0, R.bS1 - hd[0] + nh, p.LS, z);
-            hd[0] = nh;
-        }
-#pragma unroll
-        for (int l = 0; l < 8; l++) R.accS[l] = 0.f;
-        R.bS0 = 0.f;
-        R.bS1 = 0.f;
-    }
-}
+};
 
-// First lag of levels (k, k+1) handled by one pair pass.
-__host__ __device__ __forceinline__ int pair_lag0(int k, bool first17) { return first17 ? 0 : (kP + 1) + (k - 1) * 8; }
-
-// One (pixel, segment) of levels k and k+1: the register-ring pass over the
-// segment's level-k samples from `src`.  heads: this thread's heads (stride
-// nt floats); sst / smon (optional): shared-memory block statistics (written
-// back by the caller) and monitors of the pass's lags, from pair_lag0 on,
-// stride nt.
-template <bool CCF, bool FIRST17, bool TWO, class Src>
-__device__ __forceinline__ void c2_pair_body(const C2Args &a, Src &src, float *outA, float *outB, int k, int pix,
-                                             int seg, float *heads, int nt, float *sst = nullptr,
-                                             const float2 *smon = nullptr)
+// Sixteen samples n .. n+15 of a level's stream (0 from nk on).
+__device__ __forceinline__ void load16(float (&v)[16], const float *in, int n, int nk, int npix)
 {
-    C2Ctx c;
-    c2_ctx(c, a, pix, seg, k);
-    if (sst) { c.sst = sst; c.sst_stride = nt; c.lag0 = pair_lag0(k, FIRST17); }
-    if (smon) { c.smon = smon; c.smon_stride = nt; c.lag0 = pair_lag0(k, FIRST17); }
-    PairGeo p;
-    p.outA = outA;
-    p.outB = outB;
-    p.k = k;
-    p.nk = a.numbin[k];
-    p.nk1 = TWO ? a.numbin[k + 1] : 0;
-    p.nk2 = (TWO && k + 2 < a.q) ? a.numbin[k + 2] : 0;
-    const int s0 = seg << a.seg_log[k];
-    const int s1 = s0 + (1 << a.seg_log[k]);
-    p.sk0 = s0 >> k;
-    p.sk1 = s1 >= a.num ? p.nk : (s1 >> k);
-    p.LF = 1 << (c.ind - k);
-    p.LS = 1 << (c.ind - k - 1);
-    p.lagF = FIRST17 ? 0 : (kP + 1) + (k - 1) * 8;
-    p.lagS = (kP + 1) + k * 8;
-
-    if (c.valid) {
-        for (int lag = p.lagF; lag < p.lagF + PairReg<FIRST17>::NF; lag++)
-            for (int st = 0; st < kStatN; st++) c.stat(lag, st) = 0.f;
-        if (TWO)
-            for (int lag = p.lagS; lag < p.lagS + 8; lag++)
-                for (int st = 0; st < kStatN; st++) c.stat(lag, st) = 0.f;
+    const float *p = in + (size_t)n * npix;
+    if (n + 16 <= nk) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = __ldg(&p[(size_t)i * npix]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = n + i < nk ? __ldg(&p[(size_t)i * npix]) : 0.f;
     }
-    for (int f = 0; f < kHeadFields; f++) heads[f * nt] = 0.f;
-
-    PairReg<FIRST17> R;
-#pragma unroll
-    for (int i = 0; i < 32; i++) { R.wB[i] = 0.f; R.wA[i] = 0.f; R.rB[i] = 0.f; R.rA[i] = 0.f; }
-#pragma unroll
-    for (int d = 0; d < PairReg<FIRST17>::NF; d++) R.accF[d] = 0.f;
-#pragma unroll
-    for (int l = 0; l < 8; l++) R.accS[l] = 0.f;
-    R.bF0 = R.bF1 = R.bS0 = R.bS1 = 0.f;
-    if (!src.acquire(0)) return;
-    src.prep(p.sk0 / 16);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        R.curA[i] = CCF ? src.a(p.sk0 + i, i) : 0.f;
-        R.curB[i] = src.b(p.sk0 + i, i);
-    }
-    // groups of 16 samples: the segment's, then 48 more (the second level's
-    // last direct samples need 16 second-level samples past the segment);
-    // group r (relative) reads the samples of group r + 1
-    const int g0 = p.sk0 / 16;
-    int ng = (p.sk1 - p.sk0 + 48 + 15) / 16;
-    ng = (ng + 3) & ~3;
-    for (int r = 0; r < ng; r += 4) {
-        const int g = g0 + r;
-        if (!src.acquire(r + 1)) return;
-        c2_pair_group<CCF, FIRST17, TWO, 0>(c, p, heads, nt, R, g, src);
-        src.release(r);
-        if (!src.acquire(r + 2)) return;
-        c2_pair_group<CCF, FIRST17, TWO, 1>(c, p, heads, nt, R, g + 1, src);
-        src.release(r + 1);
-        if (!src.acquire(r + 3)) return;
-        c2_pair_group<CCF, FIRST17, TWO, 2>(c, p, heads, nt, R, g + 2, src);
-        src.release(r + 2);
-        if (!src.acquire(r + 4)) return;
-        c2_pair_group<CCF, FIRST17, TWO, 3>(c, p, heads, nt, R, g + 3, src);
-        src.release(r + 3);
-    }
-    // the partial blocks at the end into the totals
-#pragma unroll
-    for (int l = 0; l < PairReg<FIRST17>::NF; l++) c2_add_total(c, p.lagF + l, R.accF[l]);
-    if (TWO)
-#pragma unroll
-        for (int l = 0; l < 8; l++) c2_add_total(c, p.lagS + l, R.accS[l]);
 }
 
 template <bool CCF, bool FIRST17, bool TWO, int NT>
-__global__ void __launch_bounds__(NT) c2_pair_kernel(C2Args a, const float *inA, const float *inB,
+__global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const float *inA, const float *inB,
                                                      float *outA, float *outB, int k)
 {
-    constexpr int NL = (FIRST17 ? kP + 1 : 8) + (TWO ? 8 : 0);
-    __shared__ float heads_sm[kHeadFields * NT];
-    // block statistics and monitors of this pass's lags in shared memory: the
-    // read-modify-writes at block ends stay on chip; written back at the end
-    __shared__ float sst[NL * kStatN * NT];
-    __shared__ float2 smon[NL * NT];
-    const int nt = blockDim.x, tid = threadIdx.x;
-    const int pix = blockIdx.x * nt + tid, seg = blockIdx.y;
-    if (pix >= a.npix) return;          // no block-wide synchronisation below
-    if ((seg << a.seg_log[k]) >= a.num) return;
-    const int lag0 = pair_lag0(k, FIRST17);
-    {
-        const float4 *m = a.mon + (size_t)pix * a.chanum + lag0;
-        for (int l = 0; l < NL; l++) {
-            const float4 v = __ldg(&m[l]);
-            smon[l * nt + tid] = make_float2(v.x, v.y);
-        }
-    }
-    GlobalSrc src{CCF ? inA : inB, inB, a.numbin[k], a.npix, pix};
-    c2_pair_body<CCF, FIRST17, TWO>(a, src, outA, outB, k, pix, seg, heads_sm + tid, nt, sst + tid, smon + tid);
+    constexpr int NF = FIRST17 ? kP + 1 : 8;          // first-level lags
+    constexpr int DF = FIRST17 ? 0 : 9;               // delay of the first of them
+    constexpr int NS = TWO ? 8 : 0;
+    __shared__ float sm[(NF + NS) * kPairFields * NT];
+    const int tid = threadIdx.x;
+    const int pix = blockIdx.x * NT + tid, seg = blockIdx.y;
+    const int s0 = seg << a.seg_log[k];
+    if (pix >= a.npix || s0 >= a.num) return;          // no block-wide synchronisation below
+    const int s1 = s0 + (1 << a.seg_log[k]);
+    const int nk = a.numbin[k], nk1 = TWO ? a.numbin[k + 1] : 0;
+    const int nk2 = (TWO && k + 2 < a.q) ? a.numbin[k + 2] : 0;
+    const int y0 = s0 >> k, y1 = s1 >= a.num ? nk : (s1 >> k);      // direct samples of level k
+    const int ind = a.blk_ind[pix];
+    const int LF = 1 << (ind - k), LS = 1 << (ind - k - 1);
+    const int lag0 = FIRST17 ? 0 : (kP + 1) + (k - 1) * 8;
     float *gst = a.o.stats + (size_t)seg * a.stat_stride;
-    for (int l = 0; l < NL; l++)
-        for (int st = 0; st < kStatN; st++)
-            stat_ref(gst, a.npix, lag0 + l, st, pix) = sst[(size_t)(l * kStatN + st) * nt + tid];
+    PairBlocks<NT> pb;
+    pb.sm = sm + tid;
+    pb.mon = a.mon + (size_t)pix * a.chanum + lag0;
+    pb.rst = &stat_ref(gst, a.npix, lag0, 4, pix);
+    pb.bprod = a.o.gls ? a.o.bprod + ((ptrdiff_t)pix * (a.chanum - 1) + (lag0 - 1)) * a.o.pnum_stride : nullptr;
+    pb.npix = a.npix;
+    pb.pnum_stride = a.o.pnum_stride;
+    pb.pnum = a.li->pnum_by_ind[ind];
+    pb.zfirst = s0 >> ind;
+    pb.skip0 = FIRST17;
+#pragma unroll
+    for (int l = 0; l < NF + NS; l++)
+#pragma unroll
+        for (int f = 0; f < kPairFields; f++) pb.at(l, f) = 0.f;
+    // a segment without a counted block leaves its shift zero
+    if (pb.zfirst >= pb.pnum)
+        for (int l = 0; l < NF + NS; l++) pb.rst[(size_t)l * kStatN * a.npix] = 0.f;
+    inA += pix;
+    inB += pix;
+    if (outB) {
+        outA += pix;
+        outB += pix;
+    }
+
+    float w[32], cur[16];              // first-level samples y .. y+31; the next 16, loading
+    float x[16];                       // CCF: direct-trace samples y .. y+15
+    float r[24], rx[8];                // second-level samples y/2-8 .. y/2+15; CCF: direct ones y/2-8 .. y/2-1
+    float accF[NF], accS[8];
+    float bF = 0.f, bFd = 0.f, bS = 0.f, bSd = 0.f;
+#pragma unroll
+    for (int l = 0; l < NF; l++) accF[l] = 0.f;
+#pragma unroll
+    for (int l = 0; l < 8; l++) accS[l] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 24; i++) r[i] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) rx[i] = 0.f;
+    load16(cur, inB, y0, nk, a.npix);
+#pragma unroll
+    for (int i = 0; i < 16; i++) w[16 + i] = cur[i];
+    load16(cur, inB, y0 + 16, nk, a.npix);
+    // heads of the first blocks, and the second level's first eight samples
+    {
+        float h = 0.f;
+        if (FIRST17) pb.at(0, 4) = 0.f;
+#pragma unroll
+        for (int d = 1; d <= kP; d++) {
+            h += w[16 + d - 1];
+            if (d >= DF) pb.at(d - DF, 4) = h;
+        }
+        if (TWO)
+#pragma unroll
+            for (int i = 0; i < 8; i++) r[16 + i] = (y0 >> 1) + i < nk1 ? w[16 + 2 * i] + w[17 + 2 * i] : 0.f;
+    }
+    // one step more than first-level steps: the second level is a step behind
+    const int ysteps = y0 + ((y1 - y0 + 15) & ~15);
+#pragma unroll 1
+    for (int y = y0; y < ysteps + (TWO ? 16 : 0); y += 16) {
+        const bool first_level = y < ysteps;
+        const bool second_level = TWO && y > y0;
+        float xn[8];                   // CCF: second-level direct samples of this step
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            w[i] = w[16 + i];
+            w[16 + i] = cur[i];
+        }
+        if (CCF) load16(x, inA, y, nk, a.npix);
+        load16(cur, inB, y + 32, nk, a.npix);
+        if (TWO) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) r[i] = r[i + 8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) r[16 + i] = (y >> 1) + 8 + i < nk1 ? w[16 + 2 * i] + w[17 + 2 * i] : 0.f;
+            if (CCF)
+#pragma unroll
+                for (int i = 0; i < 8; i++) xn[i] = (y >> 1) + i < nk1 ? x[2 * i] + x[2 * i + 1] : 0.f;
+        }
+        if (first_level) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const float d = CCF ? x[j] : w[j];
+#pragma unroll
+                for (int l = 0; l < NF; l++) accF[l] = fmaf(d, w[j + DF + l], accF[l]);
+                bF += d;
+                if (CCF) bFd += w[j];
+            }
+            if (TWO && outB) {         // level k+2: pair sums of second-level samples y/2 .. y/2+7
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int m = (y >> 2) + i;
+                    if (m < nk2 && m < (s1 >> (k + 2))) {
+                        outB[(size_t)m * a.npix] = r[8 + 2 * i] + r[9 + 2 * i];
+                        if (CCF) outA[(size_t)m * a.npix] = xn[2 * i] + xn[2 * i + 1];
+                    }
+                }
+            }
+            if (((y + 16) & (LF - 1)) == 0) {
+                float nh[NF], h = 0.f;
+                if (FIRST17) nh[0] = 0.f;
+#pragma unroll
+                for (int d = 1; d <= kP; d++) {
+                    h += w[16 + d - 1];
+                    if (d >= DF) nh[d - DF] = h;
+                }
+                pb.template end<NF>(0, accF, bF, CCF ? bFd : bF, nh, LF, (y + 16) / LF - 1);
+                bF = 0.f;
+                bFd = 0.f;
+            }
+        }
+        if (second_level) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float d = CCF ? rx[i] : r[i];
+#pragma unroll
+                for (int l = 0; l < 8; l++) accS[l] = fmaf(d, r[i + 9 + l], accS[l]);
+                bS += d;
+                if (CCF) bSd += r[i];
+            }
+            if (((y >> 1) & (LS - 1)) == 0) {
+                float nh[8], h = 0.f;
+#pragma unroll
+                for (int d = 1; d <= 16; d++) {
+                    h += r[8 + d - 1];
+                    if (d >= 9) nh[d - 9] = h;
+                }
+                pb.template end<8>(NF, accS, bS, CCF ? bSd : bS, nh, LS, (y >> 1) / LS - 1);
+                bS = 0.f;
+                bSd = 0.f;
+            }
+        } else if (TWO) {              // the first step: heads of the second level's first block
+            float h = 0.f;
+#pragma unroll
+            for (int d = 1; d <= 16; d++) {
+                h += r[8 + d - 1];
+                if (d >= 9) pb.at(NF + d - 9, 4) = h;
+            }
+        }
+        if (CCF && TWO)
+#pragma unroll
+            for (int i = 0; i < 8; i++) rx[i] = xn[i];
+    }
+    // the partial blocks at the end into the totals; everything out
+#pragma unroll
+    for (int l = 0; l < NF + NS; l++) {
+        ff t = {pb.at(l, 0), pb.at(l, 1)};
+        ff_add(t, l < NF ? accF[l < NF ? l : 0] : accS[l < NF ? 0 : l - NF]);
+        stat_ref(gst, a.npix, lag0 + l, 0, pix) = t.hi;
+        stat_ref(gst, a.npix, lag0 + l, 1, pix) = t.lo;
+        stat_ref(gst, a.npix, lag0 + l, 2, pix) = pb.at(l, 2);
+        stat_ref(gst, a.npix, lag0 + l, 3, pix) = pb.at(l, 3);
+    }
 }
 
 // ---------------------------------------------------------------------------
 // Tail kernel: one level k >= k0 of one (pixel, segment) per thread, for the
 // top levels whose blocks may be as short as one sample.  The thread builds
-// its level-k samples from the level-k0 stream (sums of 2^(k-k0) samples),
-// keeps a ring of its last 32 samples in shared memory and its lags' block
-// sums and block statistics in registers; the statistics are written once.
+// its level-k samples from the level-k0 stream (pairwise sums of 2^(k-k0)
+// samples), 16 a step, with the 32 samples from the step's first on, its lags'
+// block sums and block statistics in registers; the statistics are written
+// once.
 // ---------------------------------------------------------------------------
-// (8 warps per SM at least: 128 registers, a few spilled, against 160 at
-// 6 warps -- the kernel waits on its loads, 6.44 -> 6.18 ms for the chain)
+// Samples n .. n+15 of level k0 + LM (0 from nkk on), pairwise sums of the
+// level-k0 stream (java:9467-9476).
+template <int LM>
+__device__ __forceinline__ void tail_samples(float *v, const float *in, int n, int nkk, int npix)
+{
+    constexpr int M = 1 << LM;
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+        float t[M];
+        const bool inside = n + u < nkk;
+        const float *p = in + (size_t)(n + u) * M * npix;
+#pragma unroll
+        for (int i = 0; i < M; i++) t[i] = inside ? __ldg(&p[(size_t)i * npix]) : 0.f;
+#pragma unroll
+        for (int h = M / 2; h >= 1; h /= 2)
+#pragma unroll
+            for (int i = 0; i < h; i++) t[i] = t[2 * i] + t[2 * i + 1];
+        v[u] = t[0];
+    }
+}
+__device__ __forceinline__ void tail_load(float *v, const float *in, int n, int lm, int nkk, int npix)
+{
+    if (lm == 0) tail_samples<0>(v, in, n, nkk, npix);
+    else if (lm == 1) tail_samples<1>(v, in, n, nkk, npix);
+    else if (lm == 2) tail_samples<2>(v, in, n, nkk, npix);
+    else tail_samples<3>(v, in, n, nkk, npix);
+}
+
 template <bool CCF, int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) c2_tail_kernel(C2Args a, const float *inA, const float *inB, int k0)
 {
-    __shared__ float ring_sm[(CCF ? 2 : 1) * 32 * NT];
+    __shared__ float2 mon_sm[8 * NT];               // the lags' monitors
     const int tid = threadIdx.x;
     const int pix = blockIdx.x * NT + tid, seg = blockIdx.y, k = k0 + blockIdx.z;
-    if (pix >= a.npix || k >= a.q) return;          // no block-wide synchronisation below
-    float *rb = ring_sm + tid;
-    float *ra = CCF ? ring_sm + 32 * NT + tid : rb;
-    if (!CCF) inA = inB;
-    C2Ctx c;
-    c2_ctx(c, a, pix, seg, k);
     const int s0 = seg << a.seg_log[k];
-    if (s0 >= a.num) return;
+    if (pix >= a.npix || k >= a.q || s0 >= a.num) return;          // no block-wide synchronisation below
     const int s1 = min(s0 + (1 << a.seg_log[k]), a.num);
-    const int nkk = a.numbin[k], nk0 = a.numbin[k0];
+    const int nkk = a.numbin[k], lm = k - k0;
     const int ys0 = s0 >> k, ys1 = (s1 >= a.num) ? nkk : (s1 >> k);
-    const int m = 1 << (k - k0);
     const int lag0 = (kP + 1) + (k - 1) * 8;
-    const int lk = c.ind - k;
-    const int L = lk > 0 ? (1 << lk) : 1;
-
-    float ma[8], mb[8];
+    const int ind = a.blk_ind[pix], pnum = a.li->pnum_by_ind[ind], zfirst = s0 >> ind;
+    const int L = ind > k ? 1 << (ind - k) : 1, logL = ind > k ? ind - k : 0;
+    const float fL = (float)L, iL = 1.f / fL;
+    float *bprod = a.o.gls ? a.o.bprod + ((size_t)pix * (a.chanum - 1) + (lag0 - 1)) * a.o.pnum_stride : nullptr;
+    inA += pix;
+    inB += pix;
+    float2 *ms = mon_sm + tid;
 #pragma unroll
-    for (int l = 0; l < 8; l++) {
-        const float4 mm = __ldg(&c.mon[lag0 + l]);
-        ma[l] = mm.x;
-        mb[l] = mm.y;
-    }
+    for (int l = 0; l < 8; l++) ms[l * NT] = __ldg((const float2 *)&a.mon[(size_t)pix * a.chanum + lag0 + l]);
+
     float acc[8], head[8], thi[8], tlo[8], S1[8], S2[8], rr[8];
 #pragma unroll
-    for (int l = 0; l < 8; l++) {
-        acc[l] = head[l] = thi[l] = tlo[l] = S1[l] = S2[l] = rr[l] = 0.f;
-    }
+    for (int l = 0; l < 8; l++) acc[l] = thi[l] = tlo[l] = S1[l] = S2[l] = rr[l] = 0.f;
     float b0 = 0.f, b1 = 0.f;
-
-    // samples ys0 .. ys1 + 15 (the last direct samples' delayed partners);
-    // samples from nkk on are zero.  Loads are issued 8 samples at a time.
-    const int nend = ys1 + 16;
-#pragma unroll 1
-    for (int nb = ys0; nb < nend; nb += 8) {
-        float vb[8], va[8];
+    float w[32], x[16];
+    tail_load(w + 16, inB, ys0, lm, nkk, a.npix);
+    {
+        float h = 0.f;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            vb[u] = 0.f;
-            va[u] = 0.f;
-            const int n = nb + u;
-            if (n < nkk && n < nend) {
-                if (m <= 8) {
-                    // pairwise sums, as the levels are built (java:9467-9476)
-                    float wb[8], wa[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int q = n * m + i;
-                        const bool in = i < m && q < nk0;
-                        wb[i] = in ? __ldg(&inB[(size_t)q * a.npix + pix]) : 0.f;
-                        wa[i] = (CCF && in) ? __ldg(&inA[(size_t)q * a.npix + pix]) : 0.f;
-                    }
-#pragma unroll
-                    for (int w = 1; w < 8; w *= 2)
-#pragma unroll
-                        for (int i = 0; i < 8; i += 2 * w) {
-                            wb[i] += wb[i + w];
-                            wa[i] += wa[i + w];
-                        }
-                    vb[u] = wb[0];
-                    va[u] = wa[0];
-                } else {
-                    for (int i = 0; i < m; i++) {
-                        const int q = n * m + i;
-                        if (q < nk0) {
-                            vb[u] += __ldg(&inB[(size_t)q * a.npix + pix]);
-                            if (CCF) va[u] += __ldg(&inA[(size_t)q * a.npix + pix]);
-                        }
-                    }
-                }
-            }
+        for (int i = 0; i < 16; i++) {
+            h += w[16 + i];
+            if (i + 1 >= 9) head[i + 1 - 9] = h;
         }
+    }
+#pragma unroll 1
+    for (int y = ys0; y < ys1; y += 16) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int n = nb + u;
-            if (n >= nend) break;
-            rb[(n & 31) * NT] = vb[u];
-            if (CCF) ra[(n & 31) * NT] = va[u];
-            const int y = n - 16;
-            if (y < ys0) continue;
-            if (y == ys0) {
+        for (int i = 0; i < 16; i++) w[i] = w[16 + i];
+        tail_load(w + 16, inB, y + 16, lm, nkk, a.npix);
+        if (CCF) tail_load(x, inA, y, lm, nkk, a.npix);
+        // a segment may end inside the step
+        const int left = ys1 - y;
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            if (j >= left) break;
+            const float d = CCF ? x[j] : w[j];
+#pragma unroll
+            for (int l = 0; l < 8; l++) acc[l] = fmaf(d, w[j + 9 + l], acc[l]);
+            b0 += d;
+            if (CCF) b1 += w[j];
+            if (((y + j + 1) & (L - 1)) == 0) {
+                // heads of the next block: sums of the delayed samples y+j+1 .. y+j+d
                 float h = 0.f;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    h += rb[((y + i) & 31) * NT];
-                    if (i + 1 >= 9) head[i + 1 - 9] = h;
-                }
-            }
-            const float x0 = ra[(y & 31) * NT];
-#pragma unroll
-            for (int l = 0; l < 8; l++) acc[l] = fmaf(x0, rb[((y + 9 + l) & 31) * NT], acc[l]);
-            b0 += x0;
-            b1 += rb[(y & 31) * NT];
-            if (((y + 1) & (L - 1)) == 0) {
-                // heads of the next block: sums of the delayed samples y+1 .. y+d
-                float nh[8], h = 0.f;
-#pragma unroll
-                for (int i = 1; i <= 16; i++) {
-                    h += rb[((y + i) & 31) * NT];
-                    if (i >= 9) nh[i - 9] = h;
-                }
-                const int z = y / L;
-                const bool stat = z < c.pnum;
+                for (int i = 1; i <= 8; i++) h += w[j + i];
+                const int z = (y + j) >> logL;
+                const bool stat = z < pnum;
 #pragma unroll
                 for (int l = 0; l < 8; l++) {
-                    const float D = b1 - head[l] + nh[l];
-                    const float P = (acc[l] - mb[l] * b0 - ma[l] * D + (float)L * ma[l] * mb[l]) / (float)L;
+                    h += w[j + 9 + l];
+                    const float2 m = ms[l * NT];
+                    const float P = block_product(acc[l], b0, (CCF ? b1 : b0) - head[l] + h, m.x, m.y, fL, iL);
                     ff t = {thi[l], tlo[l]};
                     ff_add(t, acc[l]);
                     thi[l] = t.hi;
                     tlo[l] = t.lo;
                     if (stat) {
-                        if (z == c.zfirst) rr[l] = P;
+                        if (z == zfirst) rr[l] = P;
                         const float dv = P - rr[l];
                         S1[l] += dv;
                         S2[l] = fmaf(dv, dv, S2[l]);
-                        if (c.gls)
-                            c.bprod[((size_t)pix * (c.chanum - 1) + (lag0 + l - 1)) * c.pnum_stride + z] = P;
+                        if (bprod) bprod[(size_t)l * a.o.pnum_stride + z] = P;
                     }
-                    head[l] = nh[l];
+                    head[l] = h;
                     acc[l] = 0.f;
                 }
                 b0 = 0.f;
@@ -561,15 +431,16 @@ __global__ void __launch_bounds__(NT, 512 / NT) c2_tail_kernel(C2Args a, const f
             }
         }
     }
+    float *gst = a.o.stats + (size_t)seg * a.stat_stride;
 #pragma unroll
     for (int l = 0; l < 8; l++) {
         ff t = {thi[l], tlo[l]};
         ff_add(t, acc[l]);
-        stat_ref(c.stats, c.npix, lag0 + l, 0, pix) = t.hi;
-        stat_ref(c.stats, c.npix, lag0 + l, 1, pix) = t.lo;
-        stat_ref(c.stats, c.npix, lag0 + l, 2, pix) = S1[l];
-        stat_ref(c.stats, c.npix, lag0 + l, 3, pix) = S2[l];
-        stat_ref(c.stats, c.npix, lag0 + l, 4, pix) = rr[l];
+        stat_ref(gst, a.npix, lag0 + l, 0, pix) = t.hi;
+        stat_ref(gst, a.npix, lag0 + l, 1, pix) = t.lo;
+        stat_ref(gst, a.npix, lag0 + l, 2, pix) = S1[l];
+        stat_ref(gst, a.npix, lag0 + l, 3, pix) = S2[l];
+        stat_ref(gst, a.npix, lag0 + l, 4, pix) = rr[l];
     }
 }
 
