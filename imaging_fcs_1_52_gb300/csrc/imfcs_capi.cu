@@ -107,6 +107,14 @@ bool build_lag_info(int p, int q, int num, LagInfo &li, int &chanum, int &blockn
     blocknum = (int)floor(log(mtab[1]) / log(2)) - 2;
     if (blocknum < 4) { err = "too few frames for the blocking transform"; return false; }
     if (blocknum > kMaxBlockLevels) { err = "too many blocking levels"; return false; }
+    for (int x = 0; x < chanum; x++) li.inv_prodnum[x] = 1.0 / li.prodnum[x];
+    for (int ind = 0; ind < kMaxBlockLevels; ind++) {
+        li.inv_pnum[ind] = 1.0 / li.pnum_by_ind[ind];
+        li.inv_pnum1[ind] = 1.0 / (li.pnum_by_ind[ind] - 1);
+        const double n = ind < 31 ? (double)((num - 1) >> ind) : 0.0;
+        li.blk_inv_n[ind] = 1.0 / n;
+        li.blk_err[ind] = 1.0 / sqrt(2.0 * (n - 1.0));
+    }
     return true;
 }
 
@@ -236,6 +244,7 @@ struct imfcs_plan {
     size_t bytes = 0;
     // scratch
     float *trace = nullptr, *bparams = nullptr, *basis = nullptr;
+    unsigned *trace_sums = nullptr;   // only where s0 is too small to hold the trace's raw sums
     double *proj = nullptr;
     int *snap_pos = nullptr;
     float2 *segtot = nullptr, *snap_part = nullptr;
@@ -462,6 +471,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     AS(pl->stats, corr_stats_floats(j));
     AS(pl->streams, corr_stream_floats(j));
     AS(pl->s0, level0_stream_floats(j));
+    if (trace_sums_elems(j) > level0_stream_floats(j)) AS(pl->trace_sums, trace_sums_elems(j));
     AS(pl->acf_int, np * chanum);
     AS(pl->var_int, np * chanum);
     AL(pl->lagtime, chanum);
@@ -700,7 +710,9 @@ int plan_execute_any(imfcs_plan *pl, const void *dev_stack, const imfcs_outputs 
     for (int i = 0; i <= imfcs_plan::kStages; i++) pl->ev_used[i] = false;
     pl->launches = 0;
     pl->mark(0, s);
-    CK(launch_trace(j, dev_stack, pl->trace, s));
+    // the trace's raw sums are read before the streaming pass writes s0
+    CK(launch_trace(j, dev_stack, pl->trace_sums ? pl->trace_sums : (unsigned *)pl->s0, pl->trace, s));
+    if (trace_sums_elems(j)) pl->launches += 1;
     if (pl->given_bleach) CK(launch_center_given(j, pl->trace, pl->bparams, s));
     else CK(launch_bleach(j, pl->trace, pl->proj, (float)pl->uscale, (float)pl->uoff, pl->bparams, s));
     pl->launches += 2;
@@ -721,7 +733,7 @@ int plan_execute_any(imfcs_plan *pl, const void *dev_stack, const imfcs_outputs 
         for (int i = 3; i <= 6; i++) pl->mark(i, s);
         return 0;
     }
-    CK(launch_block(j, pl->s0, pl->blkmon, pl->nbseg, pl->s1, pl->s2, pl->segsum, pl->blk_ind, pl->blk_ok, s));
+    CK(launch_block(j, pl->li_dev, pl->s0, pl->blkmon, pl->nbseg, pl->s1, pl->s2, pl->segsum, pl->blk_ind, pl->blk_ok, s));
     pl->launches += 2;
     pl->mark(3, s);
     CK(launch_corr(j, pl->li_dev, dev_stack, pl->bparams, pl->basis, pl->s0, pl->mon, pl->blk_ind, acf, var,

@@ -67,6 +67,10 @@ __device__ __forceinline__ float block_product(float A, float B, float D, float 
 // code, 336 FMAs for levels 0-1, serves every step and block ends are in it
 // once.  What only block ends touch -- totals, statistics, heads -- is in
 // shared memory, the monitors and the statistics' shift in the L1.
+// Bound by issue (60 % active at 12 warps an SM, 44 instructions a frame and
+// pixel of which 25 are the products): 2.90 -> 1.48 ms for levels 0-1 and 0.85
+// -> 0.46 for 2-3 at 16,384 pixels x 50,000 frames against four unrolled
+// copies of the step with 32-entry rings and per-lag head sums.
 // ---------------------------------------------------------------------------
 constexpr int kPairFields = 5;    // per lag in shared memory: Ahi, Alo, S1, S2, head
 
@@ -318,7 +322,8 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
 // its level-k samples from the level-k0 stream (pairwise sums of 2^(k-k0)
 // samples), 16 a step, with the 32 samples from the step's first on, its lags'
 // block sums and block statistics in registers; the statistics are written
-// once.
+// once.  1.65 -> 0.73 ms at 16,384 pixels x 50,000 frames against a ring in
+// shared memory read sample by sample.
 // ---------------------------------------------------------------------------
 // Samples n .. n+15 of level k0 + LM (0 from nkk on), pairwise sums of the
 // level-k0 stream (java:9467-9476).
@@ -690,57 +695,91 @@ __global__ void __launch_bounds__(kCgThreads, 6) cg_blocks_kernel(CgArgs a)
 // (java:9491-9531).
 // ---------------------------------------------------------------------------
 // Outputs of one (pixel, lag) from its product total A and the statistics of
-// its pnum blocked products (sums S1, S2 shifted by r).
+// its pnum blocked products (sums S1, S2 shifted by r), FP64.
 __device__ __forceinline__ void write_lag(const CorrOut &o, const float4 *mon, const LagInfo *li, int chanum, int pix,
-                                          int lag, int pnum, double A, double S1, double S2, double r)
+                                          int lag, int ind, double A, double S1, double S2, double r)
 {
     const float4 m = mon[(size_t)pix * chanum + lag];
-    const double n = li->prodnum[lag];
-    const double dmDm = (double)m.z * (double)m.w;
-    const double sumprod = A - n * (double)m.x * (double)m.y;
-    const double corav = sumprod / (n * dmDm);
-    const double pn = pnum;
-    const double bv = (S2 / pn - (S1 / pn) * (S1 / pn)) / ((pn - 1) * dmDm * dmDm);
-    double acf = corav;
-    if (o.gls) acf = (lag == 0) ? 0.0 : (S1 + pn * r) / (pn * dmDm);   // mcov (java:9526-9531)
+    const double n = li->prodnum[lag], ip = li->inv_pnum[ind];
+    const double idm = newton_rcp(f2d(m.z) * f2d(m.w));
+    const double cov = fma(-(n * f2d(m.x)), f2d(m.y), A) * li->inv_prodnum[lag];    // mean of the centred products
+    const double mean = S1 * ip;
+    const double bv = fma(S2, ip, -mean * mean) * li->inv_pnum1[ind] * idm * idm;
+    double acf = cov * idm;
+    if (o.gls) acf = (lag == 0) ? 0.0 : (mean + r) * idm;   // mcov (java:9526-9531)
     if (o.acf) o.acf[(size_t)pix * chanum + lag] = acf;
     if (o.var) o.var[(size_t)pix * chanum + lag] = bv;
-    if (o.sd) o.sd[(size_t)pix * chanum + lag] = sqrt(bv);
+    if (o.sd) o.sd[(size_t)pix * chanum + lag] = newton_sqrt(bv);
     if (lag == 1) {
         if (o.nb_mean) o.nb_mean[pix] = m.z;
-        if (o.nb_cov) o.nb_cov[pix] = sumprod / n;
+        if (o.nb_cov) o.nb_cov[pix] = cov;
     }
 }
 
-__global__ void c2_finalize_kernel(C2Args a)
+// The segments combined in FP64 alone, for sums that left the FP32 range.
+static __device__ __noinline__ void plain_segments(const float *st, size_t np, size_t stride, int nseg, int sl, int num,
+                                                   int ind, int pnum, double r0, double &A, double &S1, double &S2)
 {
-    // lag-major threads: the segment statistics [lag][stat][pixel] are read
-    // coalesced (they are most of this kernel's traffic)
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.npix * a.chanum) return;
-    const int lag = i / a.npix, pix = i % a.npix;
+    A = S1 = S2 = 0.0;
+    for (int sg = 0; sg < nseg; sg++, st += stride) {
+        A += (double)st[0] + (double)st[np];
+        const int f0 = sg << sl, f1 = min(f0 + (1 << sl), num);
+        const int cnt = min(pnum, (f1 + (1 << ind) - 1) >> ind) - (f0 >> ind);
+        if (cnt <= 0) continue;
+        const double d1 = st[2 * np], dr = (double)st[4 * np] - r0;
+        S1 += d1 + cnt * dr;
+        S2 += st[3 * np] + 2.0 * dr * d1 + cnt * dr * dr;
+    }
+}
+
+// Grid (pixel blocks, lags).  Bound by FP64 issue (1/64 of the FP32 rate):
+// plain sums of FP32 values run as compensated FP32 sums (their error, below
+// 1e-14, is FP64's own of a dozen terms), only the products with the segments'
+// shifts are FP64, conversions go to the integer pipe.  0.56 -> 0.19 ms at
+// 16,384 pixels x 50,000 frames.  Float-float for those products too was
+// no faster and moved results by 1e-13, enough to round some of the fits' FP32
+// data and weights the other way.
+__global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
+{
+    const int pix = blockIdx.x * 128 + threadIdx.x, lag = blockIdx.y;
+    if (pix >= a.npix) return;
     const int ind = a.blk_ind[pix];
     const int pnum = a.li->pnum_by_ind[ind];
     const int level = lag <= a.p ? 0 : 1 + (lag - (a.p + 1)) / (a.p / 2);
     const int sl = a.seg_log[level];
     const int nseg = (a.num + (1 << sl) - 1) >> sl;
-    double A = 0.0, S1 = 0.0, S2 = 0.0, r = 0.0;
-    bool have_r = false;
-    for (int sg = 0; sg < nseg; sg++) {
-        float *st = a.o.stats + sg * a.stat_stride;
-        A += (double)stat_ref(st, a.npix, lag, 0, pix) + (double)stat_ref(st, a.npix, lag, 1, pix);
-        const int s0 = sg << sl, s1 = min(s0 + (1 << sl), a.num);
-        const int z0 = s0 >> ind, z1 = (s1 + (1 << ind) - 1) >> ind;
-        const int cnt = max(0, min(pnum, z1) - z0);
-        if (cnt == 0) continue;
-        const double rs = stat_ref(st, a.npix, lag, 4, pix);
-        const double s1s = stat_ref(st, a.npix, lag, 2, pix), s2s = stat_ref(st, a.npix, lag, 3, pix);
-        if (!have_r) { r = rs; have_r = true; }
-        const double dr = rs - r;
-        S1 += s1s + cnt * dr;
-        S2 += s2s + 2.0 * dr * s1s + cnt * dr * dr;
+    const float *st = &stat_ref(a.o.stats, a.npix, lag, 0, pix);
+    const size_t np = a.npix;
+    const double r0 = f2d(__ldg(&st[4 * np]));      // segment 0 always has a counted block
+    ff A = {0.f, 0.f}, s1 = {0.f, 0.f}, s2 = {0.f, 0.f};
+    double S1 = 0.0, S2 = 0.0;
+    const float4 m = a.mon[(size_t)pix * a.chanum + lag];
+    const bool bad = m.x != m.x || m.y != m.y;      // a non-finite frame in the lag's windows: NaN, whatever the sums
+#pragma unroll 2
+    for (int sg = 0; sg < nseg && !bad; sg++, st += a.stat_stride) {
+        const float hi = __ldg(&st[0]), lo = __ldg(&st[np]), s1f = __ldg(&st[2 * np]), s2f = __ldg(&st[3 * np]),
+                    rf = __ldg(&st[4 * np]);
+        ff_add(A, hi);
+        A.lo = __fadd_rn(A.lo, lo);
+        // the segment's blocks that count
+        const int f0 = sg << sl, f1 = min(f0 + (1 << sl), a.num);
+        const int cnt = min(pnum, (f1 + (1 << ind) - 1) >> ind) - (f0 >> ind);
+        if (cnt <= 0) continue;
+        // sums of P - r0 from those of P - r: with dr = r - r0,
+        // S1 += s1 + cnt dr and S2 += s2 + dr (2 s1 + cnt dr)
+        ff_add(s1, s1f);
+        ff_add(s2, s2f);
+        const double dr = f2d(rf) - r0, c = f2d((float)cnt);
+        S1 = fma(c, dr, S1);
+        S2 = fma(dr, fma(c, dr, f2d(2.f * s1f)), S2);
     }
-    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, pnum, A, S1, S2, r);
+    S1 += f2d(s1.hi) + f2d(s1.lo);
+    S2 += f2d(s2.hi) + f2d(s2.lo);
+    double Ad = f2d(A.hi) + f2d(A.lo);
+    if (!(isfinite(A.hi) && isfinite(s1.hi) && isfinite(s2.hi)) && !bad)
+        plain_segments(&stat_ref(a.o.stats, a.npix, lag, 0, pix), np, a.stat_stride, nseg, sl, a.num, ind, pnum, r0, Ad,
+                       S1, S2);
+    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, ind, Ad, S1, S2, r0);
 }
 
 // P = 32: the block statistics of one (pixel, lag) over its blocks in order
@@ -750,7 +789,8 @@ __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
     const int pc = blockIdx.x * 128 + threadIdx.x, lag = blockIdx.y;
     if (pc >= a.np) return;
     const int pix = a.p0 + pc;
-    const int pnum = a.li->pnum_by_ind[a.blk_ind[pix]];
+    const int ind = a.blk_ind[pix];
+    const int pnum = a.li->pnum_by_ind[ind];
     const float *pz = a.pz + (size_t)lag * a.pnum_max * a.cs + pc;
     const float r = pnum > 0 ? pz[0] : 0.f;
     float S1 = 0.f, S2 = 0.f;
@@ -771,9 +811,9 @@ __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
     double A = 0.0;
     for (int sg = 0; sg < nseg; sg++) {
         const float2 t = a.tot[((size_t)sg * a.chanum + lag) * a.cs + pc];
-        A += (double)t.x + (double)t.y;
+        A += f2d(t.x) + f2d(t.y);
     }
-    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, pnum, A, S1, S2, r);
+    write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, ind, A, f2d(S1), f2d(S2), f2d(r));
 }
 
 // ---------------------------------------------------------------------------
@@ -1015,8 +1055,7 @@ cudaError_t launch_corr2(const Job &j, const LagInfo *li, const float *s0, const
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const int n = j.npix * j.chanum;
-    c2_finalize_kernel<<<(n + 255) / 256, 256, 0, stream>>>(a);
+    c2_finalize_kernel<<<dim3((j.npix + 127) / 128, j.chanum), 128, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

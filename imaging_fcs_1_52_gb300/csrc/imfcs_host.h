@@ -32,7 +32,9 @@ struct GlsArgs;
 cudaError_t launch_gls(const GlsArgs &g, cudaStream_t stream);
 
 // prep launchers (imfcs_prep_launch.cu)
-cudaError_t launch_trace(const Job &j, const void *stack, float *trace, cudaStream_t s);
+// sums: trace_sums_elems scratch values (0 of them: the one-pass kernel runs)
+cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float *trace, cudaStream_t s);
+size_t trace_sums_elems(const Job &j);
 cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, float uscale,
                           float uoff, float *bparams, cudaStream_t s);
 cudaError_t launch_center_given(const Job &j, const float *trace, float *bparams, cudaStream_t s);
@@ -45,7 +47,7 @@ cudaError_t launch_monitor_finalize(const Job &j, const LagInfo *li_dev, const f
 // N&B mode: lag-1 mean and covariance only (sum: npix doubles of scratch)
 cudaError_t launch_nb_lag1(const Job &j, const float *s0, const float4 *mon, double *sum, double *nb_mean,
                            double *nb_cov, cudaStream_t s);
-cudaError_t launch_block(const Job &j, const float *s0, const float4 *blkmon, int nbseg, float *s1, float *s2,
+cudaError_t launch_block(const Job &j, const LagInfo *li, const float *s0, const float4 *blkmon, int nbseg, float *s1, float *s2,
                          float *segsum, int *ind, int *ok, cudaStream_t s);
 cudaError_t launch_binning(const float *in, float *out, int win, int hin, int wt, int ht,
                            int frames, int bx, int by, cudaStream_t s);

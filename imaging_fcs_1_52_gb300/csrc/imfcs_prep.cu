@@ -53,6 +53,97 @@ __global__ void __launch_bounds__(256) trace_kernel(Job j, const void *stack, fl
     }
 }
 
+// The same in two passes where the traces read most of the frames' columns:
+// the sums of `ave` frames of every raw pixel of the rows read, once and with
+// wide loads (sums[x][pixel], bound by HBM), then the windows of the sums.
+// VEC raw pixels per thread: 8 (16-byte loads), 2 or 1 by the frames' length
+// and alignment.  One pass with a guarded 2-byte load per raw value was bound
+// by issue: 0.67 -> 0.28 ms at 128x128x50,000 (read once at 6.8 TB/s: 0.24),
+// 0.73 -> 0.09 for overlapping 5 x 5 windows at 101x67x12,345.
+template <int VEC>
+__global__ void __launch_bounds__(128) trace_sums_kernel(const uint16_t *base, size_t fsz, int nelem, int ave,
+                                                         unsigned *sums)
+{
+    const int i = (blockIdx.x * 128 + threadIdx.x) * VEC;
+    if (i >= nelem) return;
+    const uint16_t *p = base + (size_t)blockIdx.y * ave * fsz + i;
+    unsigned acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; e++) acc[e] = 0;
+    auto add2 = [](unsigned w, unsigned *a) {         // two 16-bit values, one integer dot product each
+        a[0] = __dp2a_lo(w, 0x0001u, a[0]);
+        a[1] = __dp2a_lo(w, 0x0100u, a[1]);
+    };
+    constexpr int U = VEC == 8 ? 4 : 8;
+    int f = 0;
+    for (; f + U <= ave; f += U, p += (size_t)U * fsz) {
+        if constexpr (VEC == 8) {
+            uint4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = __ldcs((const uint4 *)(p + (size_t)u * fsz));
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                add2(v[u].x, acc);
+                add2(v[u].y, acc + 2);
+                add2(v[u].z, acc + 4);
+                add2(v[u].w, acc + 6);
+            }
+        } else if constexpr (VEC == 2) {
+            unsigned v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = __ldcs((const unsigned *)(p + (size_t)u * fsz));
+#pragma unroll
+            for (int u = 0; u < U; u++) add2(v[u], acc);
+        } else {
+            uint16_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) v[u] = __ldcs(p + (size_t)u * fsz);
+#pragma unroll
+            for (int u = 0; u < U; u++) acc[0] += v[u];
+        }
+    }
+    for (; f < ave; f++, p += fsz)
+#pragma unroll
+        for (int e = 0; e < VEC; e++) acc[e] += p[e];
+    unsigned *o = sums + (size_t)blockIdx.y * nelem + i;
+#pragma unroll
+    for (int e = 0; e < VEC; e++) o[e] = acc[e];
+}
+
+// Block (32 traces) x (8 rows), 4 points per thread, transposed through a
+// shared tile like trace_kernel.  row0: the first raw row of the sums.
+__global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigned *sums, int row0, int nelem,
+                                                            float *trace_out)
+{
+    __shared__ float tile[32][33];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int trace = blockIdx.x * 32 + tx;
+    const int xbase = blockIdx.y * 32;
+    if (trace < j.ntrace) {
+        int x0, y0;
+        trace_origin(j, trace, x0, y0);
+        const int bg = trace_bg_avg(j, trace) * j.ave;
+        const unsigned *w = sums + (size_t)(y0 - row0) * j.in_w + x0;
+        int acc[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) acc[r] = 0;
+        for (int k = 0; k < j.biny; k++)
+            for (int i = 0; i < j.binx; i++)
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int x = min(xbase + ty * 4 + r, j.nopit - 1);
+                    acc[r] += (int)__ldg(&w[(size_t)x * nelem + k * j.in_w + i]);
+                }
+#pragma unroll
+        for (int r = 0; r < 4; r++) tile[tx][ty * 4 + r] = (float)((acc[r] - bg) / j.ave);
+    }
+    __syncthreads();
+    for (int r = 0; r < 4; r++) {
+        const int tl = ty * 4 + r, tr = blockIdx.x * 32 + tl, x = xbase + tx;
+        if (tr < j.ntrace && x < j.nopit) trace_out[(size_t)tr * j.nopit + x] = tile[tl][tx];
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Polynomial bleach fit: least squares in the Legendre basis of
 // u = t * uscale + uoff (t = averaged-trace time), coefficients = proj * y
@@ -665,83 +756,98 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
 // window that contains one gives a NaN monitor, so exactly the lags whose
 // windows hold a bad frame become non-finite, as calculateCF's sums do
 // (java:9484-9491).
-__global__ void monitor_finalize_kernel(Job j, const LagInfo *li, const float *bparams,
+// Bound by FP64 issue (1/64 of the FP32 rate): conversions on the integer
+// pipe, the divisions by the product counts from their reciprocals in the lag
+// table, the counts of non-finite frames as integers (0.31 -> 0.13 ms at
+// 16,384 pixels x 50,000 frames).
+
+// x / n, correctly rounded, from inv = 1 / n correctly rounded (n a small
+// whole number): the quotient's remainder corrects it (Markstein).  The means
+// of unbleached recordings are ratios of short numbers that sit on FP32
+// rounding ties, so x * inv alone would round some of them the other way.
+__device__ __forceinline__ double div_by(double x, double n, double inv)
+{
+    const double q = x * inv;
+    return fma(fma(-q, n, x), inv, q);
+}
+__global__ void __launch_bounds__(128) monitor_finalize_kernel(Job j, const LagInfo *li, const float *bparams,
                                         int nseg, const float2 *segtot, const float2 *snap_part,
                                         const int *segbad, const int *snap_bad, float4 *mon, float4 *blkmon)
 {
     extern __shared__ double sh[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int pix = blockIdx.x * (blockDim.x >> 5) + wid;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int pix = blockIdx.x * nw + wid;
     if (pix >= j.npix) return;
-    double *scan = sh + (size_t)wid * (nseg + 1 + 4 * j.nsnap);
+    double *scan = sh + (size_t)wid * (nseg + 1 + 2 * j.nsnap);
     double *pre0 = scan + nseg + 1;
     double *pre1 = pre0 + j.nsnap;
-    double *bad0 = pre1 + j.nsnap;      // prefix counts of non-finite frames
-    double *bad1 = bad0 + j.nsnap;
+    // the same for the counts of non-finite frames
+    int *bscan = (int *)(sh + (size_t)nw * (nseg + 1 + 2 * j.nsnap)) + (size_t)wid * (nseg + 1 + 2 * j.nsnap);
+    int *bad0 = bscan + nseg + 1, *bad1 = bad0 + j.nsnap;
     for (int which = 0; which < (j.is_ccf ? 2 : 1); which++) {
-        int tr = which ? j.npix + pix : pix;
+        const size_t tr = which ? j.npix + pix : pix;
         double *pre = which ? pre1 : pre0;
-        double *bpre = which ? bad1 : bad0;
-        // exclusive scans of the segment totals (pass 0) and of the
-        // non-finite frame counts (pass 1), then the snapshot prefixes
-        for (int pass = 0; pass < 2; pass++) {
-            double carry = 0.0;
-            for (int s0 = 0; s0 < nseg; s0 += 32) {
-                int s = s0 + lane;
-                double v = 0.0;
-                if (s < nseg) {
-                    if (pass == 0) { float2 t = segtot[(size_t)tr * nseg + s]; v = (double)t.x + (double)t.y; }
-                    else v = (double)segbad[(size_t)tr * nseg + s];
-                }
-                double incl = v;
-                for (int o = 1; o < 32; o <<= 1) {
-                    double u = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += u;
-                }
-                if (s < nseg) scan[s] = carry + incl - v;
-                carry += __shfl_sync(0xffffffffu, incl, 31);
+        int *bpre = which ? bad1 : bad0;
+        // exclusive scans of the segment totals and counts, then the snapshot prefixes
+        double carry = 0.0;
+        int bcarry = 0;
+        for (int s0 = 0; s0 < nseg; s0 += 32) {
+            const int s = s0 + lane;
+            double v = 0.0;
+            int bv = 0;
+            if (s < nseg) {
+                const float2 t = __ldg(&segtot[tr * nseg + s]);
+                v = f2d(t.x) + f2d(t.y);
+                bv = __ldg(&segbad[tr * nseg + s]);
             }
-            if (lane == 0) scan[nseg] = carry;
-            __syncwarp();
-            for (int sj = lane; sj < j.nsnap; sj += 32) {
-                int p = li->snap_pos[sj];
-                double v = 0.0;
-                if (p > 0) {
-                    int seg = (p - 1) / kSeg;
-                    if (pass == 0) {
-                        float2 t = snap_part[(size_t)tr * j.nsnap + sj];
-                        v = scan[seg] + (double)t.x + (double)t.y;
-                    } else {
-                        v = scan[seg] + (double)snap_bad[(size_t)tr * j.nsnap + sj];
-                    }
-                }
-                (pass == 0 ? pre : bpre)[sj] = v;
+            double incl = v;
+            int bincl = bv;
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u = __shfl_up_sync(0xffffffffu, incl, o);
+                const int bu = __shfl_up_sync(0xffffffffu, bincl, o);
+                if (lane >= o) { incl += u; bincl += bu; }
             }
-            __syncwarp();
+            if (s < nseg) { scan[s] = carry + incl - v; bscan[s] = bcarry + bincl - bv; }
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+            bcarry += __shfl_sync(0xffffffffu, bincl, 31);
         }
+        __syncwarp();
+        for (int sj = lane; sj < j.nsnap; sj += 32) {
+            const int p = li->snap_pos[sj];
+            double v = 0.0;
+            int bv = 0;
+            if (p > 0) {
+                const int seg = (p - 1) / kSeg;
+                const float2 t = __ldg(&snap_part[tr * j.nsnap + sj]);
+                v = scan[seg] + f2d(t.x) + f2d(t.y);
+                bv = bscan[seg] + __ldg(&snap_bad[tr * j.nsnap + sj]);
+            }
+            pre[sj] = v;
+            bpre[sj] = bv;
+        }
+        __syncwarp();
     }
-    if (!j.is_ccf)
-        for (int sj = lane; sj < j.nsnap; sj += 32) { pre1[sj] = pre0[sj]; bad1[sj] = bad0[sj]; }
-    __syncwarp();
-    const double c0 = bparams[(size_t)pix * kBleachStride + 12];
-    const double c1 = bparams[(size_t)(j.is_ccf ? j.npix + pix : pix) * kBleachStride + 12];
+    if (!j.is_ccf) { pre1 = pre0; bad1 = bad0; }
+    const double c0 = f2d(bparams[(size_t)pix * kBleachStride + 12]);
+    const double c1 = f2d(bparams[(size_t)(j.is_ccf ? j.npix + pix : pix) * kBleachStride + 12]);
+    const float qnan = __int_as_float(0x7fc00000);
     for (int x = lane; x < j.chanum; x += 32) {
-        int k = li->level[x];
-        double n = li->prodnum[x];
-        double a = pre0[li->snap_dir_end[x]] / n;
-        double b = (pre1[li->snap_del_end[x]] - pre1[li->snap_del_beg[x]]) / n;
-        if (bad0[li->snap_dir_end[x]] > 0.0) a = nan("");
-        if (bad1[li->snap_del_end[x]] - bad1[li->snap_del_beg[x]] > 0.0) b = nan("");
-        double sc = (double)(1 << k);
-        mon[(size_t)pix * j.chanum + x] =
-            make_float4((float)a, (float)b, (float)(a + sc * c0), (float)(b + sc * c1));
+        const int k = li->level[x];
+        const double n = li->prodnum[x], in = li->inv_prodnum[x];
+        const int de = li->snap_dir_end[x], lb = li->snap_del_beg[x], le = li->snap_del_end[x];
+        const double a = div_by(pre0[de], n, in), b = div_by(pre1[le] - pre1[lb], n, in);
+        const double sc = __hiloint2double((1023 + k) << 20, 0);        // 2^k
+        float4 m = make_float4((float)a, (float)b, (float)fma(sc, c0, a), (float)fma(sc, c1, b));
+        if (bad0[de] > 0) m.x = m.z = qnan;
+        if (bad1[le] - bad1[lb] > 0) m.y = m.w = qnan;
+        mon[(size_t)pix * j.chanum + x] = m;
     }
     if (lane == 0) {
-        double T1 = j.num - 1;
-        double dm1 = (pre0[li->snap_tm2] + (j.num - 2) * c0) / T1;   // zero-led direct window
-        double Dm1 = (pre1[li->snap_tm1] + (j.num - 1) * c1) / T1;
-        if (bad0[li->snap_tm2] > 0.0) dm1 = nan("");
-        if (bad1[li->snap_tm1] > 0.0) Dm1 = nan("");
+        const double T1 = j.num - 1, iT1 = li->blk_inv_n[0];
+        double dm1 = div_by(fma((double)(j.num - 2), c0, pre0[li->snap_tm2]), T1, iT1);   // zero-led direct window
+        double Dm1 = div_by(fma((double)(j.num - 1), c1, pre1[li->snap_tm1]), T1, iT1);
+        if (bad0[li->snap_tm2] > 0) dm1 = nan("");
+        if (bad1[li->snap_tm1] > 0) Dm1 = nan("");
         blkmon[pix] = make_float4((float)(dm1 - c0), (float)(Dm1 - c1), (float)dm1, (float)Dm1);
     }
 }
@@ -755,6 +861,20 @@ __global__ void monitor_finalize_kernel(Job j, const LagInfo *li, const float *b
 // and squared block means of the complete blocks inside its segment, and the
 // segment sum for the higher levels.
 // ---------------------------------------------------------------------------
+// One product into a level-0 sum pair, one block into a level's.
+__device__ __forceinline__ void blk_add(float &S1, float &S2, float m)
+{
+    S1 = __fadd_rn(S1, m);
+    S2 = fmaf(m, m, S2);
+}
+
+// A whole segment is sixteen steps of sixteen products: levels 1 to 4 are
+// sums inside a step, levels 5 to 8 are carried between steps (the same
+// branches for every thread).  Run-time carries for every product took 58
+// instructions each; HBM-bound now (4 B a frame-pixel): 1.45 -> 0.59 ms at
+// 16,384 pixels x 50,000 frames.  Four segments a thread, to halve the
+// statistics written, gained nothing (0.62 + 0.18 against 0.59 + 0.22 ms).
+template <bool CCF>
 __global__ void __launch_bounds__(128) block_kernel(Job j, const float *s0a, const float *s0b,
                                                     const float4 *blkmon, int nbseg, float *s1, float *s2,
                                                     float *segsum)
@@ -762,7 +882,6 @@ __global__ void __launch_bounds__(128) block_kernel(Job j, const float *s0a, con
     const int pix = blockIdx.x * blockDim.x + threadIdx.x;
     const int seg = blockIdx.y;
     if (pix >= j.npix) return;
-    const float *sb = j.is_ccf ? s0b : s0a;
     const float4 bm = blkmon[pix];   // a1 = dm1 - c0, b1 = Dm1 - c1, dm1, Dm1
     const int nprod = j.num - 1;
     const int j0 = seg * kBlkSeg, j1 = min(j0 + kBlkSeg, nprod);
@@ -771,46 +890,77 @@ __global__ void __launch_bounds__(128) block_kernel(Job j, const float *s0a, con
     for (int y = 0; y <= kBlkSegLog; y++) { S1[y] = 0.f; S2[y] = 0.f; pend[y] = 0.f; }
     // direct element of product jj is J_jj = v_{jj-1} (J_0 = 0); s0 holds the
     // corrected values centred on c, so J - dm1 = s0 - (dm1 - c)
-    float u_prev = (j0 == 0) ? -bm.z : __ldg(&s0a[(size_t)(j0 - 1) * j.npix + pix]) - bm.x;
+    const float *pa = s0a + (size_t)j0 * j.npix + pix, *pb = s0b + (size_t)j0 * j.npix + pix;
+    float u_prev = (j0 == 0) ? -bm.z : __ldg(pa - j.npix) - bm.x;
     float segv = 0.f;
-    for (int tb = j0; tb < j1; tb += 8) {
-        float va[8], vb[8];
+    int t = j0;
+    constexpr int kStep = 16, kStepLog = 4;
+#pragma unroll 1
+    for (; t + kStep <= j1; t += kStep) {
+        float v[kStep], w[kStep];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const bool in = tb + u < j1;
-            va[u] = in ? __ldg(&s0a[(size_t)(tb + u) * j.npix + pix]) : 0.f;
-            vb[u] = (in && j.is_ccf) ? __ldg(&sb[(size_t)(tb + u) * j.npix + pix]) : va[u];
+        for (int u = 0; u < kStep; u++) {
+            v[u] = __ldg(&pa[(size_t)u * j.npix]);
+            w[u] = CCF ? __ldg(&pb[(size_t)u * j.npix]) : v[u];
+        }
+        pa += (size_t)kStep * j.npix;
+        pb += (size_t)kStep * j.npix;
+#pragma unroll
+        for (int u = 0; u < kStep; u++) {
+            const float p = __fmul_rn(u_prev, w[u] - bm.y);
+            u_prev = v[u] - bm.x;    // next direct element J_{t+u+1} = v_{t+u}
+            blk_add(S1[0], S2[0], p);
+            v[u] = p;
         }
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int jj = tb + u;
-            if (jj >= j1) break;
-            const float w = vb[u] - bm.y;
-            const float p = u_prev * w;
-            u_prev = va[u] - bm.x;   // next direct element J_{jj+1} = v_jj
-            const int rel = jj - j0;
-            S1[0] += p;
-            S2[0] += p * p;
-            // pairwise block means: level y+1 completes when bit y of rel is
-            // set; unrolled so that every array index is a constant (registers)
-            float v = p;
-            bool carry = true;
+        for (int y = 1; y <= kStepLog; y++)
 #pragma unroll
-            for (int y = 0; y < kBlkSegLog; y++) {
-                if (carry) {
-                    if ((rel >> y) & 1) {
-                        v = pend[y] + v;
-                        const float m = v * (1.f / (float)(1 << (y + 1)));
-                        S1[y + 1] += m;
-                        S2[y + 1] += m * m;
-                    } else {
-                        pend[y] = v;
-                        carry = false;
-                    }
+            for (int i = 0; i < (kStep >> y); i++) {
+                v[i] = __fadd_rn(v[2 * i], v[2 * i + 1]);
+                blk_add(S1[y], S2[y], v[i] * (1.f / (float)(1 << y)));
+            }
+        float c = v[0];
+        const int rel = (t - j0) >> kStepLog;
+        bool carry = true;
+#pragma unroll
+        for (int y = kStepLog; y < kBlkSegLog; y++) {
+            if (carry) {
+                if ((rel >> (y - kStepLog)) & 1) {
+                    c = __fadd_rn(pend[y], c);
+                    blk_add(S1[y + 1], S2[y + 1], c * (1.f / (float)(1 << (y + 1))));
+                } else {
+                    pend[y] = c;
+                    carry = false;
                 }
             }
-            if (carry) segv = v;
         }
+        if (carry) segv = c;
+    }
+    // the last segment's remaining products, one by one
+#pragma unroll 1
+    for (; t < j1; t++) {
+        const float va = __ldg(pa), vb = CCF ? __ldg(pb) : va;
+        pa += j.npix;
+        pb += j.npix;
+        const float p = __fmul_rn(u_prev, vb - bm.y);
+        u_prev = va - bm.x;
+        blk_add(S1[0], S2[0], p);
+        const int rel = t - j0;
+        float c = p;
+        bool carry = true;
+#pragma unroll
+        for (int y = 0; y < kBlkSegLog; y++) {
+            if (carry) {
+                if ((rel >> y) & 1) {
+                    c = __fadd_rn(pend[y], c);
+                    blk_add(S1[y + 1], S2[y + 1], c * (1.f / (float)(1 << (y + 1))));
+                } else {
+                    pend[y] = c;
+                    carry = false;
+                }
+            }
+        }
+        if (carry) segv = c;
     }
     // [level][segment][pixel]: coalesced here and in the finaliser
 #pragma unroll
@@ -822,92 +972,161 @@ __global__ void __launch_bounds__(128) block_kernel(Job j, const float *s0a, con
     segsum[(size_t)seg * j.npix + pix] = segv;     // used only for complete segments
 }
 
-// Blocking decision.  A CTA serves 32 pixels with 8 threads each: thread
-// (pixel, t) sums the segments' statistics of levels t, t + 8, ... in FP64
-// (coalesced across pixels; each level's sum in segment order), the levels
-// above the segment size from segment sums; then one thread per pixel
-// applies the overlap / monotonic-increase criteria of java:9339-9380.
-constexpr int kBlkFinPix = 32, kBlkFinLev = 8;
+// Blocking decision.  A CTA serves 32 pixels with 16 threads each: thread
+// (pixel, y) sums the segments' statistics of level y (and y + 16) in
+// float-float (coalesced across pixels, in segment order), the levels above
+// the segment size from segment sums, and takes the level's standard deviation
+// in FP64; then one thread per pixel applies the overlap / monotonic-increase
+// criteria of java:9339-9380.  FP64 sums by 8 threads a pixel: 0.39 ms at
+// 16,384 pixels x 50,000 frames, this 0.06.
+constexpr int kBlkFinPix = 32, kBlkFinLev = 16;
+
+// f(value, value) over n pairs `stride` apart, the loads of U at a time.
+template <int U, bool TWO, class F>
+__device__ __forceinline__ void blk_walk(const float *p1, const float *p2, size_t stride, int n, F f)
+{
+    int i = 0;
+    for (; i + U <= n; i += U) {
+        float v[U], w[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            v[u] = __ldg(&p1[u * stride]);
+            w[u] = TWO ? __ldg(&p2[u * stride]) : 0.f;
+        }
+        p1 += U * stride;
+        p2 += U * stride;
+#pragma unroll
+        for (int u = 0; u < U; u++) f(v[u], w[u]);
+    }
+    for (; i < n; i++) {
+        f(__ldg(p1), TWO ? __ldg(p2) : 0.f);
+        p1 += stride;
+        p2 += stride;
+    }
+}
+
+// Sums a1, a2 of the means and squared means of nb blocks of S * parts segment
+// sums each (inv: 1 / products of a block), loads of 16 at a time: whole
+// blocks where S < 16.
+template <int S>
+__device__ __forceinline__ void blk_upper(const float *p, size_t stride, int nb, int parts, float inv, ff &a1, ff &a2)
+{
+    constexpr int G = 16 / S;             // blocks per batch
+    auto block = [&](const ff &sb) {
+        // the block's mean m (exact scaling) and its square
+        const f2 m = f2_quick(sb.hi * inv, sb.lo * inv), m2 = f2_mul(m, m);
+        ff_add(a1, m.hi);
+        ff_add(a2, m2.hi);
+        a1.lo = __fadd_rn(a1.lo, m.lo);
+        a2.lo = __fadd_rn(a2.lo, m2.lo);
+    };
+    for (int b = 0; b < nb; b += G) {
+        ff sb[G];
+#pragma unroll
+        for (int g = 0; g < G; g++) sb[g] = {0.f, 0.f};
+        for (int q = 0; q < parts; q++, p += 16 * stride) {
+            float v[16];
+#pragma unroll
+            for (int u = 0; u < 16; u++) v[u] = b + u / S < nb ? __ldg(&p[u * stride]) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 16; u++) ff_add(sb[u / S], v[u]);
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++)
+            if (b + g < nb) block(sb[g]);
+    }
+}
+
+// The same sums of level y in FP64, for statistics that left the FP32 range.
+static __device__ __noinline__ void blk_plain_sums(const float *s1, const float *s2, const float *segsum, int y,
+                                                   int nbseg, int full_segs, size_t npix, int pix, double &A1,
+                                                   double &A2)
+{
+    A1 = A2 = 0.0;
+    if (y <= kBlkSegLog) {
+        for (int seg = 0; seg < nbseg; seg++) {
+            A1 += (double)s1[((size_t)y * nbseg + seg) * npix + pix];
+            A2 += (double)s2[((size_t)y * nbseg + seg) * npix + pix];
+        }
+        return;
+    }
+    const int span = 1 << (y - kBlkSegLog);
+    for (int seg = 0; seg + span <= full_segs; seg += span) {
+        double sb = 0.0;
+        for (int k = 0; k < span; k++) sb += (double)segsum[(size_t)(seg + k) * npix + pix];
+        sb /= (double)(1 << y);
+        A1 += sb;
+        A2 += sb * sb;
+    }
+}
+
 __global__ void __launch_bounds__(kBlkFinPix * kBlkFinLev)
-block_finalize_kernel(Job j, int q, int nbseg, const float *s1, const float *s2, const float *segsum,
+block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s1, const float *s2, const float *segsum,
                       const float4 *blkmon, int *ind_out, int *ok_out)
 {
-    __shared__ double S1s[kMaxBlockLevels][kBlkFinPix], S2s[kMaxBlockLevels][kBlkFinPix];
+    __shared__ double vb[kMaxBlockLevels][kBlkFinPix];
     const int pl = threadIdx.x % kBlkFinPix, ty = threadIdx.x / kBlkFinPix;
     const int pix = blockIdx.x * kBlkFinPix + pl;
     const int blocknum = j.blocknum;
     const int full_segs = (j.num - 1) / kBlkSeg;   // segments holding kBlkSeg products
-    if (pix < j.npix) {
+    if (pix < j.npix && ty < blocknum) {
+        const float4 bm = blkmon[pix];
+        const double iq = newton_rcp(f2d(bm.z) * f2d(bm.w));
+        const double iq2 = iq * iq;
         for (int y = ty; y < blocknum; y += kBlkFinLev) {
-            double a1 = 0.0, a2 = 0.0;
+            if (bm.x != bm.x || bm.y != bm.y) {     // a non-finite frame: every product is non-finite
+                vb[y][pl] = __longlong_as_double(0x7ff8000000000000ll);
+                continue;
+            }
+            ff a1 = {0.f, 0.f}, a2 = {0.f, 0.f};
             if (y <= kBlkSegLog) {
-                const float *p1 = s1 + (size_t)y * nbseg * j.npix + pix, *p2 = s2 + (size_t)y * nbseg * j.npix + pix;
-                for (int seg = 0; seg < nbseg; seg++) {
-                    a1 += (double)__ldg(&p1[(size_t)seg * j.npix]);
-                    a2 += (double)__ldg(&p2[(size_t)seg * j.npix]);
-                }
+                const size_t o = (size_t)y * nbseg * j.npix + pix;
+                blk_walk<16, true>(s1 + o, s2 + o, j.npix, nbseg, [&](float v, float w) {
+                    ff_add(a1, v);
+                    ff_add(a2, w);
+                });
             } else {
                 // levels above the segment: block y spans 2^(y-8) consecutive
                 // complete segments (a non-finite segment sum, from a
                 // non-finite frame, propagates like the Java sums)
-                const int span = 1 << (y - kBlkSegLog);
-                const double inv = 1.0 / (double)(1 << y);
-                for (int b = 0; (b + 1) * span <= full_segs; b++) {
-                    double sb = 0.0;
-                    for (int k = 0; k < span; k++) sb += (double)__ldg(&segsum[(size_t)(b * span + k) * j.npix + pix]);
-                    const double m = sb * inv;
-                    a1 += m;
-                    a2 += m * m;
-                }
+                const int span = 1 << (y - kBlkSegLog), nb = full_segs / span;
+                const float inv = 1.f / (float)(1 << y);
+                const float *p = segsum + pix;
+                if (span == 2) blk_upper<2>(p, j.npix, nb, 1, inv, a1, a2);
+                else if (span == 4) blk_upper<4>(p, j.npix, nb, 1, inv, a1, a2);
+                else if (span == 8) blk_upper<8>(p, j.npix, nb, 1, inv, a1, a2);
+                else blk_upper<16>(p, j.npix, nb, span / 16, inv, a1, a2);
             }
-            S1s[y][pl] = a1;
-            S2s[y][pl] = a2;
+            double A1 = f2d(a1.hi) + f2d(a1.lo), A2 = f2d(a2.hi) + f2d(a2.lo);
+            if (!(isfinite(a1.hi) && isfinite(a2.hi)))
+                blk_plain_sums(s1, s2, segsum, y, nbseg, full_segs, j.npix, pix, A1, A2);
+            const double in = li->blk_inv_n[y];
+            const double m1 = A1 * in, m2 = A2 * in;
+            vb[y][pl] = newton_sqrt((m2 - m1 * m1) * in * iq2);
         }
     }
     __syncthreads();
     if (ty != 0 || pix >= j.npix) return;
-    double S1[kMaxBlockLevels], S2[kMaxBlockLevels];
-    for (int y = 0; y < blocknum; y++) {
-        S1[y] = S1s[y][pl];
-        S2[y] = S2s[y][pl];
+    // criteria as bit masks over the levels: error bars of neighbours overlap
+    // (crt), the deviation grows (pos)
+    unsigned crt = 0, pos = 0;
+    double v0 = vb[0][pl], e0 = v0 * li->blk_err[0];
+    for (int x = 0; x + 1 < blocknum; x++) {
+        const double v1 = vb[x + 1][pl], e1 = v1 * li->blk_err[x + 1];
+        if (v0 + e0 > v1 - e1 && v1 + e1 > v0 - e0) crt |= 1u << x;
+        if (v1 - v0 > 0) pos |= 1u << x;
+        v0 = v1;
+        e0 = e1;
     }
-    const float4 bm = blkmon[pix];
-    const double dmDm = (double)bm.z * (double)bm.w;
-    const int nprod = j.num - 1;
-    double vb1[kMaxBlockLevels], upper[kMaxBlockLevels], lower[kMaxBlockLevels];
-    int crt[kMaxBlockLevels] = {0}, cr12[kMaxBlockLevels] = {0}, cr3[kMaxBlockLevels] = {0},
-        diffpos[kMaxBlockLevels] = {0};
-    for (int y = 0; y < blocknum; y++) {
-        double n = (double)(nprod >> y);
-        double v = (S2[y] / n - (S1[y] / n) * (S1[y] / n)) / (n * dmDm * dmDm);
-        vb1[y] = sqrt(v);
-        double e = vb1[y] / sqrt(2 * (n - 1));
-        upper[y] = vb1[y] + e;
-        lower[y] = vb1[y] - e;
-    }
-    for (int x = 0; x < blocknum - 1; x++)
-        if (upper[x] > lower[x + 1] && upper[x + 1] > lower[x]) crt[x] = 1;
-    for (int x = 0; x < blocknum - 2; x++)
-        if (crt[x] * crt[x + 1] == 1) cr12[x] = 1;
-    for (int x = 0; x < blocknum - 1; x++)
-        if (vb1[x + 1] - vb1[x] > 0) diffpos[x] = 1;
-    for (int x = 0; x < blocknum - 2; x++)
-        if (diffpos[x] * diffpos[x + 1] == 1) cr3[x] = 1;
-    int last0 = 0;
-    for (int x = 0; x < blocknum - 2; x++)
-        if (cr3[x] == 1 && cr12[x] == 0) last0 = x;
-    for (int x = 0; x <= last0; x++) cr12[x] = 0;
-    if (blocknum >= 3) cr12[blocknum - 3] = 0;
-    if (blocknum >= 4) cr12[blocknum - 4] = 0;
-    int ind = 0, ok;
-    for (int x = blocknum - 5; x > 0; x--)
-        if (cr12[x] == 1) ind = x + 1;
-    if (ind == 0) {
-        ok = 0;
-        ind = (blocknum - 3 > 0) ? blocknum - 3 : blocknum - 1;
-    } else {
-        ok = 1;
-    }
+    const unsigned below = (1u << (blocknum - 2)) - 1;
+    unsigned cr12 = crt & (crt >> 1) & below;
+    const unsigned rise = pos & (pos >> 1) & below & ~cr12;
+    const int last0 = rise ? 31 - __clz(rise) : 0;
+    cr12 &= ~((2u << last0) - 1);
+    cr12 &= ~(3u << (blocknum - 4));
+    cr12 &= (1u << (blocknum - 4)) - 2;              // levels 1 .. blocknum - 5
+    const int ok = cr12 != 0;
+    int ind = ok ? __ffs(cr12) : (blocknum - 3 > 0 ? blocknum - 3 : blocknum - 1);
     if (ind < q - 1) ind = q - 1;
     ind_out[pix] = ind;
     ok_out[pix] = ok;
@@ -976,9 +1195,45 @@ template __global__ void bleach_exp_kernel<5>(Job, const float *, float *);
 
 namespace imfcs {
 
-cudaError_t launch_trace(const Job &j, const void *stack, float *trace, cudaStream_t s)
+// Raw rows the traces read: the first one, and the elements per frame of
+// trace_sums_kernel's output (0: the one-pass kernel).  A region narrower
+// than half the frame would have the two-pass form read columns nobody wants.
+static void trace_rows(const Job &j, int &row0, size_t &nelem)
+{
+    row0 = j.map_y0 * j.pixbiny + (j.cfy < 0 ? j.cfy : 0);
+    const int row1 = (j.map_y0 + j.out_h - 1) * j.pixbiny + j.biny + (j.cfy > 0 ? j.cfy : 0);
+    const int cols = (j.out_w - 1) * j.pixbinx + j.binx + (j.cfx < 0 ? -j.cfx : j.cfx);
+    nelem = j.input_float || 2 * cols < j.in_w ? 0 : (size_t)(row1 - row0) * j.in_w;
+    if (nelem > (1u << 30)) nelem = 0;
+}
+
+size_t trace_sums_elems(const Job &j)
+{
+    int row0;
+    size_t nelem;
+    trace_rows(j, row0, nelem);
+    return nelem * j.nopit;
+}
+
+cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float *trace, cudaStream_t s)
 {
     dim3 grid((j.ntrace + 31) / 32, (j.nopit + 31) / 32), block(32, 8);
+    int row0;
+    size_t nelem;
+    trace_rows(j, row0, nelem);
+    if (nelem) {
+        const size_t fsz = (size_t)j.in_w * j.in_h;
+        const uint16_t *base = (const uint16_t *)stack + (size_t)j.first * fsz + (size_t)row0 * j.in_w;
+        const int n = (int)nelem;
+        auto grid1 = [&](int vec) { return dim3((n / vec + 127) / 128, j.nopit); };
+        if ((uintptr_t)base % 16 == 0 && fsz % 8 == 0 && n % 8 == 0)
+            trace_sums_kernel<8><<<grid1(8), 128, 0, s>>>(base, fsz, n, j.ave, sums);
+        else if ((uintptr_t)base % 4 == 0 && fsz % 2 == 0 && n % 2 == 0)
+            trace_sums_kernel<2><<<grid1(2), 128, 0, s>>>(base, fsz, n, j.ave, sums);
+        else trace_sums_kernel<1><<<grid1(1), 128, 0, s>>>(base, fsz, n, j.ave, sums);
+        trace_windows_kernel<<<grid, block, 0, s>>>(j, sums, row0, n, trace);
+        return cudaGetLastError();
+    }
     trace_kernel<<<grid, block, 0, s>>>(j, stack, trace);
     return cudaGetLastError();
 }
@@ -1016,7 +1271,7 @@ cudaError_t launch_monitor_finalize(const Job &j, const LagInfo *li_dev, const f
                                     const int *snap_bad, float4 *mon, float4 *blkmon, cudaStream_t s)
 {
     const int wpb = 4;
-    size_t smem = (size_t)wpb * (nseg + 1 + 4 * j.nsnap) * sizeof(double);
+    size_t smem = (size_t)wpb * (nseg + 1 + 2 * j.nsnap) * (sizeof(double) + sizeof(int));
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(monitor_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     monitor_finalize_kernel<<<(j.npix + wpb - 1) / wpb, wpb * 32, smem, s>>>(j, li_dev, bparams, nseg, segtot,
@@ -1025,16 +1280,17 @@ cudaError_t launch_monitor_finalize(const Job &j, const LagInfo *li_dev, const f
     return cudaGetLastError();
 }
 
-cudaError_t launch_block(const Job &j, const float *s0, const float4 *blkmon, int nbseg, float *s1, float *s2,
+cudaError_t launch_block(const Job &j, const LagInfo *li, const float *s0, const float4 *blkmon, int nbseg, float *s1, float *s2,
                          float *segsum, int *ind, int *ok, cudaStream_t s)
 {
     dim3 grid((j.npix + 127) / 128, nbseg);
     const float *s0b = j.is_ccf ? s0 + (size_t)j.npix * j.num : s0;
-    block_kernel<<<grid, 128, 0, s>>>(j, s0, s0b, blkmon, nbseg, s1, s2, segsum);
+    if (j.is_ccf) block_kernel<true><<<grid, 128, 0, s>>>(j, s0, s0b, blkmon, nbseg, s1, s2, segsum);
+    else block_kernel<false><<<grid, 128, 0, s>>>(j, s0, s0b, blkmon, nbseg, s1, s2, segsum);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     block_finalize_kernel<<<(j.npix + kBlkFinPix - 1) / kBlkFinPix, kBlkFinPix * kBlkFinLev, 0, s>>>(
-        j, j.q, nbseg, s1, s2, segsum, blkmon, ind, ok);
+        j, li, j.q, nbseg, s1, s2, segsum, blkmon, ind, ok);
     return cudaGetLastError();
 }
 
