@@ -19,13 +19,20 @@
 //   sum_z (e_x e_y / (sd_x sd_y) - r_xy)^2 = (S2_xy - (pnum - 2) c_xy^2) / (c_xx c_yy)
 // with c = S1 / (pnum - 1) and r = c / (sd_x sd_y).  Divisions by per-lag
 // quantities are multiplications by their reciprocals; the median is a
-// parallel rank selection; the FP64 Cholesky's updates spread over the whole
-// CTA on the packed lower triangle in shared memory.  GB300 issues FP64 at
-// 1/64 of the FP32 rate, so what needs more than FP32 but not the
-// FP64 Cholesky -- the centred samples, the sums across chunks,
-// L^-1 (one column per thread) and L^-1 mcov -- runs in float-float
+// parallel rank selection on the variances' bits; the FP64 Cholesky runs in
+// panels of 8 columns on the packed lower triangle in shared memory.  GB300
+// issues FP64 at 1/64 of the FP32 rate, so what needs more than FP32 but not
+// the FP64 Cholesky -- the centred samples, the sums across chunks,
+// L^-1 (one column per lane) and L^-1 mcov -- runs in float-float
 // (compensated products and sums, about 44 bits) on the FP32 pipe; L^-1
 // leaves the kernel as FP32.
+//
+// Bound by FP64 issue (6,200 FP64 warp instructions a pixel at 72 lags, 1.4 ms
+// of 2.2 at 4,096 pixels) and the factorisation's serial panels: 2.71 -> 2.21
+// ms by panels in one warp's registers instead of three barriers a column,
+// uniform loops for L^-1 and four CTAs per SM.  Shrinkage and regularisation
+// in float-float would save a tenth more, but L^-1 magnifies its last bits
+// past FP32 rounding and weakly determined fits take other steps.
 #include <math.h>
 
 #include "imfcs_internal.cuh"
@@ -34,9 +41,10 @@
 
 namespace imfcs {
 
-constexpr int kGlsThreads = 256;
-constexpr int kGlsZChunk = 80;                  // samples per staged chunk
-constexpr int kGlsZStride = kGlsZChunk + 1;     // odd row stride: rows in distinct banks
+constexpr int kGlsThreads = 192;                // 171 tiles of pairs at 72 lags
+constexpr int kGlsZChunk = 80;                  // samples summed in FP32 before float-float
+constexpr int kGlsZStage = 20;                  // samples staged at a time (four CTAs per SM)
+constexpr int kGlsZStride = kGlsZStage + 1;     // odd row stride: rows in distinct banks
 constexpr int kMaxN1 = 96;                      // chanum - 1 limit of this kernel
 constexpr int kGlsTile = 4;                     // pairs per thread: 4 x 4
 
@@ -57,36 +65,99 @@ __device__ __forceinline__ void ff_dot_step(float ah, float al, float bh, float 
     sh = t;
 }
 
-__global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
+// Columns k0 .. k0 + kPanel - 1 of the Cholesky factor, one warp: lane l holds
+// rows k0 + l, k0 + l + 32, ... of the panel.  Per pivot: 1/sqrt by
+// Newton-Raphson from an FP32 estimate (two steps: ~1e-16), sqrt(d) =
+// d / sqrt(d) corrected once, the column scaled, the panel's later columns
+// updated.  False where a pivot is not above commons-math's threshold.
+constexpr int kPanel = 8;
+constexpr int kPanelRows = (kMaxN1 + 31) / 32;
+__device__ __forceinline__ bool chol_panel(double *lp, int n1, int k0, double *rdiag, int lane)
+{
+    double a[kPanelRows][kPanel];
+#pragma unroll
+    for (int t = 0; t < kPanelRows; t++)
+#pragma unroll
+        for (int j = 0; j < kPanel; j++) {
+            const int r = k0 + lane + 32 * t;
+            a[t][j] = r < n1 && k0 + j <= r ? lp[tri(r, k0 + j)] : 0.0;
+        }
+#pragma unroll
+    for (int j = 0; j < kPanel; j++) {
+        if (k0 + j >= n1) break;
+        const double d = __shfl_sync(0xffffffffu, a[0][j], j);
+        if (!(d > 1e-10)) return false;
+        double rs, r;
+        if (d < 1e30) {
+            const double h = -0.5 * d;
+            rs = f2d(rsqrtf((float)d));
+            rs = rs * fma(h * rs, rs, 1.5);
+            rs = rs * fma(h * rs, rs, 1.5);
+            r = d * rs;
+            r = fma(0.5 * rs, fma(-r, r, d), r);
+        } else {
+            r = sqrt(d);
+            rs = 1.0 / r;
+        }
+        if (lane == j) rdiag[k0 + j] = rs;
+#pragma unroll
+        for (int t = 0; t < kPanelRows; t++) {
+            if (k0 + 32 * t >= n1) break;
+            a[t][j] = t == 0 && lane == j ? r : a[t][j] * rs;
+        }
+#pragma unroll
+        for (int c = j + 1; c < kPanel; c++) {
+            const double m = __shfl_sync(0xffffffffu, a[0][j], c);      // L[k0 + c][k0 + j]
+#pragma unroll
+            for (int t = 0; t < kPanelRows; t++) {
+                if (k0 + 32 * t >= n1) break;
+                a[t][c] = fma(-a[t][j], m, a[t][c]);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < kPanelRows; t++)
+#pragma unroll
+        for (int j = 0; j < kPanel; j++) {
+            const int r = k0 + lane + 32 * t;
+            if (r < n1 && k0 + j <= r) lp[tri(r, k0 + j)] = a[t][j];
+        }
+    return true;
+}
+
+__global__ void __launch_bounds__(kGlsThreads, 4) gls_kernel(GlsArgs g)
 {
     extern __shared__ double gsh[];
     const int n1 = g.chanum - 1;
     const int npairs = n1 * (n1 + 1) / 2;
     const int nrt = (n1 + kGlsTile - 1) / kGlsTile;    // tile rows
-    double *lp = gsh;                  // [npairs] covariance/correlation -> regularised -> Cholesky factor
-    double *s2 = gsh + npairs;         // [npairs] S2 -> t_xy
-    float2 *a1s = (float2 *)lp, *a2s = (float2 *)s2;   // S1, S2 in float-float during the sample pass
-    float *eb = (float *)(gsh + 2 * npairs);   // [nrt*4][kGlsZStride] one chunk of centred samples
-    float *lh = eb, *ll = eb + npairs;         // L in float-float (after the Cholesky)
-    float *xh = (float *)s2, *xl = xh + npairs;   // L^-1 in float-float
-    __shared__ double mcov[kMaxN1], inv_dm[kMaxN1], cdiag[kMaxN1], isd[kMaxN1], sq[kMaxN1], rdiag[kMaxN1];
+    // [npairs] each, 8 bytes a pair: S1 (float-float) -> covariance (FP64) ->
+    // correlation -> regularised covariance -> Cholesky factor (FP64, then
+    // float-float), and S2 (float-float) -> t_xy (FP64) -> L^-1 (float-float)
+    f2 *cf = (f2 *)gsh, *s2f = (f2 *)(gsh + npairs);
+    double *lp = gsh, *s2 = gsh + npairs;
+    float *eb = (float *)(gsh + 2 * npairs);   // [nrt*4][kGlsZStride] a stage of centred samples
+    __shared__ double cdiag[kMaxN1], isd[kMaxN1], sq[kMaxN1], rdiag[kMaxN1];
     __shared__ f2 inv_dmf[kMaxN1], mcovf[kMaxN1], rdf[kMaxN1];
     __shared__ double red[2][kGlsThreads / 32];
-    __shared__ double s_med[2], s_lamvar, s_lamcov, s_piv;
+    __shared__ double s_med[2], s_lamvar, s_lamcov, s_inv[2], s_f;
     __shared__ int s_fail;
 
     const int pix = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pnum = g.pnum_by_ind[g.blk_ind[pix]];
     const float *bp = g.bprod + (size_t)pix * n1 * g.pnum_stride;
-    const double inv_pm1 = 1.0 / (double)(pnum - 1), inv_pnum = 1.0 / (double)pnum;
     if (tid < n1) {
         const float4 m = g.mon[(size_t)pix * g.chanum + tid + 1];
-        inv_dm[tid] = 1.0 / ((double)m.z * (double)m.w);
-        inv_dmf[tid] = f2_from_d(inv_dm[tid]);
+        rdiag[tid] = 1.0 / (f2d(m.z) * f2d(m.w));
+        inv_dmf[tid] = f2_from_d(rdiag[tid]);
+    } else if (tid == kGlsThreads - 1) {               // a warp of its own
+        s_fail = 0;
+        s_inv[0] = 1.0 / (double)(pnum - 1);
+        s_inv[1] = 1.0 / (double)pnum;
+        s_f = (double)pnum / pow((double)pnum - 1.0, 3);
     }
-    if (tid == 0) s_fail = 0;
-    for (int i = tid; i < npairs; i += kGlsThreads) { lp[i] = 0.0; s2[i] = 0.0; }
+    for (int i = tid; i < npairs; i += kGlsThreads) cf[i] = s2f[i] = {0.f, 0.f};
     // rows past n1 of the staging buffer stay zero
     for (int i = n1 * kGlsZStride + tid; i < nrt * kGlsTile * kGlsZStride; i += kGlsThreads) eb[i] = 0.f;
     // mcov (java:9526-9531): sum of the blocked products (float-float per
@@ -103,13 +174,11 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
             const f2 other = {__shfl_xor_sync(0xffffffffu, sum.hi, o), __shfl_xor_sync(0xffffffffu, sum.lo, o)};
             sum = f2_add(sum, other);
         }
-        if (lane == 0) mcov[x] = (double)sum.hi + (double)sum.lo;
+        if (lane == 0) mcovf[x] = sum;
     }
-    __syncthreads();                  // inv_dm (threads < n1) and the sums (warps)
-    if (tid < n1) {
-        mcov[tid] = mcov[tid] * inv_dm[tid] * inv_pnum;
-        mcovf[tid] = f2_from_d(mcov[tid]);
-    }
+    __syncthreads();                  // 1 / dm Dm (threads < n1), the constants and the sums (warps)
+    const double inv_pm1 = s_inv[0], inv_pnum = s_inv[1];
+    if (tid < n1) mcovf[tid] = f2_from_d((f2d(mcovf[tid].hi) + f2d(mcovf[tid].lo)) * rdiag[tid] * inv_pnum);
     __syncthreads();
 
     // S1, S2 per pair: thread t owns tile (bx, by), bx >= by, of the pairs
@@ -125,53 +194,55 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
             by = t - bx * (bx + 1) / 2;
         }
         for (int z0 = 0; z0 < pnum; z0 += kGlsZChunk) {
-            const int zn = min(kGlsZChunk, pnum - z0);
-            __syncthreads();
-            // centred sample e = b / (dm Dm) - mcov in float-float: the
-            // product exactly as hi + lo, then the subtraction of the mean
-            for (int i = tid; i < n1 * kGlsZChunk; i += kGlsThreads) {
-                const int x = i / kGlsZChunk, z = i - x * kGlsZChunk;
-                if (z < zn) {
-                    const float b = bp[(size_t)x * g.pnum_stride + z0 + z];
-                    const f2 iv = inv_dmf[x], mc = mcovf[x];
-                    const float ph = __fmul_rn(b, iv.hi);
-                    const float pl = fmaf(b, iv.lo, fmaf(b, iv.hi, -ph));
-                    eb[x * kGlsZStride + z] = __fadd_rn(__fsub_rn(ph, mc.hi), __fsub_rn(pl, mc.lo));
-                }
-            }
-            __syncthreads();
-            if (t >= ntiles) continue;
             float a1[kGlsTile][kGlsTile], a2[kGlsTile][kGlsTile];
 #pragma unroll
             for (int i = 0; i < kGlsTile; i++)
 #pragma unroll
                 for (int j = 0; j < kGlsTile; j++) { a1[i][j] = 0.f; a2[i][j] = 0.f; }
-            const float *ex = eb + (kGlsTile * bx) * kGlsZStride, *ey = eb + (kGlsTile * by) * kGlsZStride;
-            for (int z = 0; z < zn; z++) {
-                float vx[kGlsTile], vy[kGlsTile];
-#pragma unroll
-                for (int i = 0; i < kGlsTile; i++) { vx[i] = ex[i * kGlsZStride + z]; vy[i] = ey[i * kGlsZStride + z]; }
-#pragma unroll
-                for (int i = 0; i < kGlsTile; i++)
-#pragma unroll
-                    for (int j = 0; j < kGlsTile; j++) {
-                        const float u = vx[i] * vy[j];
-                        a1[i][j] += u;
-                        a2[i][j] = fmaf(u, u, a2[i][j]);
+            for (int zs = z0; zs < min(z0 + kGlsZChunk, pnum); zs += kGlsZStage) {
+                const int zn = min(kGlsZStage, pnum - zs);
+                __syncthreads();
+                // centred sample e = b / (dm Dm) - mcov in float-float: the
+                // product exactly as hi + lo, then the subtraction of the mean
+                for (int i = tid; i < n1 * kGlsZStage; i += kGlsThreads) {
+                    const int x = i / kGlsZStage, z = i - x * kGlsZStage;
+                    if (z < zn) {
+                        const float b = bp[(size_t)x * g.pnum_stride + zs + z];
+                        const f2 iv = inv_dmf[x], mc = mcovf[x];
+                        const float ph = __fmul_rn(b, iv.hi);
+                        const float pl = fmaf(b, iv.lo, fmaf(b, iv.hi, -ph));
+                        eb[x * kGlsZStride + z] = __fadd_rn(__fsub_rn(ph, mc.hi), __fsub_rn(pl, mc.lo));
                     }
+                }
+                __syncthreads();
+                if (t >= ntiles) continue;
+                const float *ex = eb + (kGlsTile * bx) * kGlsZStride, *ey = eb + (kGlsTile * by) * kGlsZStride;
+                for (int z = 0; z < zn; z++) {
+                    float vx[kGlsTile], vy[kGlsTile];
+#pragma unroll
+                    for (int i = 0; i < kGlsTile; i++) { vx[i] = ex[i * kGlsZStride + z]; vy[i] = ey[i * kGlsZStride + z]; }
+#pragma unroll
+                    for (int i = 0; i < kGlsTile; i++)
+#pragma unroll
+                        for (int j = 0; j < kGlsTile; j++) {
+                            const float u = __fmul_rn(vx[i], vy[j]);
+                            a1[i][j] = __fadd_rn(a1[i][j], u);
+                            a2[i][j] = fmaf(u, u, a2[i][j]);
+                        }
+                }
             }
+            if (t >= ntiles) continue;
 #pragma unroll
             for (int i = 0; i < kGlsTile; i++)
 #pragma unroll
                 for (int j = 0; j < kGlsTile; j++) {
                     const int x = kGlsTile * bx + i, y = kGlsTile * by + j;
                     if (x < n1 && y <= x) {
-                        float2 v = a1s[tri(x, y)];
-                        f2 sv = f2_two_sum(v.x, a1[i][j]);
-                        a1s[tri(x, y)] = make_float2(sv.hi, __fadd_rn(v.y, sv.lo));
-                        v = a2s[tri(x, y)];
-                        sv = f2_two_sum(v.x, a2[i][j]);
-                        a2s[tri(x, y)] = make_float2(sv.hi, __fadd_rn(v.y, sv.lo));
+                        f2 v = cf[tri(x, y)], sv = f2_two_sum(v.hi, a1[i][j]);
+                        cf[tri(x, y)] = {sv.hi, __fadd_rn(v.lo, sv.lo)};
+                        v = s2f[tri(x, y)];
+                        sv = f2_two_sum(v.hi, a2[i][j]);
+                        s2f[tri(x, y)] = {sv.hi, __fadd_rn(v.lo, sv.lo)};
                     }
                 }
         }
@@ -179,9 +250,9 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
     __syncthreads();
     // covariance (java:9534-9542), S2 in FP64, standard deviations
     for (int i = tid; i < npairs; i += kGlsThreads) {
-        const float2 v = a1s[i], w = a2s[i];
-        lp[i] = ((double)v.x + (double)v.y) * inv_pm1;
-        s2[i] = (double)w.x + (double)w.y;
+        const f2 v = cf[i], w = s2f[i];
+        lp[i] = (f2d(v.hi) + f2d(v.lo)) * inv_pm1;
+        s2[i] = f2d(w.hi) + f2d(w.lo);
     }
     __syncthreads();
     if (tid < n1) {
@@ -193,19 +264,28 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
     // median of the chanum diagonal entries incl. the zero-lag slot that
     // stays 0 (java:9563-9573): rank selection, ties ordered by index
     if (tid <= n1) {
+        // (variances order like their bits: no FP64 comparison; a NaN, above
+        // all numbers here, compares with nothing and takes rank 0)
+        const long long above = 0x7fffffffffffffffll;
+        auto key_of = [&](int j) {
+            const double w = j == 0 ? 0.0 : cdiag[j - 1];
+            return w != w ? above : __double_as_longlong(w);
+        };
         const double v = tid == 0 ? 0.0 : cdiag[tid - 1];
+        const long long key = key_of(tid);
         int rank = 0;
         for (int j = 0; j <= n1; j++) {
-            const double w = j == 0 ? 0.0 : cdiag[j - 1];
-            rank += (w < v) || (w == v && j < tid);
+            const long long w = key_of(j);
+            rank += (w < key) || (w == key && j < tid);
         }
+        if (key == above) rank = 0;
         const int c = n1 + 1;
         const int pos1 = (c - 1) / 2, pos2 = c / 2;     // floor / ceil of (c - 1) / 2
         if (rank == pos1) s_med[0] = v;
         if (rank == pos2) s_med[1] = v;
     }
     // t_xy and correlations; lamvar's and lamcov's sums
-    const double f = (double)pnum / pow((double)pnum - 1.0, 3);
+    const double f = s_f;
     const double pm2 = (double)(pnum - 2);
     for (int i = tid; i < npairs; i += kGlsThreads) {
         int x = (int)((sqrtf(8.f * i + 1.f) - 1.f) * 0.5f);
@@ -291,45 +371,42 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
             const int x = i / n1, y = i - x * n1;
             g.covmats_out[(size_t)pix * n1 * n1 + i] = x >= y ? lp[tri(x, y)] : lp[tri(y, x)];
         }
-    // Cholesky in commons-math's order (java:13717): pivot i, scale its
-    // column, then the trailing update A[q][p] -= A[q][i] A[p][i] (p <= q),
-    // FP64.  The pivot's 1/sqrt by Newton-Raphson from an FP32 estimate
-    // (two steps: ~1e-16), sqrt(d) = d / sqrt(d) corrected once; the update
-    // spreads its (q, p) over the whole CTA.
-    for (int i = 0; i < n1; i++) {
-        if (tid == 0) {
-            const double d = lp[tri(i, i)];
-            if (!(d > 1e-10)) {
-                s_fail = 1;
-            } else {
-                double rs, r;
-                if (d < 1e30) {
-                    rs = (double)rsqrtf((float)d);
-                    rs = rs * fma(-0.5 * d * rs, rs, 1.5);
-                    rs = rs * fma(-0.5 * d * rs, rs, 1.5);
-                    r = d * rs;
-                    r = fma(0.5 * rs, fma(-r, r, d), r);
-                } else {
-                    r = sqrt(d);
-                    rs = 1.0 / r;
-                }
-                lp[tri(i, i)] = r;
-                s_piv = rs;
-                rdiag[i] = rs;
-            }
-        }
+    // Cholesky in panels of kPanel columns: warp 0 factors a panel in
+    // registers, then all warps subtract its columns' products from the rest
+    // (18 barriers instead of 216; a panel ahead, with the other warps at the
+    // columns behind, was no faster: warp 0 is the critical path).  Every
+    // element sees the pivots' updates A[q][p] -= A[q][i] A[p][i] in
+    // commons-math's order (java:13717).
+    for (int k0 = 0; k0 < n1; k0 += kPanel) {
+        if (warp == 0 && !chol_panel(lp, n1, k0, rdiag, lane) && lane == 0) s_fail = 1;
         __syncthreads();
         if (s_fail) break;
-        for (int q = i + 1 + tid; q < n1; q += kGlsThreads) lp[tri(q, i)] *= s_piv;
-        __syncthreads();
-        const int m = n1 - 1 - i;
-        const int cnt = m * (m + 1) / 2;
-        for (int e = tid; e < cnt; e += kGlsThreads) {
-            int a = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
-            while ((a + 1) * (a + 2) / 2 <= e) a++;
-            while (a * (a + 1) / 2 > e) a--;
-            const int q = i + 1 + a, pp = i + 1 + (e - a * (a + 1) / 2);
-            lp[tri(q, pp)] -= lp[tri(q, i)] * lp[tri(pp, i)];
+        // 2 x 2 elements per thread, q >= p, both past the panel
+        const int k1 = k0 + kPanel, half = n1 > k1 ? (n1 - k1 + 1) / 2 : 0;
+        for (int e = tid; e < half * (half + 1) / 2; e += kGlsThreads) {
+            int bq = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
+            while ((bq + 1) * (bq + 2) / 2 <= e) bq++;
+            while (bq * (bq + 1) / 2 > e) bq--;
+            const int q0 = k1 + 2 * bq, p0 = k1 + 2 * (e - bq * (bq + 1) / 2);
+            const bool two_q = q0 + 1 < n1, upper = p0 + 1 <= q0;   // rows q0 + 1; element (q0, p0 + 1)
+            const int rq0 = tri(q0, 0), rq1 = two_q ? tri(q0 + 1, 0) : rq0;
+            const int rp0 = tri(p0, 0), rp1 = p0 + 1 < n1 ? tri(p0 + 1, 0) : rp0;
+            double a00 = lp[rq0 + p0], a01 = upper ? lp[rq0 + p0 + 1] : 0.0;
+            double a10 = lp[rq1 + p0], a11 = two_q ? lp[rq1 + p0 + 1] : 0.0;
+#pragma unroll
+            for (int i = 0; i < kPanel; i++) {
+                const double x0 = lp[rq0 + k0 + i], x1 = lp[rq1 + k0 + i], y0 = lp[rp0 + k0 + i], y1 = lp[rp1 + k0 + i];
+                a00 = fma(-x0, y0, a00);
+                a01 = fma(-x0, y1, a01);
+                a10 = fma(-x1, y0, a10);
+                a11 = fma(-x1, y1, a11);
+            }
+            lp[rq0 + p0] = a00;
+            if (upper) lp[rq0 + p0 + 1] = a01;
+            if (two_q) {
+                lp[rq1 + p0] = a10;
+                lp[rq1 + p0 + 1] = a11;
+            }
         }
         __syncthreads();
     }
@@ -338,43 +415,57 @@ __global__ void __launch_bounds__(kGlsThreads) gls_kernel(GlsArgs g)
         return;
     }
     // L and 1/diag(L) in float-float for the triangular inverse on the FP32
-    // pipe (the output L^-1 is FP32)
-    for (int i = tid; i < npairs; i += kGlsThreads) {
-        const double v = lp[i];
-        const float hi = (float)v;
-        lh[i] = hi;
-        ll[i] = (float)(v - (double)hi);
-    }
+    // pipe (the output L^-1 is FP32), in the place of the FP64 factor
+    f2 *L = cf, *X = s2f;
+    for (int i = tid; i < npairs; i += kGlsThreads) L[i] = f2_from_d(lp[i]);
     if (tid < n1) rdf[tid] = f2_from_d(rdiag[tid]);
     __syncthreads();
-    // L^-1, column c on thread c: X[c][c] = 1/L[c][c],
-    // X[r][c] = -(sum_{m=c}^{r-1} L[r][m] X[m][c]) / L[r][r]
-    if (tid < n1) {
-        const int c = tid;
-        xh[tri(c, c)] = rdf[c].hi;
-        xl[tri(c, c)] = rdf[c].lo;
-        for (int r = c + 1; r < n1; r++) {
-            const int rb = tri(r, 0);
+    // L^-1, column c on lane c of a warp's 32 columns: X[c][c] = 1/L[c][c],
+    // X[r][c] = -(sum_{m=c}^{r-1} L[r][m] X[m][c]) / L[r][r].  All lanes are at
+    // the same (r, m) -- L is a broadcast, a row of X consecutive -- and take
+    // zeros up to their column (with r starting at each lane's own column
+    // both loads were spread over the banks, and bound the kernel).
+    if (tid < ((n1 + 31) & ~31)) {
+        const int c = tid, c0 = tid & ~31;
+        for (int r = c0; r < n1; r++) {
             float sh = 0.f, sl = 0.f;
-            int xi = tri(c, c);
-            for (int m = c; m < r; m++) {
-                ff_dot_step(lh[rb + m], ll[rb + m], xh[xi], xl[xi], sh, sl);
-                xi += m + 1;
+            const f2 *Lr = L + tri(r, 0), *Xc = X + tri(c0, 0) + c;
+            int m = c0;
+            for (; m < min(r, c0 + 32); m++) {          // the warp's own columns: zeros above the diagonal
+                const f2 x = c <= m ? *Xc : f2{0.f, 0.f};
+                Xc += m + 1;
+                ff_dot_step(Lr[m].hi, Lr[m].lo, x.hi, x.lo, sh, sl);
             }
-            const f2 x = f2_mul(f2_two_sum(sh, sl), rdf[r]);
-            xh[tri(r, c)] = -x.hi;
-            xl[tri(r, c)] = -x.lo;
+            for (; m + 8 <= r; m += 8) {
+                f2 xv[8], lv[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    xv[u] = Xc[u * m + u * (u + 1) / 2];
+                    lv[u] = Lr[m + u];
+                }
+                Xc += 8 * m + 36;
+#pragma unroll
+                for (int u = 0; u < 8; u++) ff_dot_step(lv[u].hi, lv[u].lo, xv[u].hi, xv[u].lo, sh, sl);
+            }
+            for (; m < r; m++) {
+                const f2 x = *Xc;
+                Xc += m + 1;
+                ff_dot_step(Lr[m].hi, Lr[m].lo, x.hi, x.lo, sh, sl);
+            }
+            if (c < r) X[tri(r, c)] = f2_neg(f2_mul(f2_two_sum(sh, sl), rdf[r]));
+            else if (c == r) X[tri(r, r)] = rdf[r];
+            __syncwarp();
         }
     }
     __syncthreads();
     float *lo = g.linv + (size_t)pix * npairs;
-    for (int i = tid; i < npairs; i += kGlsThreads) lo[i] = __fadd_rn(xh[i], xl[i]);
+    for (int i = tid; i < npairs; i += kGlsThreads) lo[i] = __fadd_rn(X[i].hi, X[i].lo);
     // transformed data L^-1 mcov
     if (tid < n1) {
-        const int r = tid, rb = tri(r, 0);
+        const f2 *Xr = X + tri(tid, 0);
         float sh = 0.f, sl = 0.f;
-        for (int c = 0; c <= r; c++) ff_dot_step(xh[rb + c], xl[rb + c], mcovf[c].hi, mcovf[c].lo, sh, sl);
-        g.ytrans[(size_t)pix * n1 + r] = sh + sl;
+        for (int c = 0; c <= tid; c++) ff_dot_step(Xr[c].hi, Xr[c].lo, mcovf[c].hi, mcovf[c].lo, sh, sl);
+        g.ytrans[(size_t)pix * n1 + tid] = sh + sl;
     }
     if (tid == 0) g.ok[pix] = 1;
 }
@@ -384,8 +475,7 @@ size_t gls_smem_bytes(int chanum)
     const int n1 = chanum - 1;
     const size_t npairs = (size_t)n1 * (n1 + 1) / 2;
     const size_t rows = (size_t)((n1 + kGlsTile - 1) / kGlsTile) * kGlsTile;
-    const size_t stage = rows * kGlsZStride * sizeof(float);
-    return 2 * npairs * sizeof(double) + (stage > npairs * sizeof(double) ? stage : npairs * sizeof(double));
+    return 2 * npairs * sizeof(double) + rows * kGlsZStride * sizeof(float);
 }
 
 cudaError_t launch_gls(const GlsArgs &g, cudaStream_t stream)

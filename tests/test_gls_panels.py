@@ -1,0 +1,32 @@
+"""GLS covariance, Cholesky factor and whitened fit at matrix sizes around the
+factorisation's panels of 8 columns and the warps' 32 (lags 24 to 72), against
+the FP64 oracle; tolerances of the GLS parity tests."""
+import numpy as np
+import pytest
+
+from imaging_fcs_1_52_gb300 import engine
+from tests.helpers import FIT_TOL, run_both
+from tests.synth import brownian_stack
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("q", [2, 3, 4, 5, 6, 7, 8])
+def test_matrix_sizes_match_oracle(q):
+    st = brownian_stack(6, 5, 9000, seed=61, density=3.0, cps=1e5)
+    cfg = engine.FCSConfig(width=6, height=5, frames=9000, background=100, q=q, gls=True)
+    gpu, ref = run_both(st, cfg)
+    np.testing.assert_array_equal(gpu["blocked_ind"], ref["blocked_ind"])
+    n1 = cfg.chanum - 1
+    g, r = gpu["covmats"].reshape(-1, n1, n1), ref["covmats"].reshape(-1, n1, n1)
+    fin = np.isfinite(r).all(axis=(1, 2))
+    assert fin.sum() >= 15
+    scale = np.abs(r[fin]).max(axis=(1, 2), keepdims=True)
+    assert np.max(np.abs(g[fin] - r[fin]) / scale) <= 1e-4
+    if q < 5:
+        return                # lag times too short for the fit to be determined at FIT_TOL
+    both = (gpu["fitted"] == 1) & (ref["fitted"] == 1)
+    assert both.sum() >= 0.8 * (ref["fitted"] == 1).sum()
+    for i in (0, 1):
+        err = np.abs(gpu["fitres"][both, i] / ref["fitres"][both, i] - 1)
+        assert both.sum() == 0 or err.max() <= FIT_TOL, (i, err.max())
