@@ -32,8 +32,9 @@ struct FitArgs {
     const int *todo;         // [fit]: 0 = leave this fit's outputs untouched; nullptr = fit all
     int *counter;            // zeroed work counter: warps take fits dynamically; nullptr = static stride
     int tirf_zero_held;      // the held parameters (vx, vy, F2, F3, Ftrip) are zero for every fit
-    int two_zero_held;       // the same without F2: vx, vy, F3 and Ftrip are zero for every fit
-    float one;               // 1.f (see two_model_f)
+    int plain_held;          // held flow, F3 and Ftrip (k = 3: and F2) are zero and without effect in every fit,
+                             // with cst: and every fit's window offset
+    float one;               // 1.f (see plain_model_f)
 };
 
 struct EpilogueArgs {

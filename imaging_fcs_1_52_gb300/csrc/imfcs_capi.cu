@@ -619,8 +619,8 @@ static int run_lm(imfcs_plan *pl, cudaStream_t s, const float *y, const float *w
     // default one-component model (seeds change only N, D, G)
     a.tirf_zero_held = c.init[2] == 0 && c.init[3] == 0 && c.init[5] == 0 && c.init[7] == 0 && c.init[9] == 0;
     // the initial values of the Bayes fits hold everything else at zero
-    a.two_zero_held = init == pl->bfit_init2 ||
-                      (c.init[2] == 0 && c.init[3] == 0 && c.init[7] == 0 && c.init[9] == 0);
+    a.plain_held = init == pl->bfit_init2 || (k == 5 && c.init[2] == 0 && c.init[3] == 0 && c.init[7] == 0 &&
+                                              c.init[9] == 0 && c.init[10] >= 0);
     a.one = 1.f;
     CK(launch_lm(a, pl->num_sms, s));
     pl->launches += 1;

@@ -28,8 +28,9 @@ cudaError_t launch_lm_k5(const FitArgs &a, bool big, int blocks, int threads, si
 cudaError_t launch_lm_k11(const FitArgs &a, bool big, int blocks, int threads, size_t smem, cudaStream_t s);
 // specialised kernel of the default fit (imfcs_lm_tirf.cu)
 bool lm_tirf_applies(const FitArgs &a, bool tirf_zero_held);
-bool lm_two_applies(const FitArgs &a);
-cudaError_t launch_lm_two(const FitArgs &a, int num_sms, cudaStream_t s);
+// specialised kernels of the plain one- and two-component fits (imfcs_lm_comp.cu)
+bool lm_comp_applies(const FitArgs &a);
+cudaError_t launch_lm_comp(const FitArgs &a, cudaStream_t s);
 cudaError_t launch_lm_tirf(const FitArgs &a, int blocks, int threads, cudaStream_t s);
 
 size_t lm_smem_bytes(const FitArgs &a, int km, int warps)
@@ -49,11 +50,11 @@ cudaError_t launch_lm(const FitArgs &a, int num_sms, cudaStream_t stream)
     int blocks = (a.nfits + warps - 1) / warps;
     int cap = num_sms * 16;
     if (blocks > cap) blocks = cap;
+    if (lm_comp_applies(a)) return launch_lm_comp(a, stream);
     if (a.counter) {
         const cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(int), stream);
         if (e != cudaSuccess) return e;
     }
-    if (lm_two_applies(a)) return launch_lm_two(a, num_sms, stream);
     if (lm_tirf_applies(a, a.tirf_zero_held != 0)) return launch_lm_tirf(a, blocks, warps * 32, stream);
     if (km == 3) return launch_lm_k3(a, big, blocks, warps * 32, smem, stream);
     if (km == 5) return launch_lm_k5(a, big, blocks, warps * 32, smem, stream);

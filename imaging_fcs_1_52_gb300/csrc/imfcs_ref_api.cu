@@ -396,6 +396,14 @@ extern "C" int imfcs_fit(int n_fits, int n_points, const float *data, const floa
     a.out_chi2 = dchi;
     a.out_state = dst;
     a.out_iter = dit;
+    a.one = 1.f;
+    a.plain_held = acf;
+    for (int f = 0; f < n_fits && a.plain_held; f++) {
+        // the one-component model without flow, triplet or window offset
+        const float *p0 = &init[(size_t)f * np], *cc = &cst[(size_t)f * IMFCS_NCONST];
+        a.plain_held = p0[2] == 0.f && p0[3] == 0.f && p0[5] == 0.f && p0[7] == 0.f && p0[9] == 0.f &&
+                       p0[10] == 0.f && cc[4] == 0.f && cc[5] == 0.f && isfinite(cc[7]) && isfinite(cc[8]);
+    }
     {
         int dev = 0, sms = 1;
         cudaGetDevice(&dev);
