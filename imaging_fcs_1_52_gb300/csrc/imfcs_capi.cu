@@ -294,7 +294,6 @@ struct imfcs_plan {
         if (copy_stream) cudaStreamSynchronize(copy_stream);
         for (auto &b : bufs) cudaFree(b.p);
         if (own_arena) cudaFree(own_arena);
-        if (li_dev) cudaFree(li_dev);
         for (int i = 0; i <= kStages; i++)
             if (ev[i]) cudaEventDestroy(ev[i]);
         for (int i = 0; i < 2; i++) {
@@ -333,6 +332,29 @@ struct imfcs_plan {
             *f.ptr = base ? (void *)((char *)base + off) : nullptr;
             off += f.bytes;
         }
+    }
+    // constant tables of the plan, one allocation (each costs a call that
+    // creates a plan for itself some 40 us)
+    std::vector<ScratchField> tables;
+    template <class T>
+    void reserve_table(T *&ptr, size_t count)
+    {
+        size_t n = count * sizeof(T);
+        n = ((n ? n : 16) + 255) & ~(size_t)255;
+        tables.push_back({reinterpret_cast<void **>(&ptr), n});
+    }
+    cudaError_t alloc_tables()
+    {
+        size_t need = 0;
+        for (const ScratchField &f : tables) need += f.bytes;
+        char *p = nullptr;
+        const cudaError_t e = alloc(p, need);
+        if (e != cudaSuccess) return e;
+        for (const ScratchField &f : tables) {
+            *f.ptr = p;
+            p += f.bytes;
+        }
+        return cudaSuccess;
     }
     template <class T>
     cudaError_t alloc(T *&ptr, size_t count)
@@ -450,10 +472,9 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
 
     cudaError_t e = cudaSuccess;
     const size_t nt = j.ntrace, np = j.npix;
-#define AL(ptr, n) if (e == cudaSuccess) e = pl->alloc(ptr, (size_t)(n))
+#define AL(ptr, n) pl->reserve_table(ptr, (size_t)(n))
 #define AS(ptr, n) pl->reserve(ptr, (size_t)(n))
-    e = cudaMalloc(&pl->li_dev, sizeof(LagInfo));   // freed separately in the destructor
-    if (e != cudaSuccess) pl->li_dev = nullptr;
+    AL(pl->li_dev, 1);
     AS(pl->trace, nt * j.nopit);
     AS(pl->bparams, nt * kBleachStride);
     AL(pl->snap_pos, kMaxSnap);
@@ -507,6 +528,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     }
 #undef AL
 #undef AS
+    e = pl->alloc_tables();
     // the scratch arena (a batch binds its own instead)
     if (e == cudaSuccess && !external_scratch) {
         e = cudaMalloc(&pl->own_arena, pl->scratch_need);

@@ -22,6 +22,11 @@ int corr_kernel_count(const Job &j);        // kernels one correlator launch iss
 
 struct FitArgs;
 cudaError_t launch_lm(const FitArgs &a, int num_sms, cudaStream_t stream);
+// initial values [fit][nparam] (SI) -> internal units [fit][IMFCS_NPARAM] and constants; fitted values back
+cudaError_t launch_fit_prepare(int nfits, int nparam, int np, bool acf, const float *init_si, float *init_int,
+                               float *cst, cudaStream_t s);
+cudaError_t launch_fit_finish(int nfits, int nparam, int np, bool acf, const float *init_si, const float *par_int,
+                              float *out, cudaStream_t s);
 struct EpilogueArgs;
 cudaError_t launch_fit_epilogue(const EpilogueArgs &e, cudaStream_t stream);
 cudaError_t launch_ols_prepare(int npix, int chanum, int fitstart, int npts, const double *acf,

@@ -51,6 +51,20 @@ __global__ void noalloc_finish_kernel(int nfits, int nparam, int np, int acf, co
     }
 }
 
+cudaError_t launch_fit_prepare(int nfits, int nparam, int np, bool acf, const float *init_si, float *init_int,
+                               float *cst, cudaStream_t s)
+{
+    noalloc_prepare_kernel<<<(nfits + 127) / 128, 128, 0, s>>>(nfits, nparam, np, acf, init_si, init_int, cst);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fit_finish(int nfits, int nparam, int np, bool acf, const float *init_si, const float *par_int,
+                              float *out, cudaStream_t s)
+{
+    noalloc_finish_kernel<<<(nfits + 127) / 128, 128, 0, s>>>(nfits, nparam, np, acf, init_si, par_int, out);
+    return cudaGetLastError();
+}
+
 }  // namespace imfcs
 
 using namespace imfcs;
@@ -101,9 +115,7 @@ extern "C" int imfcs_fit_device_noalloc(int n_fits, int n_points, const float *d
     float *cst = init_int + (size_t)IMFCS_FIT_NOALLOC_MAX_FITS * IMFCS_NPARAM;
     float *par = cst + (size_t)IMFCS_FIT_NOALLOC_MAX_FITS * IMFCS_NCONST;
 
-    const int threads = 128, blocks = (n_fits + threads - 1) / threads;
-    noalloc_prepare_kernel<<<blocks, threads, 0, s>>>(n_fits, nparam, np, acf, initial_parameters, init_int, cst);
-    e = cudaGetLastError();
+    e = launch_fit_prepare(n_fits, nparam, np, acf, initial_parameters, init_int, cst, s);
     if (e != cudaSuccess) { set_error(cuda_msg(e, "noalloc prepare")); return -1; }
 
     FitArgs a;
@@ -130,9 +142,7 @@ extern "C" int imfcs_fit_device_noalloc(int n_fits, int n_points, const float *d
     e = launch_lm(a, sms, s);
     if (e != cudaSuccess) { set_error(cuda_msg(e, "lm_kernel")); return -1; }
 
-    noalloc_finish_kernel<<<blocks, threads, 0, s>>>(n_fits, nparam, np, acf, initial_parameters, par,
-                                                     output_parameters);
-    e = cudaGetLastError();
+    e = launch_fit_finish(n_fits, nparam, np, acf, initial_parameters, par, output_parameters, s);
     if (e != cudaSuccess) { set_error(cuda_msg(e, "noalloc finish")); return -1; }
     return 0;
 }
