@@ -243,7 +243,7 @@ struct imfcs_plan {
     std::vector<DevBuf> bufs;
     size_t bytes = 0;
     // scratch
-    float *trace = nullptr, *bparams = nullptr, *basis = nullptr;
+    float *trace = nullptr, *bparams = nullptr, *basis = nullptr, *grid = nullptr;
     unsigned *trace_sums = nullptr;   // only where s0 is too small to hold the trace's raw sums
     double *proj = nullptr;
     int *snap_pos = nullptr;
@@ -501,6 +501,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
         AL(pl->proj, (size_t)(j.poly_order + 1) * j.nopit);
         AL(pl->basis, (size_t)basis_stride(j.poly_order) * j.num);
     }
+    if (j.bleach == IMFCS_BLEACH_SINGLE_EXP) AL(pl->grid, bleach_grid_floats());
     if (cfg->gls) {
         AS(pl->bprod, np * (chanum - 1) * (size_t)pl->pnum_max);
         AS(pl->linv, np * (size_t)(chanum - 1) * chanum / 2);
@@ -557,6 +558,10 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
         legendre_basis_table(j.poly_order, j.num, cfg->frametime, pl->uscale, pl->uoff, table.data());
         e = cudaMemcpy(pl->proj, proj.data(), proj.size() * sizeof(double), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(pl->basis, table.data(), table.size() * sizeof(float), cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess && j.bleach == IMFCS_BLEACH_SINGLE_EXP) {
+        e = launch_bleach_grid_table(j, pl->grid, nullptr);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     }
     if (e == cudaSuccess && (cfg->do_fit || cfg->bayes)) {
         std::vector<float> xs(pl->nfitpts), init(IMFCS_NPARAM);
@@ -740,7 +745,8 @@ int plan_execute_any(imfcs_plan *pl, const void *dev_stack, const imfcs_outputs 
     CK(launch_trace(j, dev_stack, pl->trace_sums ? pl->trace_sums : (unsigned *)pl->s0, pl->trace, s));
     if (trace_sums_elems(j)) pl->launches += 1;
     if (pl->given_bleach) CK(launch_center_given(j, pl->trace, pl->bparams, s));
-    else CK(launch_bleach(j, pl->trace, pl->proj, (float)pl->uscale, (float)pl->uoff, pl->bparams, s));
+    else CK(launch_bleach(j, pl->trace, pl->proj, (float)pl->uscale, (float)pl->uoff, pl->grid, pl->bparams, s));
+    if (!pl->given_bleach && j.bleach == IMFCS_BLEACH_SINGLE_EXP) pl->launches += 1;
     pl->launches += 2;
     pl->mark(1, s);
     // one streaming pass over the raw stack: the corrected, centred level-0

@@ -40,8 +40,11 @@ cudaError_t launch_gls(const GlsArgs &g, cudaStream_t stream);
 // sums: trace_sums_elems scratch values (0 of them: the one-pass kernel runs)
 cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float *trace, cudaStream_t s);
 size_t trace_sums_elems(const Job &j);
+// grid: launch_bleach_grid_table's table (single exponential), else unused
 cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, float uscale,
-                          float uoff, float *bparams, cudaStream_t s);
+                          float uoff, const float *grid, float *bparams, cudaStream_t s);
+size_t bleach_grid_floats();
+cudaError_t launch_bleach_grid_table(const Job &j, float *tab, cudaStream_t s);
 cudaError_t launch_center_given(const Job &j, const float *trace, float *bparams, cudaStream_t s);
 cudaError_t launch_stream(const Job &j, const void *stack, const float *bparams, const float *basis,
                           const int *snap_pos, int nseg, float *s0, float2 *segtot, float2 *snap_part, int *segbad,

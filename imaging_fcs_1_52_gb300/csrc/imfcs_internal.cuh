@@ -453,4 +453,33 @@ __device__ __forceinline__ double warp_sum_d(double v)
     return v;
 }
 
+// Sums over the warp of N values, each in the order of warp_sum (lanes 16, 8,
+// 4, 2, 1 apart): every exchange halves the values a lane still carries, 21
+// shuffles for 20 values instead of 100.  Returns a sum and its index in
+// `pos` (-1: padding).
+template <int N, int O>
+__device__ __forceinline__ float warp_sums(const float (&v)[N], int lane, int &pos)
+{
+    if constexpr (N == 1 || O == 0) {
+        float r = v[0];
+#pragma unroll
+        for (int o = O; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        pos = 0;
+        return r;
+    } else {
+        constexpr int H = (N + 1) / 2;
+        const bool up = lane & O;
+        float a[H];
+#pragma unroll
+        for (int i = 0; i < H; i++) {
+            const float hi = i + H < N ? v[i + H < N ? i + H : 0] : 0.f;
+            const float keep = up ? hi : v[i], send = up ? v[i] : hi;
+            a[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+        }
+        const float r = warp_sums<H, O / 2>(a, lane, pos);
+        if (up) pos = pos >= 0 && pos + H < N ? pos + H : -1;
+        return r;
+    }
+}
+
 }  // namespace imfcs

@@ -326,110 +326,91 @@ __device__ __forceinline__ float exp_d2udk2(float k, float ik, float t, float e,
     return (-t * t * e - 2.f * uk) * ik;
 }
 
-// One evaluation of the scaled model at p over the trace (warp).
-//   precise = false: FP32 residuals, A = J^T J (Gauss-Newton matrix), g = J^T r;
-//   precise = true:  residuals in float-float (the exponentials by a per-lane
-//                    recurrence e <- e q seeded in FP64), A = the full Hessian
-//                    of chi^2/2, J^T J - sum_i r_i d2f_i (FP32), g = J^T r
-//                    accumulated in float-float and reduced in FP64.
-// Returns chi^2 (float-float summed when precise).
-template <int K>
-__device__ __noinline__ double exp_normal(const float *y, int n, float dts, float iy, const double *p, bool precise,
-                                          float *A, double *g, int lane)
+// One evaluation of the scaled model at p over the trace (warp): residuals in
+// float-float (the exponentials by a per-lane recurrence e <- e q seeded in
+// FP64), A = the full Hessian of chi^2/2, J^T J - sum_i r_i d2f_i (FP32),
+// g = J^T r accumulated in float-float and reduced in FP64.  VALUE: chi^2
+// alone.  Returns chi^2 (float-float summed).
+template <int K, bool VALUE>
+__device__ __noinline__ double exp_normal(const float *y, int n, float dts, float iy, const double *p, float *A,
+                                          double *g, int lane)
 {
     constexpr int NC = (K - 1) / 2;
     constexpr int NA = K * (K + 1) / 2;
-    float acc[NA], gf[K];
+    float acc[NA];
     f2 gp[K];
     for (int i = 0; i < NA; i++) acc[i] = 0.f;
-    for (int i = 0; i < K; i++) { gf[i] = 0.f; gp[i] = {0.f, 0.f}; }
+    for (int i = 0; i < K; i++) gp[i] = {0.f, 0.f};
     float pf[K], ik[NC];
     for (int i = 0; i < K; i++) pf[i] = (float)p[i];
     for (int c = 0; c < NC; c++) ik[c] = 1.f / pf[2 + 2 * c];
-    f2 e[NC], q[NC], invk[NC], sp[NC], f0;
+    f2 e[NC], q[NC], invk[NC], sp[NC];
     bool slow[NC];
-    if (precise) {
-        f0 = f2_from_d(p[0]);
-        for (int c = 0; c < NC; c++) {
-            const double k = p[2 + 2 * c];
-            e[c] = f2_from_d(exp(-k * ((double)lane + 0.5) * (double)dts));
-            q[c] = f2_from_d(exp(-k * 32.0 * (double)dts));
-            slow[c] = fabs(k * (double)n * (double)dts) < 1e-4;
-            invk[c] = f2_from_d(slow[c] ? 0.0 : 1.0 / k);
-            sp[c] = f2_from_d(p[1 + 2 * c]);
-        }
+    const f2 f0 = f2_from_d(p[0]);
+    for (int c = 0; c < NC; c++) {
+        const double k = p[2 + 2 * c];
+        e[c] = f2_from_d(exp(-k * ((double)lane + 0.5) * (double)dts));
+        q[c] = f2_from_d(exp(-k * 32.0 * (double)dts));
+        slow[c] = fabs(k * (double)n * (double)dts) < 1e-4;
+        invk[c] = f2_from_d(slow[c] ? 0.0 : 1.0 / k);
+        sp[c] = f2_from_d(p[1 + 2 * c]);
     }
-    float c2f = 0.f;            // FP32 phase: per-lane sum of ~n/32 squares
     f2 c2 = {0.f, 0.f};
     for (int x = lane; x < n; x += 32) {
         const float t = ((float)x + 0.5f) * dts;
-        float gr[K], r;
-        float hsk[NC], hkk[NC];   // d2f/(ds dk), d2f/dk2 per component (precise)
+        float gr[K];
+        float hsk[NC], hkk[NC];   // d2f/(ds dk), d2f/dk2 per component
         gr[0] = 1.f;
-        if (!precise) {
-            float f = pf[0];
-            for (int c = 0; c < NC; c++) {
-                float u, du;
-                exp_u_f(pf[2 + 2 * c], ik[c], t, u, du);
-                f -= pf[1 + 2 * c] * u;
-                gr[1 + 2 * c] = -u;
-                gr[2 + 2 * c] = -pf[1 + 2 * c] * du;
+        const f2 tf = f2_two_prod((float)x + 0.5f, dts);
+        f2 f = f0;
+        for (int c = 0; c < NC; c++) {
+            f2 u;
+            if (slow[c]) {
+                // u = t (1 - corr), corr = x/2 - x^2/6 + x^3/24 (|x| < 1e-4)
+                const float xx = pf[2 + 2 * c] * t;
+                const float corr = xx * (0.5f - xx * (1.f / 6.f - xx * (1.f / 24.f)));
+                u = f2_add(tf, f2_neg(f2_two_prod(tf.hi, corr)));
+            } else {
+                u = f2_mul(f2_add({1.f, 0.f}, f2_neg(e[c])), invk[c]);
             }
-            r = __ldg(&y[x]) * iy - f;
-            c2f = fmaf(r, r, c2f);
-        } else {
-            const f2 tf = f2_two_prod((float)x + 0.5f, dts);
-            f2 f = f0;
-            for (int c = 0; c < NC; c++) {
-                f2 u;
-                if (slow[c]) {
-                    // u = t (1 - corr), corr = x/2 - x^2/6 + x^3/24 (|x| < 1e-4)
-                    const float xx = pf[2 + 2 * c] * t;
-                    const float corr = xx * (0.5f - xx * (1.f / 6.f - xx * (1.f / 24.f)));
-                    u = f2_add(tf, f2_neg(f2_two_prod(tf.hi, corr)));
-                } else {
-                    u = f2_mul(f2_add({1.f, 0.f}, f2_neg(e[c])), invk[c]);
-                }
-                f = f2_add(f, f2_neg(f2_mul(sp[c], u)));
+            f = f2_add(f, f2_neg(f2_mul(sp[c], u)));
+            if (!VALUE) {
                 const float uf = u.hi + u.lo, ef = e[c].hi + e[c].lo;
                 const float uk = exp_dudk(pf[2 + 2 * c], ik[c], t, ef, uf);
                 gr[1 + 2 * c] = -uf;
                 gr[2 + 2 * c] = -pf[1 + 2 * c] * uk;
                 hsk[c] = -uk;
                 hkk[c] = -pf[1 + 2 * c] * exp_d2udk2(pf[2 + 2 * c], ik[c], t, ef, uk);
-                e[c] = f2_mul(e[c], q[c]);
             }
-            const f2 rr = f2_add(f2_two_prod(__ldg(&y[x]), iy), f2_neg(f));
-            r = rr.hi + rr.lo;
-            c2 = f2_add(c2, f2_mul(rr, rr));
-            for (int a = 0; a < K; a++) gp[a] = f2_add(gp[a], f2_two_prod(gr[a], rr.hi));
-            for (int a = 0; a < K; a++) gp[a] = f2_add(gp[a], f2_two_prod(gr[a], rr.lo));
+            e[c] = f2_mul(e[c], q[c]);
         }
+        const f2 rr = f2_add(f2_two_prod(__ldg(&y[x]), iy), f2_neg(f));
+        c2 = f2_add(c2, f2_mul(rr, rr));
+        if (VALUE) continue;
+        const float r = rr.hi + rr.lo;
+        for (int a = 0; a < K; a++) gp[a] = f2_add(gp[a], f2_two_prod(gr[a], rr.hi));
+        for (int a = 0; a < K; a++) gp[a] = f2_add(gp[a], f2_two_prod(gr[a], rr.lo));
         int qa = 0;
         for (int a = 0; a < K; a++)
             for (int b = 0; b <= a; b++) acc[qa++] += gr[a] * gr[b];
-        if (precise) {
-            // - r d2f: the only nonzero second derivatives are (s_c, k_c) and (k_c, k_c)
-            for (int c = 0; c < NC; c++) {
-                const int is = 1 + 2 * c, ikk = 2 + 2 * c;
-                acc[ikk * (ikk + 1) / 2 + is] -= r * hsk[c];
-                acc[ikk * (ikk + 1) / 2 + ikk] -= r * hkk[c];
-            }
-        } else {
-            for (int a = 0; a < K; a++) gf[a] += gr[a] * r;
+        // - r d2f: the only nonzero second derivatives are (s_c, k_c) and (k_c, k_c)
+        for (int c = 0; c < NC; c++) {
+            const int is = 1 + 2 * c, ikk = 2 + 2 * c;
+            acc[ikk * (ikk + 1) / 2 + is] -= r * hsk[c];
+            acc[ikk * (ikk + 1) / 2 + ikk] -= r * hkk[c];
         }
     }
-    int qa = 0;
-    for (int a = 0; a < K; a++)
-        for (int b = 0; b <= a; b++) {
-            float v = warp_sum(acc[qa++]);
-            A[a * K + b] = v;
-            A[b * K + a] = v;
-        }
-    for (int a = 0; a < K; a++)
-        g[a] = precise ? warp_sum_d((double)gp[a].hi + (double)gp[a].lo) : (double)warp_sum(gf[a]);
-    const double c2d = precise ? (double)c2.hi + (double)c2.lo : (double)c2f;
-    return warp_sum_d(c2d);
+    if (!VALUE) {
+        int qa = 0;
+        for (int a = 0; a < K; a++)
+            for (int b = 0; b <= a; b++) {
+                float v = warp_sum(acc[qa++]);
+                A[a * K + b] = v;
+                A[b * K + a] = v;
+            }
+        for (int a = 0; a < K; a++) g[a] = warp_sum_d((double)gp[a].hi + (double)gp[a].lo);
+    }
+    return warp_sum_d((double)c2.hi + (double)c2.lo);
 }
 
 // FP32 evaluation for phase 1 (no FP64 operation: GB300 issues FP64 at 1/64
@@ -510,8 +491,162 @@ __device__ __forceinline__ bool exp_newton_step(const float *A, const double *gd
     return ok;
 }
 
+// Scaled time per trace point; tmax: the last point's time (s).
+__host__ __device__ inline float bleach_dts(const Job &j, float &tmax)
+{
+    const double dt_pt = (double)j.frametime * (double)j.ave;
+    tmax = (float)(dt_pt * ((double)j.nopit - 0.5));
+    return (float)(dt_pt / (double)tmax);
+}
+
+// Start of the single-exponential fit: global search by variable projection.
+// For each rate of the grid x = k tmax in {0} and 96 log-spaced values 1e-3 ..
+// 1e4 (the oracle's grid), c0 + c1 e^{-kt} (k = 0: c0 + c1 t) is linear in c0,
+// c1 and chi^2 is minimised over them exactly; the best rate starts the LM.
+//
+// The centred basis b = e^{-kt} - mean and its square sum are the same for
+// every trace: bleach_grid_table_kernel lays them out once per plan, and what is
+// left per trace are 97 dot products of 1000 points.  A CTA takes T traces; a
+// warp takes eight rates at a time, a lane its points lane, lane + 32, ... in
+// that order (sums as one rate of one trace at a time gives them), so a loaded
+// basis value serves T traces and a loaded sample eight rates.  Bound by FP32
+// issue and the loads of the table (430 KB, in L2): 16,384 traces in 0.15 ms,
+// against 0.7 ms of the fit kernel when each trace's warp made its own basis.
+constexpr int kGridRates = 97, kGridPad = 104, kGridPts = 1024;
+
+// Position of point x in the table: a lane's four successive points adjoin.
+__device__ __forceinline__ int grid_pos(int x) { return ((x >> 7) * 32 + (x & 31)) * 4 + ((x >> 5) & 3); }
+
+// tab: [rate][1024] centred basis (0 past the trace), then [3][kGridPad]: mean, square sum, rate.
+__global__ void __launch_bounds__(32) bleach_grid_table_kernel(int n, float dts, float *tab)
+{
+    const int lane = threadIdx.x, jg = blockIdx.x;
+    float *row = tab + (size_t)jg * kGridPts, *stat = tab + (size_t)kGridPad * kGridPts + jg;
+    const float kx = (jg == 0 || jg >= kGridRates) ? 0.f : exp10f(-3.f + 7.f * (float)(jg - 1) / 95.f);
+    const float q = __expf(-kx * 32.f * dts), e0 = __expf(-kx * ((float)lane + 0.5f) * dts);
+    float se = 0.f, e = e0;
+    for (int x = lane; x < n; x += 32) {
+        const float tt = ((float)x + 0.5f) * dts;
+        se += jg == 0 ? tt : e;
+        e *= q;
+    }
+    const float me = warp_sum(se) / (float)n;
+    float see = 0.f;
+    e = e0;
+    for (int x = lane; x < kGridPts; x += 32) {
+        const float tt = ((float)x + 0.5f) * dts;
+        const float b = x < n ? (jg == 0 ? tt : e) - me : 0.f;
+        see = fmaf(b, b, see);
+        row[grid_pos(x)] = b;
+        e *= q;
+    }
+    const float sE = warp_sum(see);
+    if (lane == 0) {
+        stat[0] = me;
+        stat[kGridPad] = sE;
+        stat[2 * kGridPad] = kx;
+    }
+}
+
+template <int T>
+__global__ void __launch_bounds__(128) bleach_grid_kernel(Job j, const float *trace, const float *tab, float *bp_out)
+{
+    constexpr int RB = 8;                         // rates of a warp's pass
+    constexpr int NS = T * RB, NW = NS > 32 ? 32 : NS;
+    __shared__ float4 yc[T][kGridPts / 4];        // centred samples, table order
+    __shared__ float sy[T][kGridPad];             // dot products
+    __shared__ float my[T], syy[T];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tr0 = blockIdx.x * T, n = j.nopit;
+    for (int m = wid; m < T; m += 4) {
+        float *out = reinterpret_cast<float *>(yc[m]);
+        const int tr = tr0 + m;
+        if (tr >= j.ntrace) {
+            for (int x = lane; x < kGridPts; x += 32) out[x] = 0.f;
+            continue;
+        }
+        const float *y = trace + (size_t)tr * n;
+        float ym = 0.f;
+        for (int x = lane; x < n; x += 32) ym = fmaxf(ym, fabsf(__ldg(&y[x])));
+        for (int o = 16; o > 0; o >>= 1) ym = fmaxf(ym, __shfl_xor_sync(0xffffffffu, ym, o));
+        if (ym == 0.f) ym = 1.f;
+        const float iy = 1.f / ym;
+        float s = 0.f;
+        for (int x = lane; x < n; x += 32) s += __ldg(&y[x]) * iy;
+        const float mean = warp_sum(s) / (float)n;
+        float s2 = 0.f;
+        for (int x = lane; x < kGridPts; x += 32) {
+            const float v = x < n ? __ldg(&y[x]) * iy - mean : 0.f;
+            s2 = fmaf(v, v, s2);
+            out[grid_pos(x)] = v;
+        }
+        s2 = warp_sum(s2);
+        if (lane == 0) { my[m] = mean; syy[m] = s2; }
+    }
+    __syncthreads();
+    const float4 *tab4 = reinterpret_cast<const float4 *>(tab);
+    for (int jb = wid * RB; jb < kGridPad; jb += 4 * RB) {
+        float acc[NS];
+#pragma unroll
+        for (int i = 0; i < NS; i++) acc[i] = 0.f;
+#pragma unroll 1
+        for (int i = lane; i < kGridPts / 4; i += 32) {
+            float4 b[RB];
+#pragma unroll
+            for (int r = 0; r < RB; r++) b[r] = __ldg(&tab4[(size_t)(jb + r) * (kGridPts / 4) + i]);
+#pragma unroll
+            for (int m = 0; m < T; m++) {
+                const float4 v = yc[m][i];
+#pragma unroll
+                for (int r = 0; r < RB; r++) {
+                    float a = acc[m * RB + r];
+                    a = fmaf(v.x, b[r].x, a);
+                    a = fmaf(v.y, b[r].y, a);
+                    a = fmaf(v.z, b[r].z, a);
+                    acc[m * RB + r] = fmaf(v.w, b[r].w, a);
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < NS; h += NW) {
+            float part[NW];
+#pragma unroll
+            for (int i = 0; i < NW; i++) part[i] = acc[h + i];
+            int pos;
+            const float v = warp_sums<NW, 16>(part, lane, pos);
+            if (pos >= 0) sy[(h + pos) / RB][jb + (h + pos) % RB] = v;
+        }
+    }
+    __syncthreads();
+    const float *stat = tab + (size_t)kGridPad * kGridPts;
+    for (int m = wid; m < T; m += 4) {
+        if (tr0 + m >= j.ntrace) break;
+        // the first rate of least chi^2 (below 3.4e38)
+        float bc = 3.4e38f, b1 = 0.f;
+        int bj = kGridPad;
+        for (int jg = lane; jg < kGridRates; jg += 32) {
+            const float sE = __ldg(&stat[kGridPad + jg]), sY = sy[m][jg];
+            const float c1 = sE > 0.f ? sY / sE : 0.f;
+            const float c2 = syy[m] - c1 * sY;
+            if (c2 < bc) { bc = c2; b1 = c1; bj = jg; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float oc = __shfl_xor_sync(0xffffffffu, bc, o), o1 = __shfl_xor_sync(0xffffffffu, b1, o);
+            const int oj = __shfl_xor_sync(0xffffffffu, bj, o);
+            if (oc < bc || (oc == bc && oj < bj)) { bc = oc; b1 = o1; bj = oj; }
+        }
+        if (lane == 0) {
+            float *bp = bp_out + (size_t)(tr0 + m) * kBleachStride;
+            const bool any = bj < kGridPad;
+            bp[0] = any ? my[m] - b1 * __ldg(&stat[bj]) : 0.f;
+            bp[1] = b1;
+            bp[2] = any ? __ldg(&stat[2 * kGridPad + bj]) : 0.f;
+        }
+    }
+}
+
 template <int K>
-__global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
+__global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *trace, float *bp_out)
 {
     constexpr int NC = (K - 1) / 2;
     const int lane = threadIdx.x & 31;
@@ -520,8 +655,8 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
     const int n = j.nopit;
     const float *y = trace + (size_t)tr * n;
     const double dt_pt = (double)j.frametime * (double)j.ave;      // time per trace point (s)
-    const float tmax = (float)(dt_pt * ((double)n - 0.5));
-    const float dts = (float)(dt_pt / (double)tmax);               // scaled time per point
+    float tmax;
+    const float dts = bleach_dts(j, tmax);
     float ym = 0.f;
     for (int x = lane; x < n; x += 32) ym = fmaxf(ym, fabsf(__ldg(&y[x])));
     for (int o = 16; o > 0; o >>= 1) ym = fmaxf(ym, __shfl_xor_sync(0xffffffffu, ym, o));
@@ -529,68 +664,9 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
     const float iy = 1.f / ym;
     double p[K];
     if constexpr (K == 3) {
-        // global search by variable projection: for each rate of the grid
-        // x = k tmax in {0} and 96 log-spaced values 1e-3 .. 1e4 (the oracle's
-        // grid), c0 + c1 e^{-kt} (k = 0: c0 + c1 t) is linear in c0, c1 and
-        // chi^2 is minimised over them exactly; the best rate starts the LM
-        float sy = 0.f;
-        for (int x = lane; x < n; x += 32) sy += __ldg(&y[x]) * iy;
-        const float my = warp_sum(sy) / (float)n;
-        float syy = 0.f;
-        for (int x = lane; x < n; x += 32) { const float yc = __ldg(&y[x]) * iy - my; syy = fmaf(yc, yc, syy); }
-        syy = warp_sum(syy);
-        // eight rates per pass over the trace: independent recurrences and
-        // reductions overlap (the per-rate sums are those of one rate at a
-        // time, so the choice is the same)
-        constexpr int RB = 8;
-        float bc = 3.4e38f, b0 = 0.f, b1 = 0.f, bk = 0.f;
-        for (int jb = 0; jb < 97; jb += RB) {
-            float kx[RB], q[RB], e0[RB], se[RB], e[RB];
-#pragma unroll
-            for (int r = 0; r < RB; r++) {
-                const int jg = jb + r;
-                kx[r] = (jg == 0 || jg > 96) ? 0.f : exp10f(-3.f + 7.f * (float)(jg - 1) / 95.f);
-                q[r] = __expf(-kx[r] * 32.f * dts);
-                e0[r] = __expf(-kx[r] * ((float)lane + 0.5f) * dts);
-                se[r] = 0.f;
-                e[r] = e0[r];
-            }
-            for (int x = lane; x < n; x += 32) {
-                const float tt = ((float)x + 0.5f) * dts;
-#pragma unroll
-                for (int r = 0; r < RB; r++) {
-                    se[r] += (jb + r == 0) ? tt : e[r];
-                    e[r] *= q[r];
-                }
-            }
-            float me[RB], see[RB], sye[RB];
-#pragma unroll
-            for (int r = 0; r < RB; r++) {
-                me[r] = warp_sum(se[r]) / (float)n;
-                see[r] = 0.f;
-                sye[r] = 0.f;
-                e[r] = e0[r];
-            }
-            for (int x = lane; x < n; x += 32) {
-                const float tt = ((float)x + 0.5f) * dts;
-                const float yc = __ldg(&y[x]) * iy - my;
-#pragma unroll
-                for (int r = 0; r < RB; r++) {
-                    const float b = ((jb + r == 0) ? tt : e[r]) - me[r];
-                    see[r] = fmaf(b, b, see[r]);
-                    sye[r] = fmaf(yc, b, sye[r]);
-                    e[r] *= q[r];
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < RB; r++) {
-                const float sE = warp_sum(see[r]), sY = warp_sum(sye[r]);
-                if (jb + r > 96) continue;
-                const float c1 = sE > 0.f ? sY / sE : 0.f;
-                const float c2 = syy - c1 * sY;
-                if (c2 < bc) { bc = c2; b1 = c1; b0 = my - c1 * me[r]; bk = kx[r]; }
-            }
-        }
+        // bleach_grid_kernel's start: c0 + c1 e^{-kt} (k = 0: c0 + c1 t)
+        const float *st = bp_out + (size_t)tr * kBleachStride;
+        const float b0 = st[0], b1 = st[1], bk = st[2];
         if (bk == 0.f) { p[0] = b0; p[1] = -b1; p[2] = 0.0; }                  // f = c0 + c1 t
         else { p[0] = (double)b0 + b1; p[1] = (double)b1 * bk; p[2] = bk; }       // f = c0 + c1 e^{-kt}
     } else {
@@ -615,11 +691,13 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
     float chi2f = exp_normal32<K>(y, n, dts, iy, pf, A, gf, lane);
     const bool ok = isfinite(chi2f);
     int evals = 1, rejected = 0;
+    unsigned fix = 0;
+    bool gn_near = false;      // Gauss-Newton step within 0.05 sigma
+    bool fresh = true;         // the Gauss-Newton step stays what it was after a rejected one
     for (int it_n = 0; ok && it_n < 100; it_n++) {
         float h[K];
-        unsigned fix;
-        bool gn_near = false;      // Gauss-Newton step within 0.05 sigma
-        if (exp_newton_step32<K>(A, gf, pf, fix, h)) {
+        if (fresh) gn_near = false;
+        if (fresh && exp_newton_step32<K>(A, gf, pf, fix, h)) {
             bool conv = true;
             gn_near = true;
             for (int a = 0; a < K; a++) {
@@ -630,6 +708,7 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
             }
             if (conv) break;
         }
+        fresh = false;
         if (!solve_scaled_k<K>(A, gf, lambda, fix, h)) {
             lambda *= 10.f;
             if (lambda > 1e10f) break;
@@ -647,6 +726,7 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
             chi2f = c2n;
             lambda = fmaxf(lambda * 0.1f, 1e-12f);
             rejected = 0;
+            fresh = true;
         } else {
             // two rejected steps in a row while the Gauss-Newton step is
             // within 0.05 sigma: FP32 chi^2 no longer resolves the descent
@@ -663,7 +743,7 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
     // gradient, to the least-squares minimum: until the step is below
     // 1e-9 sigma + 1e-12 |p|, while chi^2 does not increase.
     if (ok) {
-        chi2 = exp_normal<K>(y, n, dts, iy, p, true, A, g, lane);
+        chi2 = exp_normal<K, false>(y, n, dts, iy, p, A, g, lane);
         evals++;
         for (int it_n = 0; it_n < 20 && isfinite(chi2); it_n++) {
             float h[K];
@@ -680,13 +760,16 @@ __global__ void bleach_exp_kernel(Job j, const float *trace, float *bp_out)
             for (int c = 0; c < NC; c++) pn[2 + 2 * c] = fmax(pn[2 + 2 * c], 0.0);
             float An[K * K];
             double gn[K];
-            const double c2n = exp_normal<K>(y, n, dts, iy, pn, true, An, gn, lane);
+            // the last step only has to show that chi^2 does not rise
+            const double c2n = conv ? exp_normal<K, true>(y, n, dts, iy, pn, An, gn, lane)
+                                    : exp_normal<K, false>(y, n, dts, iy, pn, An, gn, lane);
             evals++;
             if (!(isfinite(c2n) && c2n <= chi2)) break;
-            for (int a = 0; a < K; a++) { p[a] = pn[a]; g[a] = gn[a]; }
+            for (int a = 0; a < K; a++) p[a] = pn[a];
+            if (conv) break;
+            for (int a = 0; a < K; a++) g[a] = gn[a];
             for (int a = 0; a < K * K; a++) A[a] = An[a];
             chi2 = c2n;
-            if (conv) break;
         }
     }
     // back to data units: y = y_s / iy, t = t_s tmax
@@ -1238,8 +1321,17 @@ cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float 
     return cudaGetLastError();
 }
 
+size_t bleach_grid_floats() { return (size_t)kGridPad * (kGridPts + 3); }
+
+cudaError_t launch_bleach_grid_table(const Job &j, float *tab, cudaStream_t s)
+{
+    float tmax;
+    bleach_grid_table_kernel<<<kGridPad, 32, 0, s>>>(j.nopit, bleach_dts(j, tmax), tab);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, float uscale,
-                          float uoff, float *bparams, cudaStream_t s)
+                          float uoff, const float *grid, float *bparams, cudaStream_t s)
 {
     const int threads = 128;
     const int blocks = (j.ntrace * 32 + threads - 1) / threads;
@@ -1248,6 +1340,10 @@ cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, 
         bleach_poly_kernel<<<blocks, threads, 0, s>>>(j, trace, proj, uscale, uoff, bparams);
         break;
     case IMFCS_BLEACH_SINGLE_EXP:
+        // eight traces a CTA reuse a basis value most (0.15 ms for 16,384); with
+        // fewer than two such CTAs per SM (152) two a CTA fill the chip better
+        if (j.ntrace >= 8 * 304) bleach_grid_kernel<8><<<(j.ntrace + 7) / 8, 128, 0, s>>>(j, trace, grid, bparams);
+        else bleach_grid_kernel<2><<<(j.ntrace + 1) / 2, 128, 0, s>>>(j, trace, grid, bparams);
         bleach_exp_kernel<3><<<blocks, threads, 0, s>>>(j, trace, bparams);
         break;
     case IMFCS_BLEACH_DOUBLE_EXP:

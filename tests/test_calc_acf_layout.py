@@ -1,0 +1,27 @@
+"""Lag-major outputs of calcACF at pixel and lag counts around the 32 x 32
+tiles that turn them, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import oracle
+from imaging_fcs_1_52_gb300._lib import ACFParameters
+from imaging_fcs_1_52_gb300.gpufit_imfcs import GpufitImFCS
+from tests.helpers import ACF_TOL, acf_deviation
+from tests.synth import brownian_stack
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("w,h,q", [(1, 1, 8), (31, 1, 2), (4, 8, 8), (11, 3, 3), (13, 5, 6)])
+def test_outputs_are_lag_major(w, h, q):
+    raw = brownian_stack(w, h, 3000, seed=w, density=2.0, cps=3e4)
+    ch = 17 + 8 * (q - 1)
+    p = ACFParameters(width=w, height=h, win_star=w, hin_star=h, w_temp=w, h_temp=h, pixbinX=1, pixbinY=1,
+                      binningX=1, binningY=1, firstframe=1, lastframe=3000, framediff=3000, cfXDistance=0,
+                      cfYDistance=0, correlatorp=16, correlatorq=q, frametime=1e-3, background=100, chanum=ch,
+                      isNBcalculation=0, bleachcorr_gpu=0, bleachcorr_order=0, nopit=1000, ave=3)
+    outs = [np.zeros((ch, h, w)), np.zeros((ch, h, w)), np.zeros((h, w)), np.zeros((h, w)), np.zeros((2, h, w))]
+    GpufitImFCS.calcACF(raw.astype(np.float32) - 100, *outs, None, np.zeros(ch), np.zeros(ch, np.int32), p)
+    ref = oracle.run(raw, out_w=w, out_h=h, background=100, q=q, do_fit=False)
+    assert acf_deviation({"acf": outs[0].reshape(ch, -1).T}, ref) <= ACF_TOL
+    np.testing.assert_array_equal(outs[4][0].ravel(), ref["blocked_ind"])
