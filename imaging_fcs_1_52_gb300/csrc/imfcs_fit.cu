@@ -32,6 +32,7 @@ bool lm_tirf_applies(const FitArgs &a, bool tirf_zero_held);
 bool lm_comp_applies(const FitArgs &a);
 cudaError_t launch_lm_comp(const FitArgs &a, cudaStream_t s);
 cudaError_t launch_lm_tirf(const FitArgs &a, int blocks, int threads, cudaStream_t s);
+cudaError_t launch_lm_gls(const FitArgs &a, cudaStream_t s);   // the same on whitened data (imfcs_lm_gls.cu)
 
 size_t lm_smem_bytes(const FitArgs &a, int km, int warps)
 {
@@ -50,12 +51,14 @@ cudaError_t launch_lm(const FitArgs &a, int num_sms, cudaStream_t stream)
     int blocks = (a.nfits + warps - 1) / warps;
     int cap = num_sms * 16;
     if (blocks > cap) blocks = cap;
+    const bool tirf = lm_tirf_applies(a, a.tirf_zero_held != 0);
     if (lm_comp_applies(a)) return launch_lm_comp(a, stream);
+    if (tirf && a.linv) return launch_lm_gls(a, stream);
     if (a.counter) {
         const cudaError_t e = cudaMemsetAsync(a.counter, 0, sizeof(int), stream);
         if (e != cudaSuccess) return e;
     }
-    if (lm_tirf_applies(a, a.tirf_zero_held != 0)) return launch_lm_tirf(a, blocks, warps * 32, stream);
+    if (tirf) return launch_lm_tirf(a, blocks, warps * 32, stream);
     if (km == 3) return launch_lm_k3(a, big, blocks, warps * 32, smem, stream);
     if (km == 5) return launch_lm_k5(a, big, blocks, warps * 32, smem, stream);
     return launch_lm_k11(a, big, blocks, warps * 32, smem, stream);
