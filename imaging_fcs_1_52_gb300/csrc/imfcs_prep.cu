@@ -148,38 +148,78 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
 // Polynomial bleach fit: least squares in the Legendre basis of
 // u = t * uscale + uoff (t = averaged-trace time), coefficients = proj * y
 // with the FP64 projection matrix proj[(order+1)][nopit] built on the host.
-// One warp per trace.  Also writes f0 = f(0), the centre c and flags.
+// One warp per trace.  Also writes f0 = f(0), the centre c and flags.  K:
+// order + 1, at compile time, so that the coefficients and the basis values stay in
+// registers and four points' chains overlap (with run-time counts in local
+// memory: 66 us for 441 traces, 190 for 7,938; now 27 and 108, of which FP64
+// issue is 87).
 // ---------------------------------------------------------------------------
-__global__ void bleach_poly_kernel(Job j, const float *trace, const double *proj, float uscale,
-                                   float uoff, float *bp_out)
+
+// x / d for d = 2 .. 8, the bits of the division (checked for every mantissa):
+// the quotient's remainder corrects it.
+template <int D>
+__device__ __forceinline__ float div_small(float x)
+{
+    if constexpr ((D & (D - 1)) == 0) return x * (1.f / D);
+    constexpr float inv = 1.f / D;
+    const float q = __fmul_rn(x, inv);
+    return fmaf(fmaf(-q, (float)D, x), inv, q);
+}
+
+// legendre() with its roundings.
+template <int K, int N = 1>
+__device__ __forceinline__ void legendre_k(float u, float (&out)[K])
+{
+    if constexpr (N == 1) {
+        out[0] = 1.f;
+        out[1] = u;
+    }
+    if constexpr (N + 1 < K) {
+        const float a = (float)(2 * N + 1) * u;
+        out[N + 1] = div_small<N + 1>(fmaf(a, out[N], -__fmul_rn((float)N, out[N - 1])));
+        legendre_k<K, N + 1>(u, out);
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(128) bleach_poly_kernel(Job j, const float *trace, const double *proj, float uscale,
+                                                          float uoff, float *bp_out)
 {
     const int lane = threadIdx.x & 31;
     const int tr = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (tr >= j.ntrace) return;
-    const int k = j.poly_order + 1;
     const float *y = trace + (size_t)tr * j.nopit;
-    double c[kMaxPoly + 1];
-    for (int i = 0; i < k; i++) c[i] = 0.0;
+    double c[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) c[i] = 0.0;
+#pragma unroll 4
     for (int x = lane; x < j.nopit; x += 32) {
-        double yx = (double)__ldg(&y[x]);
-        for (int i = 0; i < k; i++) c[i] = fma(__ldg(&proj[(size_t)i * j.nopit + x]), yx, c[i]);
+        const double yx = f2d(__ldg(&y[x]));
+#pragma unroll
+        for (int i = 0; i < K; i++) c[i] = fma(__ldg(&proj[(size_t)i * j.nopit + x]), yx, c[i]);
     }
-    for (int i = 0; i < k; i++) c[i] = warp_sum_d(c[i]);
-    float cf[kMaxPoly + 1], lb[kMaxPoly + 1];
-    for (int i = 0; i < k; i++) cf[i] = (float)c[i];
-    legendre(uoff, j.poly_order, lb);    // u(0) = uoff
+    float cf[K], lb[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        c[i] = warp_sum_d(c[i]);
+        cf[i] = (float)c[i];
+    }
+    legendre_k<K>(uoff, lb);             // u(0) = uoff
     double f0 = 0.0;
-    for (int i = 0; i < k; i++) f0 += c[i] * (double)lb[i];
+#pragma unroll
+    for (int i = 0; i < K; i++) f0 = fma(c[i], (double)lb[i], f0);
     float f0f = (float)f0, inv_f0 = (float)(1.0 / f0);
     // centre: mean of the finite points of the corrected averaged trace (a
     // shift the correlator removes exactly; non-finite points, where the
     // curve crosses zero, are left out so that they cannot spread)
     float csum = 0.f, cnt = 0.f;
+#pragma unroll 4
     for (int x = lane; x < j.nopit; x += 32) {
         float t = j.frametime * ((float)x + 0.5f) * (float)j.ave;
-        legendre(t * uscale + uoff, j.poly_order, lb);
+        legendre_k<K>(t * uscale + uoff, lb);
         float f = 0.f;
-        for (int i = 0; i < k; i++) f = fmaf(cf[i], lb[i], f);
+#pragma unroll
+        for (int i = 0; i < K; i++) f = fmaf(cf[i], lb[i], f);
         const float v = bleach_correct(__ldg(&y[x]), f, f0f, inv_f0);
         if (isfinite(v)) { csum += v; cnt += 1.f; }
     }
@@ -187,7 +227,8 @@ __global__ void bleach_poly_kernel(Job j, const float *trace, const double *proj
     cnt = warp_sum(cnt);
     if (lane == 0) {
         float *bp = bp_out + (size_t)tr * kBleachStride;
-        for (int i = 0; i < k; i++) bp[i] = cf[i];
+#pragma unroll
+        for (int i = 0; i < K; i++) bp[i] = cf[i];
         bp[9] = f0f;
         bp[10] = inv_f0;
         bp[11] = (isfinite(f0) && f0 != 0.0) ? 1.f : 0.f;
@@ -1337,7 +1378,11 @@ cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, 
     const int blocks = (j.ntrace * 32 + threads - 1) / threads;
     switch (j.bleach) {
     case IMFCS_BLEACH_POLYNOMIAL:
-        bleach_poly_kernel<<<blocks, threads, 0, s>>>(j, trace, proj, uscale, uoff, bparams);
+        switch (j.poly_order) {
+#define POLY(o) case o: bleach_poly_kernel<o + 1><<<blocks, threads, 0, s>>>(j, trace, proj, uscale, uoff, bparams); break
+            POLY(1); POLY(2); POLY(3); POLY(4); POLY(5); POLY(6); POLY(7); POLY(8);
+#undef POLY
+        }
         break;
     case IMFCS_BLEACH_SINGLE_EXP:
         // eight traces a CTA reuse a basis value most (0.15 ms for 16,384); with
