@@ -686,7 +686,7 @@ static int run_epilogue(imfcs_plan *pl, cudaStream_t s, const double *acf, int k
     e.mc = model_const_from(c.cst);
     e.lagtime = pl->lagtime;
     CK(launch_fit_epilogue(e, s));
-    pl->launches += 1;
+    pl->launches += logp ? 2 : 1;
     return 0;
 }
 

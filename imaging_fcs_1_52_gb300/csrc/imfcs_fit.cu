@@ -85,28 +85,50 @@ __global__ void ols_prepare_kernel(int npix, int chanum, int fitstart, int npts,
 // singularity threshold 1 (a singular covariance fails the fit exactly like
 // the catch block of standardFit, java:10412, 10441), and the Bayes terms
 // (java:10171-10207).
+//
+// A few hundred dependent FP64 operations per thread and nothing to overlap them
+// with, on every call's critical path: the parameter count is a template
+// argument (K = 3, 5; 0: at run time), so that matrices stay in registers
+// (30 -> 19 us), and the Bayes residuals, 72 model values a pixel, are a kernel
+// of their own with a warp per pixel (105 -> 41 us at 1,600 pixels, K = 3; 168 ->
+// 87, K = 5).
 // ---------------------------------------------------------------------------
 
-
-__device__ double det_lu(const double *ain, int n)
+template <int K>
+__device__ __forceinline__ double det_lu(const double *ain, int n_)
 {
+    const int n = K ? K : n_;
     // determinant by LU with partial pivoting (equal, up to rounding, to the
     // cofactor expansion of java:14752-14770)
-    double a[IMFCS_NPARAM * IMFCS_NPARAM];
+    constexpr int M = K ? K : IMFCS_NPARAM;
+    double a[M * M];
+#pragma unroll
     for (int i = 0; i < n * n; i++) a[i] = ain[i];
     double det = 1.0;
+#pragma unroll
     for (int c = 0; c < n; c++) {
         int p = c;
+        double top = fabs(a[c * n + c]);
+#pragma unroll
         for (int r = c + 1; r < n; r++)
-            if (fabs(a[r * n + c]) > fabs(a[p * n + c])) p = r;
-        if (a[p * n + c] == 0.0) return 0.0;
-        if (p != c) {
-            for (int q = 0; q < n; q++) { double t = a[c * n + q]; a[c * n + q] = a[p * n + q]; a[p * n + q] = t; }
-            det = -det;
-        }
+            if (fabs(a[r * n + c]) > top) { p = r; top = fabs(a[r * n + c]); }
+        double piv = a[c * n + c];
+#pragma unroll
+        for (int r = c + 1; r < n; r++)
+            if (r == p) piv = a[r * n + c];
+        if (piv == 0.0) return 0.0;
+#pragma unroll
+        for (int r = c + 1; r < n; r++)
+            if (r == p) {
+#pragma unroll
+                for (int q = 0; q < n; q++) { double t = a[c * n + q]; a[c * n + q] = a[r * n + q]; a[r * n + q] = t; }
+            }
+        if (p != c) det = -det;
         det *= a[c * n + c];
+#pragma unroll
         for (int r = c + 1; r < n; r++) {
             double f = a[r * n + c] / a[c * n + c];
+#pragma unroll
             for (int q = c; q < n; q++) a[r * n + q] -= f * a[c * n + q];
         }
     }
@@ -114,63 +136,130 @@ __device__ double det_lu(const double *ain, int n)
 }
 
 // Householder QR inverse with |R_ii| <= threshold -> singular.
-__device__ bool qr_inverse_d(const double *ain, int k, double threshold, double *inv)
+template <int K>
+__device__ __forceinline__ bool qr_inverse_d(const double *ain, int k_, double threshold, double *inv)
 {
-    double a[IMFCS_NPARAM * IMFCS_NPARAM], rdiag[IMFCS_NPARAM];
+    constexpr int M = K ? K : IMFCS_NPARAM;
+    const int k = K ? K : k_;
+    double a[M * M], rdiag[M];
+#pragma unroll
     for (int i = 0; i < k * k; i++) a[i] = ain[i];
+#pragma unroll
     for (int minor = 0; minor < k; minor++) {
         double xn = 0.0;
+#pragma unroll
         for (int r = minor; r < k; r++) xn += a[r * k + minor] * a[r * k + minor];
         double alpha = a[minor * k + minor] > 0 ? -sqrt(xn) : sqrt(xn);
         rdiag[minor] = alpha;
         if (alpha != 0.0) {
             a[minor * k + minor] -= alpha;
+#pragma unroll
             for (int c = minor + 1; c < k; c++) {
                 double ac = 0.0;
+#pragma unroll
                 for (int r = minor; r < k; r++) ac -= a[r * k + c] * a[r * k + minor];
                 ac /= alpha * a[minor * k + minor];
+#pragma unroll
                 for (int r = minor; r < k; r++) a[r * k + c] -= ac * a[r * k + minor];
             }
         }
     }
+#pragma unroll
     for (int i = 0; i < k; i++)
         if (!(fabs(rdiag[i]) > threshold)) return false;
+#pragma unroll
     for (int col = 0; col < k; col++) {
-        double y[IMFCS_NPARAM];
+        double y[M];
+#pragma unroll
         for (int i = 0; i < k; i++) y[i] = (i == col) ? 1.0 : 0.0;
+#pragma unroll
         for (int minor = 0; minor < k; minor++) {
             double dot = 0.0;
+#pragma unroll
             for (int r = minor; r < k; r++) dot += y[r] * a[r * k + minor];
             dot /= rdiag[minor] * a[minor * k + minor];
+#pragma unroll
             for (int r = minor; r < k; r++) y[r] += dot * a[r * k + minor];
         }
+#pragma unroll
         for (int i = k - 1; i >= 0; i--) {
             y[i] /= rdiag[i];
+#pragma unroll
             for (int r = 0; r < i; r++) y[r] -= y[i] * a[r * k + i];
         }
+#pragma unroll
         for (int i = 0; i < k; i++) inv[i * k + col] = y[i];
     }
     return true;
 }
 
+// Bayes: log-residual term of every fitted pixel (left in logp), a warp per
+// pixel; the sums in the order of one thread.
+constexpr int kResWarps = 4;
+__global__ void __launch_bounds__(32 * kResWarps) bayes_residual_kernel(EpilogueArgs e)
+{
+    __shared__ double tres_sh[kResWarps][kMaxChan], z_sh[kResWarps][kMaxChan];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int pix = blockIdx.x * kResWarps + wid;
+    if (pix >= e.npix) return;
+    double *tres = tres_sh[wid], *z = z_sh[wid];
+    float par[IMFCS_NPARAM];
+#pragma unroll
+    for (int i = 0; i < IMFCS_NPARAM; i++) par[i] = e.par_int[(size_t)pix * IMFCS_NPARAM + i];
+    const bool c2 = par[5] != 0.f, c3 = par[7] != 0.f;
+    // unweighted residuals of the fitted lags (tres)
+    for (int i = 1 + lane; i < e.chanum; i += 32) {
+        const bool in = e.gls || (i >= e.fitstart && i <= e.fitend);
+        const double v = in ? (double)fcs_model_f(par, e.mc, e.lagtime[i], nullptr, c2, c3) : 0.0;
+        tres[i - 1] = in ? e.acf[(size_t)pix * e.chanum + i] - v : 0.0;
+    }
+    __syncwarp();
+    double sum = 0.0;
+    if (!e.gls) {
+        if (lane == 0)
+            for (int i = 1; i < e.chanum - 1; i++) sum += tres[i] * tres[i];   // from index 1 (java:10170)
+    } else {
+        // tres^T covmats^-1 tres = |L^-1 tres|^2
+        const int n = e.chanum - 1;
+        const float *L = e.linv + (size_t)pix * n * (n + 1) / 2;
+        for (int i = lane; i < n; i += 32) {
+            const float *row = L + (size_t)i * (i + 1) / 2;
+            double zi = 0.0;
+            for (int c = 0; c <= i; c++) zi += (double)row[c] * tres[c];
+            z[i] = zi;
+        }
+        __syncwarp();
+        if (lane == 0)
+            for (int i = 0; i < n; i++) sum += z[i] * z[i];
+    }
+    if (lane == 0) e.logp[pix] = -0.5 * sum;
+}
+
+template <int K>
 __global__ void fit_epilogue_kernel(EpilogueArgs e)
 {
+    constexpr int M = K ? K : IMFCS_NPARAM;
     const int pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= e.npix) return;
     const float *pi = e.par_int + (size_t)pix * IMFCS_NPARAM;
     int st = e.state[pix];
     bool ok = (st == IMFCS_STATE_CONVERGED) && (!e.pre_ok || e.pre_ok[pix]);
-    double cov[IMFCS_NPARAM * IMFCS_NPARAM], jtj[IMFCS_NPARAM * IMFCS_NPARAM];
-    const int k = e.k;
+    double cov[M * M], jtj[M * M];
+    const int k = K ? K : e.k;
+#pragma unroll
     for (int aa = 0; aa < k; aa++)
+#pragma unroll
         for (int bb = 0; bb < k; bb++)
             jtj[aa * k + bb] = (double)e.hess[(size_t)pix * k * k + aa * k + bb] /
                                (param_unit(e.idx[aa]) * param_unit(e.idx[bb]));
-    if (ok) ok = qr_inverse_d(jtj, k, 1.0, cov);
-    for (int i = 0; i < k && ok; i++) ok = isfinite(cov[i * k + i]) && cov[i * k + i] > 0.0;
+    if (ok) ok = qr_inverse_d<K>(jtj, k, 1.0, cov);
+#pragma unroll
+    for (int i = 0; i < k; i++) ok = ok && isfinite(cov[i * k + i]) && cov[i * k + i] > 0.0;
     float *fr = e.fitres + (size_t)pix * IMFCS_NPARAM;
+#pragma unroll
     for (int i = 0; i < IMFCS_NPARAM; i++) {
         bool is_free = false;
+#pragma unroll
         for (int q = 0; q < k; q++) is_free |= (e.idx[q] == i);
         fr[i] = (ok || !is_free) ? (float)((double)pi[i] * param_unit(i)) : nanf("");
     }
@@ -182,34 +271,9 @@ __global__ void fit_epilogue_kernel(EpilogueArgs e)
         const double pi_j = 3.14159265359;
         double logresid, det, prodsig = 1.0;
         if (ok) {
-            // unweighted residuals of the fitted lags (tres)
-            double tres[kMaxChan];
-            float par[IMFCS_NPARAM];
-            for (int i = 0; i < IMFCS_NPARAM; i++) par[i] = pi[i];
-            bool c2 = par[5] != 0.f, c3 = par[7] != 0.f;
-            for (int i = 1; i < e.chanum; i++) {
-                bool in = e.gls || (i >= e.fitstart && i <= e.fitend);
-                double v = in ? (double)fcs_model_f(par, e.mc, e.lagtime[i], nullptr, c2, c3) : 0.0;
-                tres[i - 1] = in ? e.acf[(size_t)pix * e.chanum + i] - v : 0.0;
-            }
-            if (!e.gls) {
-                double rs = 0.0;
-                for (int i = 1; i < e.chanum - 1; i++) rs += tres[i] * tres[i];   // from index 1 (java:10170)
-                logresid = -0.5 * rs;
-            } else {
-                // tres^T covmats^-1 tres = |L^-1 tres|^2
-                const int n = e.chanum - 1;
-                const float *L = e.linv + (size_t)pix * n * (n + 1) / 2;
-                double s = 0.0;
-                for (int i = 0; i < n; i++) {
-                    const float *row = L + (size_t)i * (i + 1) / 2;
-                    double z = 0.0;
-                    for (int c = 0; c <= i; c++) z += (double)row[c] * tres[c];
-                    s += z * z;
-                }
-                logresid = -0.5 * s;
-            }
-            det = det_lu(cov, k);
+            logresid = e.logp[pix];                   // bayes_residual_kernel
+            det = det_lu<K>(cov, k);
+#pragma unroll
             for (int i = 0; i < k; i++) prodsig *= sqrt(cov[i * k + i]);
         } else {
             // failed fit: ones (java:10441-10466) -> det of the all-ones matrix
@@ -235,7 +299,11 @@ __global__ void bayes_combine_kernel(int npix, const double *lp1, const double *
 
 cudaError_t launch_fit_epilogue(const EpilogueArgs &e, cudaStream_t stream)
 {
-    fit_epilogue_kernel<<<(e.npix + 127) / 128, 128, 0, stream>>>(e);
+    if (e.logp) bayes_residual_kernel<<<(e.npix + kResWarps - 1) / kResWarps, 32 * kResWarps, 0, stream>>>(e);
+    const int blocks = (e.npix + 63) / 64;
+    if (e.k == 3) fit_epilogue_kernel<3><<<blocks, 64, 0, stream>>>(e);
+    else if (e.k == 5) fit_epilogue_kernel<5><<<blocks, 64, 0, stream>>>(e);
+    else fit_epilogue_kernel<0><<<blocks, 64, 0, stream>>>(e);
     return cudaGetLastError();
 }
 cudaError_t launch_ols_prepare(int npix, int chanum, int fitstart, int npts, const double *acf,
