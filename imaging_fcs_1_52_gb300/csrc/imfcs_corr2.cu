@@ -143,14 +143,28 @@ __device__ __forceinline__ void load16(float (&v)[16], const float *in, int n, i
     }
 }
 
-template <bool CCF, bool FIRST17, bool TWO, int NT>
-__global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const float *inA, const float *inB,
-                                                     float *outA, float *outB, int k)
+// PART: the pass's share of the lags -- 0 all, 1 the first level's (level 0:
+// its lags 0..8), 2 the second level's, with the samples it passes on, 3 lags
+// 9..16 of level 0.
+template <bool CCF, bool FIRST17, bool TWO, int NT, int PART>
+struct PairShare {
+    static constexpr int FB = PART == 3 ? 9 : 0;                      // first-level lags: from FB on,
+    static constexpr int NF = PART == 2 ? 0 : PART == 3 ? 8 : PART == 1 && FIRST17 ? 9 : FIRST17 ? kP + 1 : 8;
+    static constexpr int DF = (FIRST17 ? 0 : 9) + FB;                 // the delay of the first of them
+    static constexpr bool SECOND = TWO && (PART == 0 || PART == 2);
+    static constexpr int NS = SECOND ? 8 : 0;
+    static constexpr int LAG = PART == 2 ? (FIRST17 ? kP + 1 : 8) : FB;   // the share's first lag in the pair's
+    static constexpr int SMEM = (NF + NS) * kPairFields * NT;
+};
+
+template <bool CCF, bool FIRST17, bool TWO, int NT, int PART>
+__device__ __forceinline__ void pair_body(const C2Args &a, const float *inA, const float *inB, float *outA,
+                                          float *outB, int k, float *sm)
 {
-    constexpr int NF = FIRST17 ? kP + 1 : 8;          // first-level lags
-    constexpr int DF = FIRST17 ? 0 : 9;               // delay of the first of them
-    constexpr int NS = TWO ? 8 : 0;
-    __shared__ float sm[(NF + NS) * kPairFields * NT];
+    using Share = PairShare<CCF, FIRST17, TWO, NT, PART>;
+    constexpr int NF = Share::NF, DF = Share::DF, NS = Share::NS;
+    constexpr bool SECOND = Share::SECOND;
+    constexpr int NFA = NF ? NF : 1;
     const int tid = threadIdx.x;
     const int pix = blockIdx.x * NT + tid, seg = blockIdx.y;
     const int s0 = seg << a.seg_log[k];
@@ -161,7 +175,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
     const int y0 = s0 >> k, y1 = s1 >= a.num ? nk : (s1 >> k);      // direct samples of level k
     const int ind = a.blk_ind[pix];
     const int LF = 1 << (ind - k), LS = 1 << (ind - k - 1);
-    const int lag0 = FIRST17 ? 0 : (kP + 1) + (k - 1) * 8;
+    const int lag0 = (FIRST17 ? 0 : (kP + 1) + (k - 1) * 8) + Share::LAG;
     float *gst = a.o.stats + (size_t)seg * a.stat_stride;
     PairBlocks<NT> pb;
     pb.sm = sm + tid;
@@ -172,7 +186,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
     pb.pnum_stride = a.o.pnum_stride;
     pb.pnum = a.li->pnum_by_ind[ind];
     pb.zfirst = s0 >> ind;
-    pb.skip0 = FIRST17;
+    pb.skip0 = FIRST17 && Share::LAG == 0;
 #pragma unroll
     for (int l = 0; l < NF + NS; l++)
 #pragma unroll
@@ -190,7 +204,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
     float w[32], cur[16];              // first-level samples y .. y+31; the next 16, loading
     float x[16];                       // CCF: direct-trace samples y .. y+15
     float r[24], rx[8];                // second-level samples y/2-8 .. y/2+15; CCF: direct ones y/2-8 .. y/2-1
-    float accF[NF], accS[8];
+    float accF[NFA], accS[8];
     float bF = 0.f, bFd = 0.f, bS = 0.f, bSd = 0.f;
 #pragma unroll
     for (int l = 0; l < NF; l++) accF[l] = 0.f;
@@ -207,22 +221,22 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
     // heads of the first blocks, and the second level's first eight samples
     {
         float h = 0.f;
-        if (FIRST17) pb.at(0, 4) = 0.f;
+        if (DF == 0 && NF) pb.at(0, 4) = 0.f;
 #pragma unroll
         for (int d = 1; d <= kP; d++) {
             h += w[16 + d - 1];
-            if (d >= DF) pb.at(d - DF, 4) = h;
+            if (d >= DF && d < DF + NF) pb.at(d - DF, 4) = h;
         }
-        if (TWO)
+        if (SECOND)
 #pragma unroll
             for (int i = 0; i < 8; i++) r[16 + i] = (y0 >> 1) + i < nk1 ? w[16 + 2 * i] + w[17 + 2 * i] : 0.f;
     }
     // one step more than first-level steps: the second level is a step behind
     const int ysteps = y0 + ((y1 - y0 + 15) & ~15);
 #pragma unroll 1
-    for (int y = y0; y < ysteps + (TWO ? 16 : 0); y += 16) {
+    for (int y = y0; y < ysteps + (SECOND ? 16 : 0); y += 16) {
         const bool first_level = y < ysteps;
-        const bool second_level = TWO && y > y0;
+        const bool second_level = SECOND && y > y0;
         float xn[8];                   // CCF: second-level direct samples of this step
 #pragma unroll
         for (int i = 0; i < 16; i++) {
@@ -231,7 +245,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
         }
         if (CCF) load16(x, inA, y, nk, a.npix);
         load16(cur, inB, y + 32, nk, a.npix);
-        if (TWO) {
+        if (SECOND) {
 #pragma unroll
             for (int i = 0; i < 16; i++) r[i] = r[i + 8];
 #pragma unroll
@@ -241,6 +255,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
                 for (int i = 0; i < 8; i++) xn[i] = (y >> 1) + i < nk1 ? x[2 * i] + x[2 * i + 1] : 0.f;
         }
         if (first_level) {
+            if (NF)
 #pragma unroll
             for (int j = 0; j < 16; j++) {
                 const float d = CCF ? x[j] : w[j];
@@ -249,7 +264,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
                 bF += d;
                 if (CCF) bFd += w[j];
             }
-            if (TWO && outB) {         // level k+2: pair sums of second-level samples y/2 .. y/2+7
+            if (SECOND && outB) {      // level k+2: pair sums of second-level samples y/2 .. y/2+7
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int m = (y >> 2) + i;
@@ -259,15 +274,15 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
                     }
                 }
             }
-            if (((y + 16) & (LF - 1)) == 0) {
-                float nh[NF], h = 0.f;
-                if (FIRST17) nh[0] = 0.f;
+            if (NF && ((y + 16) & (LF - 1)) == 0) {
+                float nh[NFA], h = 0.f;
+                if (DF == 0) nh[0] = 0.f;
 #pragma unroll
                 for (int d = 1; d <= kP; d++) {
                     h += w[16 + d - 1];
-                    if (d >= DF) nh[d - DF] = h;
+                    if (d >= DF && d < DF + NF) nh[d - DF] = h;
                 }
-                pb.template end<NF>(0, accF, bF, CCF ? bFd : bF, nh, LF, (y + 16) / LF - 1);
+                pb.template end<NFA>(0, accF, bF, CCF ? bFd : bF, nh, LF, (y + 16) / LF - 1);
                 bF = 0.f;
                 bFd = 0.f;
             }
@@ -292,7 +307,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
                 bS = 0.f;
                 bSd = 0.f;
             }
-        } else if (TWO) {              // the first step: heads of the second level's first block
+        } else if (SECOND) {           // the first step: heads of the second level's first block
             float h = 0.f;
 #pragma unroll
             for (int d = 1; d <= 16; d++) {
@@ -300,7 +315,7 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
                 if (d >= 9) pb.at(NF + d - 9, 4) = h;
             }
         }
-        if (CCF && TWO)
+        if (CCF && SECOND)
 #pragma unroll
             for (int i = 0; i < 8; i++) rx[i] = xn[i];
     }
@@ -314,6 +329,28 @@ __global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const f
         stat_ref(gst, a.npix, lag0 + l, 2, pix) = pb.at(l, 2);
         stat_ref(gst, a.npix, lag0 + l, 3, pix) = pb.at(l, 3);
     }
+}
+
+template <bool CCF, bool FIRST17, bool TWO, int NT>
+__global__ void __launch_bounds__(NT, 384 / NT) c2_pair_kernel(C2Args a, const float *inA, const float *inB,
+                                                     float *outA, float *outB, int k)
+{
+    __shared__ float sm[PairShare<CCF, FIRST17, TWO, NT, 0>::SMEM];
+    pair_body<CCF, FIRST17, TWO, NT, 0>(a, inA, inB, outA, outB, k, sm);
+}
+
+// The same with a pair's lags dealt out to two or three blocks (blockIdx.z),
+// each reading the samples for itself: for grids that leave the SMs part-empty,
+// where a block's time is the latency of its instructions.  The sums are per
+// lag, so they stay what they are.
+template <bool CCF, bool FIRST17, int NT>
+__global__ void __launch_bounds__(NT, 384 / NT) c2_pair_split_kernel(C2Args a, const float *inA, const float *inB,
+                                                           float *outA, float *outB, int k)
+{
+    __shared__ float sm[9 * kPairFields * NT];
+    if (blockIdx.z == 0) pair_body<CCF, FIRST17, true, NT, 2>(a, inA, inB, outA, outB, k, sm);
+    else if (blockIdx.z == 1) pair_body<CCF, FIRST17, true, NT, 1>(a, inA, inB, outA, outB, k, sm);
+    else if (FIRST17) pair_body<CCF, FIRST17, true, NT, FIRST17 ? 3 : 1>(a, inA, inB, outA, outB, k, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -928,13 +965,29 @@ size_t corr_stream_floats(const Job &j)
 // The corrected level-0 stream s0[trace][frame][pixel] (imfcs_stream.cu).
 size_t level0_stream_floats(const Job &j) { return (size_t)(j.is_ccf ? 2 : 1) * j.npix * j.num; }
 
+// Threads up to which a grid takes the split pair kernels (levels 0-1: three
+// blocks, above: two; 152 SMs hold 58,368).  Measured, whole -> split: levels
+// 0-1, 2,560 threads 144 -> 83 us (20,000 frames), 13,312 277 -> 188 (50,000),
+// 23,040 158 -> 199 (20,000); levels 2-3, 2,560 46 -> 30, 23,040 56 -> 37,
+// 40,960 62 -> 69.
+constexpr int kSplitThreads[2] = {256 * 64, 480 * 64};
+
 // One pair kernel of the chain: variant 0 = levels 0-1, 1 = two upper
 // levels, 2 = one upper level (the last).
 template <int NT>
 static void launch_pair(bool ccf, int variant, dim3 grid, cudaStream_t stream, const C2Args &a, const float *ia,
                         const float *ib, float *oa, float *ob, int k)
 {
-    if (ccf) {
+    if (variant < 2 && (long long)grid.x * grid.y * NT <= kSplitThreads[variant]) {
+        grid.z = variant == 0 ? 3 : 2;
+        if (ccf) {
+            if (variant == 0) c2_pair_split_kernel<true, true, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
+            else c2_pair_split_kernel<true, false, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
+        } else {
+            if (variant == 0) c2_pair_split_kernel<false, true, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
+            else c2_pair_split_kernel<false, false, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
+        }
+    } else if (ccf) {
         if (variant == 0) c2_pair_kernel<true, true, true, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
         else if (variant == 1) c2_pair_kernel<true, false, true, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
         else c2_pair_kernel<true, false, false, NT><<<grid, NT, 0, stream>>>(a, ia, ib, oa, ob, k);
