@@ -86,50 +86,6 @@ __device__ __forceinline__ float gls_sig(const float *s, int i)
     return rsqrtf(fmaxf(s[i * (i + 3) / 2], 1e-30f));
 }
 
-// solve_scaled with its roundings spelled out (where its products are fused
-// into the sums depends on the code around it).
-__device__ __forceinline__ bool gls_solve(const float (&A)[9], const float (&g)[3], float lambda, float (&h)[3])
-{
-    float sc[3], L[9];
-#pragma unroll
-    for (int i = 0; i < 3; i++) sc[i] = rsqrtf(fmaxf(A[i * 3 + i], 1e-30f));
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        float d = 1.f + lambda;
-#pragma unroll
-        for (int m = 0; m < c; m++) d = fmaf(-L[c * 3 + m], L[c * 3 + m], d);
-        if (!(d > 0.f) || !isfinite(d)) return false;
-        d = sqrtf(d);
-        L[c * 3 + c] = d;
-        const float id = 1.f / d;
-#pragma unroll
-        for (int r = c + 1; r < 3; r++) {
-            float sum = __fmul_rn(__fmul_rn(A[r * 3 + c], sc[r]), sc[c]);
-#pragma unroll
-            for (int m = 0; m < c; m++) sum = fmaf(-L[r * 3 + m], L[c * 3 + m], sum);
-            L[r * 3 + c] = __fmul_rn(sum, id);
-        }
-    }
-    float yv[3], z[3];
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        float sum = r ? fmaf(g[r], sc[r], -__fmul_rn(L[r * 3], yv[0])) : __fmul_rn(g[0], sc[0]);
-#pragma unroll
-        for (int m = 1; m < r; m++) sum = fmaf(-L[r * 3 + m], yv[m], sum);
-        yv[r] = sum / L[r * 3 + r];
-    }
-#pragma unroll
-    for (int r = 2; r >= 0; r--) {
-        float sum = yv[r];
-#pragma unroll
-        for (int m = r + 1; m < 3; m++) sum = fmaf(-L[m * 3 + r], z[m], sum);
-        z[r] = sum / L[r * 3 + r];
-    }
-#pragma unroll
-    for (int r = 0; r < 3; r++) h[r] = __fmul_rn(z[r], sc[r]);
-    return true;
-}
-
 // One warp, one block per fit.
 template <bool OFF>
 __global__ void __launch_bounds__(32, 16) lm_gls_kernel(FitArgs a)
@@ -345,7 +301,7 @@ __global__ void __launch_bounds__(32, 16) lm_gls_kernel(FitArgs a)
                 bool ok = false;
 #pragma unroll 1
                 for (int pass = fresh ? 0 : 1; pass < 2; pass++) {
-                    ok = gls_solve(A, gv, pass ? lambda : 0.f, h);
+                    ok = tirf_solve(A, gv, pass ? lambda : 0.f, h);
                     if (pass == 0 && ok) {
                         bool conv = true;
 #pragma unroll
@@ -422,7 +378,7 @@ __global__ void __launch_bounds__(32, 16) lm_gls_kernel(FitArgs a)
                     for (int i = 0; i < 9; i++) H[i] = sh.H[i];
 #pragma unroll
                     for (int i = 0; i < 3; i++) gv[i] = sh.s[0][6 + i];
-                    if (!gls_solve(H, gv, 0.f, hn)) { left = true; break; }
+                    if (!tirf_solve(H, gv, 0.f, hn)) { left = true; break; }
                     bool small = true;
 #pragma unroll
                     for (int i = 0; i < 3; i++) {

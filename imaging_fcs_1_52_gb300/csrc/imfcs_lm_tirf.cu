@@ -53,21 +53,34 @@ __device__ __forceinline__ void tirf_accumulate(float (&acc)[9], const float (&g
 // One evaluation over the fit's points (warp): chi^2, J^T W J, J^T W r with
 // FP32 residuals.  No FP64 operation: GB300 issues FP64 at 1/64 of the FP32
 // rate, and the FP32 phases evaluate the model some twenty times per fit.
-template <bool OFF>
+template <bool OFF, bool SIDE>
 __device__ __noinline__ void tirf_eval32(const TirfC &c, float N, float D, float G, const float *yl,
-                                         const float *wl, const float *xl, int n, int lane, Tirf3 &s)
+                                         const float *wl, const float *xl, int n, int lane, Tirf3 &s,
+                                         float bound)
 {
     float acc[9];
 #pragma unroll
     for (int i = 0; i < 9; i++) acc[i] = 0.f;
     float c2f = 0.f, fm = 0.f;
+    constexpr int kSide = SIDE && !OFF ? 3 : 0;     // a lane's first points, their chains side by side
+    float sf[3], sN[3], sD[3], sm[3];
+#pragma unroll
+    for (int m = 0; m < kSide; m++) sf[m] = tirf_f<OFF, true>(N, D, G, c, xl[m], sN[m], sD[m], sm[m]);
 #pragma unroll
     for (int m = 0; m < kPtsPerLane; m++) {
         const int i = lane + 32 * m;
         if (i < n) {
             float gr[3], mag;
             gr[2] = 1.f;
-            const float f = tirf_f<OFF>(N, D, G, c, xl[m], gr[0], gr[1], mag);
+            float f;
+            if (m < kSide) {
+                f = sf[m];
+                gr[0] = sN[m];
+                gr[1] = sD[m];
+                mag = sm[m];
+            } else {
+                f = tirf_f<OFF>(N, D, G, c, xl[m], gr[0], gr[1], mag);
+            }
             const float w = wl[m];
             const float r = yl[m] - f;
             c2f = fmaf(w * r, r, c2f);
@@ -75,16 +88,17 @@ __device__ __noinline__ void tirf_eval32(const TirfC &c, float N, float D, float
             tirf_accumulate(acc, gr, w, r);
         }
     }
-    tirf_reduce(acc, s);
     s.chi2 = warp_sum(c2f);
     s.chi2d = 0.0;
+    if (!(s.chi2 < bound)) return;      // a rejected step: nobody reads the sums
+    tirf_reduce(acc, s);
     s.fmag = warp_sum(fm);
 }
 
 // The same with residuals of the model value in float-float at the FP64
 // parameters (Nd, Dd, Gd) -- FP64 model where the series do not apply --
 // the Jacobian in FP32 at their FP32 copies; chi^2 reduced in float-float.
-template <bool OFF>
+template <bool OFF, bool SIDE>
 __device__ __noinline__ void tirf_eval64(const TirfC &c, double Nd, double Dd, double Gd, const float *yl,
                                          const float *wl, const float *xl, int n, int lane, Tirf3 &s)
 {
@@ -123,13 +137,13 @@ __device__ __noinline__ void tirf_eval64(const TirfC &c, double Nd, double Dd, d
 }
 
 // dispatch by phase
-template <bool OFF>
+template <bool OFF, bool SIDE>
 __device__ __forceinline__ void tirf_eval(const TirfC &c, float N, float D, float G, double Nd, double Dd, double Gd,
                                           const float *yl, const float *wl, const float *xl, int n, int lane,
-                                          bool precise, Tirf3 &s)
+                                          bool precise, Tirf3 &s, float bound = INFINITY)
 {
-    if (precise) tirf_eval64<OFF>(c, Nd, Dd, Gd, yl, wl, xl, n, lane, s);
-    else tirf_eval32<OFF>(c, N, D, G, yl, wl, xl, n, lane, s);
+    if (precise) tirf_eval64<OFF, SIDE>(c, Nd, Dd, Gd, yl, wl, xl, n, lane, s);
+    else tirf_eval32<OFF, SIDE>(c, N, D, G, yl, wl, xl, n, lane, s, bound);
 }
 
 __device__ __forceinline__ float tirf_sig(const Tirf3 &s, int i) { return rsqrtf(fmaxf(s.A[i * 3 + i], 1e-30f)); }
@@ -139,7 +153,7 @@ __device__ __forceinline__ float tirf_sig(const Tirf3 &s, int i) { return rsqrtf
 // terms): 4e-6, some 70 ulp.
 constexpr float kModelRound = 4e-6f;
 
-template <bool OFF>
+template <bool OFF, bool SIDE>
 __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -170,16 +184,26 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
         bool precise = false;     // parameters and chi^2 held in FP64 (pd, chi2d)
         bool retried = false;     // Newton left its region once: FP32 LM to 1e-4 sigma, then Newton again
         Tirf3 s;
-        tirf_eval<OFF>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
+        tirf_eval<OFF, SIDE>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
         int state = IMFCS_STATE_MAX_ITERATIONS, it = 0, nprec = 0;
         float lambda = 1e-3f;
         if (!isfinite(s.chi2)) state = IMFCS_STATE_SINGULAR_HESSIAN;
         for (it = 0; state == IMFCS_STATE_MAX_ITERATIONS && it < a.max_iter; it++) {
             float h[3];
-            bool to_precise = false;
+            bool to_precise = false, ok;
             {
-                float hg[3];
-                if (solve_scaled<3>(s.A, s.g, 3, 0.f, hg)) {
+                // the undamped step of the stopping test and the damped one,
+                // each in half of the warp: a solve is one long chain
+                float hs[3], hg[3];
+                const bool oks = tirf_solve(s.A, s.g, lane < 16 ? 0.f : lambda, hs);
+                const unsigned votes = __ballot_sync(0xffffffffu, oks);
+                ok = votes >> 16 & 1;
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    hg[i] = __shfl_sync(0xffffffffu, hs[i], 0);
+                    h[i] = __shfl_sync(0xffffffffu, hs[i], 16);
+                }
+                if (votes & 1) {
                     bool conv = true;
 #pragma unroll
                     for (int i = 0; i < 3; i++) {
@@ -194,7 +218,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                 }
             }
             if (!to_precise) {
-                if (!solve_scaled<3>(s.A, s.g, 3, lambda, h)) {
+                if (!ok) {
                     lambda *= 10.f;
                     if (lambda > 1e15f) { state = IMFCS_STATE_SINGULAR_HESSIAN; break; }
                     continue;
@@ -206,13 +230,13 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                 if (precise) {
 #pragma unroll
                     for (int i = 0; i < 3; i++) { pnd[i] = pd[i] + (double)h[i]; pnf[i] = (float)pnd[i]; }
-                    tirf_eval<OFF>(c, pnf[0], pnf[1], pnf[2], pnd[0], pnd[1], pnd[2], yl, wl, xl, n, lane, true, sn);
+                    tirf_eval<OFF, SIDE>(c, pnf[0], pnf[1], pnf[2], pnd[0], pnd[1], pnd[2], yl, wl, xl, n, lane, true, sn);
                     nprec++;
                     better = isfinite(sn.chi2d) && sn.chi2d < s.chi2d;
                 } else {
 #pragma unroll
                     for (int i = 0; i < 3; i++) pnf[i] = pf[i] + h[i];
-                    tirf_eval<OFF>(c, pnf[0], pnf[1], pnf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, sn);
+                    tirf_eval<OFF, SIDE>(c, pnf[0], pnf[1], pnf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, sn, s.chi2);
                     better = isfinite(sn.chi2) && sn.chi2 < s.chi2;
                 }
                 if (better) {
@@ -242,7 +266,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                     pe[i] = pf[i] + eps;
                     const float de = pe[i] - pf[i];
                     Tirf3 se;
-                    tirf_eval<OFF>(c, pe[0], pe[1], pe[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, se);
+                    tirf_eval<OFF, SIDE>(c, pe[0], pe[1], pe[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, se);
 #pragma unroll
                     for (int r = 0; r < 3; r++) H[r * 3 + i] = (s.g[r] - se.g[r]) / de;
                 }
@@ -281,7 +305,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                             for (int i = 0; i < 3; i++) pd[i] = (double)pf[i];
                             precise = true;
                         }
-                        tirf_eval<OFF>(c, pf[0], pf[1], pf[2], pd[0], pd[1], pd[2], yl, wl, xl, n, lane, true, s);
+                        tirf_eval<OFF, SIDE>(c, pf[0], pf[1], pf[2], pd[0], pd[1], pd[2], yl, wl, xl, n, lane, true, s);
                         if (!isfinite(s.chi2d)) { left = true; break; }
                     }
                     float hn[3];
@@ -305,7 +329,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                             ni = 2;
                             stationary = true;
                         } else {
-                            tirf_eval<OFF>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
+                            tirf_eval<OFF, SIDE>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
                         }
                     }
                 }
@@ -323,7 +347,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                         for (int i = 0; i < 3; i++) pf[i] = (float)pd[i];
                         precise = false;
                     }
-                    tirf_eval<OFF>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
+                    tirf_eval<OFF, SIDE>(c, pf[0], pf[1], pf[2], 0.0, 0.0, 0.0, yl, wl, xl, n, lane, false, s);
                     lambda = 1e-3f;
                     continue;
                 }
@@ -333,7 +357,7 @@ __global__ void __launch_bounds__(128) lm_tirf_kernel(FitArgs a)
                     for (int i = 0; i < 3; i++) pd[i] = (double)pf[i];
                     precise = true;
                 }
-                tirf_eval<OFF>(c, pf[0], pf[1], pf[2], pd[0], pd[1], pd[2], yl, wl, xl, n, lane, true, s);
+                tirf_eval<OFF, SIDE>(c, pf[0], pf[1], pf[2], pd[0], pd[1], pd[2], yl, wl, xl, n, lane, true, s);
                 lambda = 1e-3f;
             }
         }
@@ -366,8 +390,12 @@ bool lm_tirf_applies(const FitArgs &a, bool tirf_zero_held)
 
 cudaError_t launch_lm_tirf(const FitArgs &a, int blocks, int threads, cudaStream_t s)
 {
-    if (a.mc.rx != 0.f || a.mc.ry != 0.f) lm_tirf_kernel<true><<<blocks, threads, 0, s>>>(a);
-    else lm_tirf_kernel<false><<<blocks, threads, 0, s>>>(a);
+    // Three points of a lane side by side shorten a fit's chain but fill the
+    // instruction caches: 64 fits 78 -> 72 us, 441 97 -> 89, 2,304 510 -> 507,
+    // 16,384 (the SMs full) 401 -> 449
+    if (a.mc.rx != 0.f || a.mc.ry != 0.f) lm_tirf_kernel<true, false><<<blocks, threads, 0, s>>>(a);
+    else if (a.nfits <= 4096) lm_tirf_kernel<false, true><<<blocks, threads, 0, s>>>(a);
+    else lm_tirf_kernel<false, false><<<blocks, threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -72,15 +72,34 @@ static __device__ __noinline__ void tirf_terms(float D, const TirfC &c, float ta
     da = dlat * psp + lat * dpsp;
 }
 
+// The same inline, without offset, for the points of a lane side by side.
+__device__ __forceinline__ void tirf_terms_plain(float D, const TirfC &c, float tau, float &a, float &da)
+{
+    const float p0 = sqrtf(fmaf(4.f * D, tau, c.s2));
+    const float inv_p0 = 1.f / p0;
+    float Lx, dLx, Ly, dLy;
+    tirf_lat(c.ax, p0, inv_p0, Lx, dLx);
+    if (c.square) { Ly = Lx; dLy = dLx; }
+    else tirf_lat(c.ay, p0, inv_p0, Ly, dLy);
+    const float dp0 = 2.f * tau * inv_p0;
+    const float lat = Lx * Ly * c.inv_norm;
+    const float dlat = fmaf(dLx, Ly, __fmul_rn(Lx, dLy)) * dp0 * c.inv_norm;   // rounded as in tirf_terms
+    const float psp = rsqrtf(fmaf(4.f * D * tau, c.inv_sz2, 1.f));
+    const float dpsp = -2.f * tau * c.inv_sz2 * psp * psp * psp;
+    a = lat * psp;
+    da = dlat * psp + lat * dpsp;
+}
+
 // Model value and gradient (d/dN, d/dD; d/dG = 1) in FP32, internal units;
 // mag = |a/N| + |G|, the magnitude of the summed terms (the rounding error
 // of the value is relative to it).
-template <bool OFF>
+template <bool OFF, bool INLINE = false>
 __device__ __forceinline__ float tirf_f(float N, float D, float G, const TirfC &c, float tau, float &gN, float &gD,
                                         float &mag)
 {
     float a, da;
-    tirf_terms<OFF>(D, c, tau, a, da);
+    if (INLINE) tirf_terms_plain(D, c, tau, a, da);
+    else tirf_terms<OFF>(D, c, tau, a, da);
     const float iN = 1.f / N;
     gN = -a * iN * iN;
     gD = iN * da;
@@ -197,6 +216,50 @@ __device__ __forceinline__ bool tirf_a_ff(f2 D, const TirfC &c, float tau, f2 &l
     if (c.square) Ly = Lx;
     else if (!tirf_lat_ff(c.ay, p0, ip0, Ly)) return false;
     lat = f2_mul(f2_mul(Lx, Ly), c.inv_normf);
+    return true;
+}
+
+// solve_scaled with its roundings spelled out (where its products are fused
+// into the sums depends on the code around it).
+__device__ __forceinline__ bool tirf_solve(const float (&A)[9], const float (&g)[3], float lambda, float (&h)[3])
+{
+    float sc[3], L[9];
+#pragma unroll
+    for (int i = 0; i < 3; i++) sc[i] = rsqrtf(fmaxf(A[i * 3 + i], 1e-30f));
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        float d = 1.f + lambda;
+#pragma unroll
+        for (int m = 0; m < c; m++) d = fmaf(-L[c * 3 + m], L[c * 3 + m], d);
+        if (!(d > 0.f) || !isfinite(d)) return false;
+        d = sqrtf(d);
+        L[c * 3 + c] = d;
+        const float id = 1.f / d;
+#pragma unroll
+        for (int r = c + 1; r < 3; r++) {
+            float sum = __fmul_rn(__fmul_rn(A[r * 3 + c], sc[r]), sc[c]);
+#pragma unroll
+            for (int m = 0; m < c; m++) sum = fmaf(-L[r * 3 + m], L[c * 3 + m], sum);
+            L[r * 3 + c] = __fmul_rn(sum, id);
+        }
+    }
+    float yv[3], z[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        float sum = r ? fmaf(g[r], sc[r], -__fmul_rn(L[r * 3], yv[0])) : __fmul_rn(g[0], sc[0]);
+#pragma unroll
+        for (int m = 1; m < r; m++) sum = fmaf(-L[r * 3 + m], yv[m], sum);
+        yv[r] = sum / L[r * 3 + r];
+    }
+#pragma unroll
+    for (int r = 2; r >= 0; r--) {
+        float sum = yv[r];
+#pragma unroll
+        for (int m = r + 1; m < 3; m++) sum = fmaf(-L[m * 3 + r], z[m], sum);
+        z[r] = sum / L[r * 3 + r];
+    }
+#pragma unroll
+    for (int r = 0; r < 3; r++) h[r] = __fmul_rn(z[r], sc[r]);
     return true;
 }
 

@@ -30,3 +30,16 @@ def test_small_and_large_grids_agree(stack, kw, w, h):
         out.append([np.asarray(r[k]).reshape(ch - dy, cw - dx, -1)[:h, :w] for k in ("acf", "var", "blocked_ind")])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(fitstart=2, fitend=40), dict(p=32, q=5),
+                                dict(cst=engine.model_constants(sz_um=1.0))], ids=["plain", "range", "p32", "spim"])
+def test_few_and_many_fits_agree(stack, kw):
+    """More than 4,096 fits and few take different instances of the fit kernel."""
+    out = []
+    for w, h in ((W, H), (14, 11)):
+        cfg = engine.FCSConfig(width=w, height=h, frames=9000, background=100, **kw)
+        r = engine.run_host(np.ascontiguousarray(stack[:, :h, :w]), cfg)
+        out.append([np.asarray(r[k]).reshape(h, w, -1)[:11, :14] for k in ("fitres", "chi2", "fitted", "iterations")])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a.view(np.int32), b.view(np.int32))
