@@ -732,13 +732,11 @@ __global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *
     float chi2f = exp_normal32<K>(y, n, dts, iy, pf, A, gf, lane);
     const bool ok = isfinite(chi2f);
     int evals = 1, rejected = 0;
-    unsigned fix = 0;
-    bool gn_near = false;      // Gauss-Newton step within 0.05 sigma
-    bool fresh = true;         // the Gauss-Newton step stays what it was after a rejected one
     for (int it_n = 0; ok && it_n < 100; it_n++) {
         float h[K];
-        if (fresh) gn_near = false;
-        if (fresh && exp_newton_step32<K>(A, gf, pf, fix, h)) {
+        unsigned fix;
+        bool gn_near = false;      // Gauss-Newton step within 0.05 sigma
+        if (exp_newton_step32<K>(A, gf, pf, fix, h)) {
             bool conv = true;
             gn_near = true;
             for (int a = 0; a < K; a++) {
@@ -749,7 +747,6 @@ __global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *
             }
             if (conv) break;
         }
-        fresh = false;
         if (!solve_scaled_k<K>(A, gf, lambda, fix, h)) {
             lambda *= 10.f;
             if (lambda > 1e10f) break;
@@ -767,7 +764,6 @@ __global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *
             chi2f = c2n;
             lambda = fmaxf(lambda * 0.1f, 1e-12f);
             rejected = 0;
-            fresh = true;
         } else {
             // two rejected steps in a row while the Gauss-Newton step is
             // within 0.05 sigma: FP32 chi^2 no longer resolves the descent
