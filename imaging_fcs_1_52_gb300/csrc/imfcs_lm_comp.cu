@@ -20,11 +20,11 @@
 //   - chi^2 first: a rejected step ends there, without the sums of the
 //     normal equations and, on the FP64 model, without the gradient;
 //   - the undamped step behind the stopping test is not solved again after a
-//     rejected step;
+//     rejected step, and beside the damped one where it is (5.15 -> 4.87 ms);
 //   - the sums over the warp as one transposed reduction (same tree);
 //   - FP64 model values two lanes a point, one component each: 5 rounds for
 //     72 points, not 6.
-// 1,600 fits of 72 points, K = 5: 14.2 -> 5.0 ms, then bound by the FP64 pipe
+// 1,600 fits of 72 points, K = 5: 14.2 -> 4.9 ms, then bound by the FP64 pipe
 // (60 % busy) and the longest fits.  16,384 fits, K = 3: 3.05 -> 1.09 ms.
 #include "imfcs_lm.cuh"
 
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(32) lm_comp_kernel(FitArgs a)
             // the damped one; one copy of the solver for both
             while (!newton && !to_precise) {
                 if (it >= a.max_iter) { done = true; break; }
-                float A[K * K], gv[K], h[K], sig[K];
+                float A[K * K], gv[K], h[K];
                 {
                     int q = 0;
 #pragma unroll
@@ -364,23 +364,27 @@ __global__ void __launch_bounds__(32) lm_comp_kernel(FitArgs a)
 #pragma unroll
                     for (int i = 0; i < K; i++) gv[i] = sh.s[0][q++];
                 }
-                bool ok = false;
-#pragma unroll 1
-                for (int pass = fresh && !GPUFIT ? 0 : 1; pass < 2; pass++) {
-                    ok = comp_solve<K>(A, gv, pass ? lambda : 0.f, h);
-                    if (pass == 0 && ok) {
-                        bool conv = true;
+                // the undamped solve in the warp's lower half beside the damped
+                // one in the upper: a solve is one long chain
+                const bool test = fresh && !GPUFIT;
+                float hs[K];
+                const bool oks = comp_solve<K>(A, gv, test && lane < 16 ? 0.f : lambda, hs);
+                const unsigned votes = __ballot_sync(0xffffffffu, oks);
+                const bool ok = votes >> 16 & 1;
 #pragma unroll
-                        for (int i = 0; i < K; i++) {
-                            sig[i] = rsqrtf(fmaxf(A[i * K + i], 1e-30f));
-                            const float tol = precise ? 1e-7f * fabsf(p[i]) + 1e-5f * sig[i] : 1e-3f * sig[i];
-                            conv = conv && (fabsf(h[i]) <= tol);
-                        }
-                        if (conv) {
-                            if (precise) { state = IMFCS_STATE_CONVERGED; done = true; }
-                            else to_precise = true;
-                            break;
-                        }
+                for (int i = 0; i < K; i++) h[i] = __shfl_sync(0xffffffffu, hs[i], 16);
+                if (test && (votes & 1)) {
+                    bool conv = true;
+#pragma unroll
+                    for (int i = 0; i < K; i++) {
+                        const float sig = rsqrtf(fmaxf(A[i * K + i], 1e-30f));
+                        const float tol = precise ? 1e-7f * fabsf(p[i]) + 1e-5f * sig : 1e-3f * sig;
+                        const float hg = __shfl_sync(0xffffffffu, hs[i], 0);
+                        conv = conv && (fabsf(hg) <= tol);
+                    }
+                    if (conv) {
+                        if (precise) { state = IMFCS_STATE_CONVERGED; done = true; }
+                        else to_precise = true;
                     }
                 }
                 if (done || to_precise) break;

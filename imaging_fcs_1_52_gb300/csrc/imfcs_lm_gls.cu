@@ -298,24 +298,28 @@ __global__ void __launch_bounds__(32, 16) lm_gls_kernel(FitArgs a)
 #pragma unroll
                     for (int i = 0; i < 3; i++) gv[i] = sh.s[0][q++];
                 }
-                bool ok = false;
-#pragma unroll 1
-                for (int pass = fresh ? 0 : 1; pass < 2; pass++) {
-                    ok = tirf_solve(A, gv, pass ? lambda : 0.f, h);
-                    if (pass == 0 && ok) {
-                        bool conv = true;
+                // the undamped solve in the warp's lower half beside the damped
+                // one in the upper: a solve is one long chain
+                const bool test = fresh;
+                float hs[3];
+                const bool oks = tirf_solve(A, gv, test && lane < 16 ? 0.f : lambda, hs);
+                const unsigned votes = __ballot_sync(0xffffffffu, oks);
+                const bool ok = votes >> 16 & 1;
 #pragma unroll
-                        for (int i = 0; i < 3; i++) {
-                            const float sig = gls_sig(sh.s[0], i);
-                            const float tol = precise ? 1e-7f * fabsf(pf[i]) + 1e-5f * sig
-                                                      : (retried ? 1e-4f : 1e-3f) * sig;
-                            conv = conv && (fabsf(h[i]) <= tol);
-                        }
-                        if (conv) {
-                            if (precise) { state = IMFCS_STATE_CONVERGED; done = true; }
-                            else to_precise = true;
-                            break;
-                        }
+                for (int i = 0; i < 3; i++) h[i] = __shfl_sync(0xffffffffu, hs[i], 16);
+                if (test && (votes & 1)) {
+                    bool conv = true;
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        const float sig = gls_sig(sh.s[0], i);
+                        const float tol = precise ? 1e-7f * fabsf(pf[i]) + 1e-5f * sig
+                                                  : (retried ? 1e-4f : 1e-3f) * sig;
+                        const float hg = __shfl_sync(0xffffffffu, hs[i], 0);
+                        conv = conv && (fabsf(hg) <= tol);
+                    }
+                    if (conv) {
+                        if (precise) { state = IMFCS_STATE_CONVERGED; done = true; }
+                        else to_precise = true;
                     }
                 }
                 if (done || to_precise) break;
