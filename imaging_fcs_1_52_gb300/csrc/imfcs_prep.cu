@@ -497,18 +497,52 @@ __device__ __noinline__ float exp_normal32(const float *y, int n, float dts, flo
     return warp_sum(c2f);
 }
 
-// FP32 counterpart of exp_newton_step (phase 1).
+// solve_scaled_k for phase 1, its first subtractions spelled out (where the
+// compiler fuses a scaling product into them depends on the code around the
+// call): x = z sc, factors apart.
 template <int K>
-__device__ __forceinline__ bool exp_newton_step32(const float *A, const float *g, const float *p, unsigned &fix,
-                                                  float *h)
+__device__ __forceinline__ bool exp_solve(const float *A, const float *b, float lambda, unsigned fix, float (&z)[K],
+                                          float (&sc)[K])
 {
-    constexpr int NC = (K - 1) / 2;
-    fix = 0;
-    bool ok = solve_scaled_k<K>(A, g, 0.f, 0u, h);
-    for (int c = 0; c < NC; c++)
-        if (p[2 + 2 * c] <= 0.f && (!ok || h[2 + 2 * c] < 0.f)) fix |= 1u << (2 + 2 * c);
-    if (fix) ok = solve_scaled_k<K>(A, g, 0.f, fix, h);
-    return ok;
+    float L[K * K];
+#pragma unroll
+    for (int i = 0; i < K; i++) sc[i] = ((fix >> i) & 1) ? 0.f : rsqrtf(fmaxf(A[i * K + i], 1e-30f));
+#pragma unroll
+    for (int c = 0; c < K; c++) {
+        float d = ((fix >> c) & 1) ? 1.f : 1.f + lambda + 1e-6f;
+#pragma unroll
+        for (int m = 0; m < c; m++) d = fmaf(-L[c * K + m], L[c * K + m], d);
+        if (!(d > 0.f) || !isfinite(d)) return false;
+        d = sqrtf(d);
+        L[c * K + c] = d;
+#pragma unroll
+        for (int r = c + 1; r < K; r++) {
+            const float t = __fmul_rn(A[r * K + c], sc[r]);
+            float sum = __fmul_rn(t, sc[c]);
+            if (c > 0)
+                sum = fmaf(t, sc[c], -__fmul_rn(L[r * K], L[c * K]));
+#pragma unroll
+            for (int m = 1; m < c; m++) sum = fmaf(-L[r * K + m], L[c * K + m], sum);
+            L[r * K + c] = sum / d;
+        }
+    }
+    float yv[K];
+#pragma unroll
+    for (int r = 0; r < K; r++) {
+        float sum = __fmul_rn(b[r], sc[r]);
+        if (r > 0) sum = fmaf(b[r], sc[r], -__fmul_rn(L[r * K], yv[0]));
+#pragma unroll
+        for (int m = 1; m < r; m++) sum = fmaf(-L[r * K + m], yv[m], sum);
+        yv[r] = sum / L[r * K + r];
+    }
+#pragma unroll
+    for (int r = K - 1; r >= 0; r--) {
+        float sum = yv[r];
+#pragma unroll
+        for (int m = r + 1; m < K; m++) sum = fmaf(-L[m * K + r], z[m], sum);
+        z[r] = sum / L[r * K + r];
+    }
+    return true;
 }
 
 // The undamped (Gauss-)Newton step on A h = g, with a rate at its bound
@@ -733,27 +767,49 @@ __global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *
     const bool ok = isfinite(chi2f);
     int evals = 1, rejected = 0;
     for (int it_n = 0; ok && it_n < 100; it_n++) {
-        float h[K];
-        unsigned fix;
+        // the undamped step of the stopping test in the warp's lower half and
+        // the damped one in the upper: a solve is one long chain (2,304
+        // double-exponential traces 1.73 -> 1.53 ms, 16,384 single 0.95 ->
+        // 0.89).  A rate at its bound whose undamped step points below it is
+        // held (second pass).
+        float hz[K], sc[K];
+        unsigned fix = 0, votes;
+#pragma unroll 1
+        for (;;) {
+            votes = __ballot_sync(0xffffffffu, exp_solve<K>(A, gf, lane < 16 ? 0.f : lambda, fix, hz, sc));
+            if (fix) break;
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const float hk = __shfl_sync(0xffffffffu, __fmul_rn(hz[2 + 2 * c], sc[2 + 2 * c]), 0);
+                if (pf[2 + 2 * c] <= 0.f && (!(votes & 1) || hk < 0.f)) fix |= 1u << (2 + 2 * c);
+            }
+            if (!fix) break;
+        }
         bool gn_near = false;      // Gauss-Newton step within 0.05 sigma
-        if (exp_newton_step32<K>(A, gf, pf, fix, h)) {
+        if (votes & 1) {
             bool conv = true;
             gn_near = true;
+#pragma unroll
             for (int a = 0; a < K; a++) {
+                const float ha = __shfl_sync(0xffffffffu, __fmul_rn(hz[a], sc[a]), 0);
                 if ((fix >> a) & 1) continue;
                 const float sig = rsqrtf(fmaxf(A[a * K + a], 1e-30f));
-                conv = conv && fabsf(h[a]) <= 1e-6f * fabsf(pf[a]) + 1e-3f * sig;
-                gn_near = gn_near && fabsf(h[a]) <= 0.05f * sig;
+                conv = conv && fabsf(ha) <= 1e-6f * fabsf(pf[a]) + 1e-3f * sig;
+                gn_near = gn_near && fabsf(ha) <= 0.05f * sig;
             }
             if (conv) break;
         }
-        if (!solve_scaled_k<K>(A, gf, lambda, fix, h)) {
+        if (!(votes >> 16 & 1)) {
             lambda *= 10.f;
             if (lambda > 1e10f) break;
             continue;
         }
         float pn[K];
-        for (int a = 0; a < K; a++) pn[a] = pf[a] + h[a];
+#pragma unroll
+        for (int a = 0; a < K; a++) {
+            const float z = __shfl_sync(0xffffffffu, hz[a], 16);
+            pn[a] = __fadd_rn(pf[a], __fmul_rn(z, sc[a]));
+        }
         for (int c = 0; c < NC; c++) pn[2 + 2 * c] = fmaxf(pn[2 + 2 * c], 0.f);
         float An[K * K], gn[K];
         const float c2n = exp_normal32<K>(y, n, dts, iy, pn, An, gn, lane);
