@@ -260,6 +260,9 @@ __global__ void __launch_bounds__(kGlsThreads, 4) gls_kernel(GlsArgs g)
         cdiag[tid] = c;
         isd[tid] = 1.0 / sqrt(c);
     }
+    // where more than half of the variances are NaN no lag has the median's
+    // rank: not what the CTA before left here
+    if (tid == 0) s_med[0] = s_med[1] = 0.0;
     __syncthreads();
     // median of the chanum diagonal entries incl. the zero-lag slot that
     // stays 0 (java:9563-9573): rank selection, ties ordered by index

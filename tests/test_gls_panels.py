@@ -4,7 +4,7 @@ the FP64 oracle; tolerances of the GLS parity tests."""
 import numpy as np
 import pytest
 
-from imaging_fcs_1_52_gb300 import engine
+from imaging_fcs_1_52_gb300 import _lib, engine
 from tests.helpers import FIT_TOL, run_both
 from tests.synth import brownian_stack
 
@@ -30,3 +30,20 @@ def test_matrix_sizes_match_oracle(q):
     for i in (0, 1):
         err = np.abs(gpu["fitres"][both, i] / ref["fitres"][both, i] - 1)
         assert both.sum() == 0 or err.max() <= FIT_TOL, (i, err.max())
+
+
+def test_covariances_with_non_finite_lags_repeat():
+    """Pixels most of whose lags are not finite (a polynomial bleach curve
+    through zero) get the same covariance entries whatever ran before them."""
+    w = h = 40
+    st = brownian_stack(w, h, 6000, seed=5, density=3.0, cps=1e5)
+    t = np.arange(6000)[:, None, None] / 6000.0
+    st = (100 + (st - 100.0) * np.maximum(0.0, 1.0 - 1.1 * t)).astype(np.uint16)
+    cfg = engine.FCSConfig(width=w, height=h, frames=6000, background=100, gls=True, bleach=_lib.BLEACH_POLYNOMIAL,
+                           poly_order=5)
+    bright = engine.FCSConfig(width=w, height=h, frames=6000, background=100, gls=True)
+    first = engine.run_host(st, cfg)["covmats"]
+    assert not np.isfinite(first).all()
+    for _ in range(3):
+        engine.run_host(st, bright)
+        np.testing.assert_array_equal(engine.run_host(st, cfg)["covmats"], first)
