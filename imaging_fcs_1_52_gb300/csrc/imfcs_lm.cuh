@@ -256,7 +256,7 @@ __device__ __forceinline__ int lm_next_fit(const FitArgs &a, int fit, int nw, in
 template <int KM, bool BIG>
 __global__ void __launch_bounds__(128) lm_kernel(FitArgs a)
 {
-    extern __shared__ float fsh[];
+    extern __shared__ __align__(16) float fsh[];   // holds FP64 arrays too
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
     const int n = a.npts;

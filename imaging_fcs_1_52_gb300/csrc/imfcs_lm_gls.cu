@@ -90,7 +90,7 @@ __device__ __forceinline__ float gls_sig(const float *s, int i)
 template <bool OFF>
 __global__ void __launch_bounds__(32, 16) lm_gls_kernel(FitArgs a)
 {
-    extern __shared__ float tsh[];
+    extern __shared__ __align__(16) float tsh[];   // holds FP64 arrays too
     __shared__ GlsFitSh sh;
     const int lane = threadIdx.x;
     const int n = a.npts;
