@@ -369,11 +369,13 @@ __global__ void __launch_bounds__(kGlsThreads, 4) gls_kernel(GlsArgs g)
         lp[i] = (x == y) ? rdiag[x] : (1.0 - lc) * lp[i] * sq[x] * sq[y] * inv_pnum;
     }
     __syncthreads();
-    if (g.covmats_out)
+    if (g.covmats_out) {
         for (int i = tid; i < n1 * n1; i += kGlsThreads) {
             const int x = i / n1, y = i - x * n1;
             g.covmats_out[(size_t)pix * n1 * n1 + i] = x >= y ? lp[tri(x, y)] : lp[tri(y, x)];
         }
+        __syncthreads();              // every warp has copied its share before warp 0 factors lp in place
+    }
     // Cholesky in panels of kPanel columns: warp 0 factors a panel in
     // registers, then all warps subtract its columns' products from the rest
     // (18 barriers instead of 216; a panel ahead, with the other warps at the

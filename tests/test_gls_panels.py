@@ -47,3 +47,22 @@ def test_covariances_with_non_finite_lags_repeat():
     for _ in range(3):
         engine.run_host(st, bright)
         np.testing.assert_array_equal(engine.run_host(st, cfg)["covmats"], first)
+
+
+def test_exported_covariances_are_copied_whole():
+    """The covariance leaves before the factorisation overwrites it in place,
+    whatever order a block's warps run in: with the GPU full every matrix is
+    symmetric bit for bit (the two copies of an entry are read by different
+    threads) and equals the one of a small grid over the same pixels."""
+    w, h, rows = 64, 48, 2
+    st = engine.simulate(w, h, 5000, steps_per_frame=1, density=4.0, seed=7)
+    outs = []
+    for kw in ({}, {"map_y0": 20, "out_h": rows}):
+        plan = engine.Plan(engine.FCSConfig(width=w, height=h, frames=5000, background=100, gls=True, do_fit=False, **kw))
+        o = plan.alloc_device_outputs()
+        plan.execute(st, o)
+        outs.append(o["covmats"].cpu().numpy())
+    full, part = outs
+    assert np.isfinite(full).all(axis=(1, 2)).sum() >= 0.9 * w * h
+    np.testing.assert_array_equal(full, full.transpose(0, 2, 1))
+    np.testing.assert_array_equal(full.reshape(h, w, *full.shape[1:])[20:20 + rows].reshape(part.shape), part)
