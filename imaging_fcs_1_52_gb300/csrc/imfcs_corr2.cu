@@ -830,6 +830,9 @@ __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
     const int pnum = a.li->pnum_by_ind[ind];
     const float *pz = a.pz + (size_t)lag * a.pnum_max * a.cs + pc;
     const float r = pnum > 0 ? pz[0] : 0.f;
+    // GLS takes the products themselves (lags 1 and up, [pixel][lag][block])
+    float *bprod = a.o.gls && lag > 0
+                       ? a.o.bprod + ((size_t)pix * (a.chanum - 1) + (lag - 1)) * a.o.pnum_stride : nullptr;
     float S1 = 0.f, S2 = 0.f;
     for (int z = 0; z < pnum; z += 8) {
         float v[8];
@@ -841,6 +844,7 @@ __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
                 const float dv = v[u] - r;
                 S1 += dv;
                 S2 = fmaf(dv, dv, S2);
+                if (bprod) bprod[z + u] = v[u];
             }
     }
     const int sl = a.seg_log[lag <= a.p ? 0 : 1 + (lag - (a.p + 1)) / (a.p / 2)];

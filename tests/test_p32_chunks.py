@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from imaging_fcs_1_52_gb300 import engine
-from tests.helpers import run_both
+from tests.helpers import ACF_TOL, acf_deviation, run_both
 from tests.synth import brownian_stack
 from tests.test_gpu_correlator import check_acf
 
@@ -34,3 +34,20 @@ def test_segment_edges_match_oracle(frames, q, kw):
     cfg = engine.FCSConfig(width=6, height=5, frames=frames, background=100, p=32, q=q, do_fit=False, **kw)
     gpu, ref = run_both(st, cfg)
     check_acf(gpu, ref)
+
+
+@pytest.mark.parametrize("q,kw", [(2, {}), (4, {"cfx": 1}), (5, {})], ids=["q2", "q4-ccf", "q5"])
+def test_gls_products_match_oracle(q, kw):
+    """GLS takes up to 96 fit lags, P = 32 with Q <= 5 among them: the
+    covariance comes from the products the P = 32 kernels hand over."""
+    st = brownian_stack(6, 5, 9000, seed=61, density=3.0, cps=1e5)
+    cfg = engine.FCSConfig(width=6, height=5, frames=9000, background=100, p=32, q=q, gls=True, **kw)
+    gpu, ref = run_both(st, cfg)
+    np.testing.assert_array_equal(gpu["blocked_ind"], ref["blocked_ind"])
+    assert acf_deviation(gpu, ref) <= ACF_TOL
+    n1 = cfg.chanum - 1
+    g, r = gpu["covmats"].reshape(-1, n1, n1), ref["covmats"].reshape(-1, n1, n1)
+    fin = np.isfinite(r).all(axis=(1, 2))
+    assert fin.sum() >= 15
+    scale = np.abs(r[fin]).max(axis=(1, 2), keepdims=True)
+    assert np.max(np.abs(g[fin] - r[fin]) / scale) <= 1e-4
