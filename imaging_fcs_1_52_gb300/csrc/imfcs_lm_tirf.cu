@@ -56,7 +56,7 @@ __device__ __forceinline__ void tirf_accumulate(float (&acc)[9], const float (&g
 template <bool OFF, bool SIDE>
 __device__ __noinline__ void tirf_eval32(const TirfC &c, float N, float D, float G, const float *yl,
                                          const float *wl, const float *xl, int n, int lane, Tirf3 &s,
-                                         float bound)
+                                         float bound)       // a trial step's: chi^2 to be lowered (else NaN)
 {
     float acc[9];
 #pragma unroll
@@ -90,7 +90,9 @@ __device__ __noinline__ void tirf_eval32(const TirfC &c, float N, float D, float
     }
     s.chi2 = warp_sum(c2f);
     s.chi2d = 0.0;
-    if (!(s.chi2 < bound)) return;      // a rejected step: nobody reads the sums
+    // a rejected trial step: nobody reads the sums (those of every other
+    // evaluation are read, whatever chi^2 is)
+    if (!isnan(bound) && !(s.chi2 < bound)) return;
     tirf_reduce(acc, s);
     s.fmag = warp_sum(fm);
 }
@@ -140,7 +142,7 @@ __device__ __noinline__ void tirf_eval64(const TirfC &c, double Nd, double Dd, d
 template <bool OFF, bool SIDE>
 __device__ __forceinline__ void tirf_eval(const TirfC &c, float N, float D, float G, double Nd, double Dd, double Gd,
                                           const float *yl, const float *wl, const float *xl, int n, int lane,
-                                          bool precise, Tirf3 &s, float bound = INFINITY)
+                                          bool precise, Tirf3 &s, float bound = NAN)
 {
     if (precise) tirf_eval64<OFF, SIDE>(c, Nd, Dd, Gd, yl, wl, xl, n, lane, s);
     else tirf_eval32<OFF, SIDE>(c, N, D, G, yl, wl, xl, n, lane, s, bound);
