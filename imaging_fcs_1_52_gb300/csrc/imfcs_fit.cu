@@ -193,7 +193,7 @@ __device__ __forceinline__ bool qr_inverse_d(const double *ain, int k_, double t
     return true;
 }
 
-// Bayes: log-residual term of every fitted pixel (left in logp), a warp per
+// Bayes: log-residual term of every converged pixel (left in logp), a warp per
 // pixel; the sums in the order of one thread.
 constexpr int kResWarps = 4;
 __global__ void __launch_bounds__(32 * kResWarps) bayes_residual_kernel(EpilogueArgs e)
@@ -202,6 +202,8 @@ __global__ void __launch_bounds__(32 * kResWarps) bayes_residual_kernel(Epilogue
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int pix = blockIdx.x * kResWarps + wid;
     if (pix >= e.npix) return;
+    // a failed fit has no residuals, a failed factorisation no L^-1
+    if (e.state[pix] != IMFCS_STATE_CONVERGED || (e.pre_ok && !e.pre_ok[pix])) return;
     double *tres = tres_sh[wid], *z = z_sh[wid];
     float par[IMFCS_NPARAM];
 #pragma unroll

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from imaging_fcs_1_52_gb300 import engine
+from tests.synth import brownian_stack
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +40,20 @@ def test_results_do_not_depend_on_other_fits(init):
     assert np.isfinite(full["fitres"][full["fitted"] == 1]).all()
     for k in ("fitted", "iterations", "fitres", "chi2"):
         np.testing.assert_array_equal(full[k][30 * w:32 * w], part[k], err_msg=k)
+
+
+@pytest.mark.parametrize("gls", [False, True])
+def test_bayes_terms_beside_failed_fits(gls):
+    """Pixels without a fit (dead: no factorisation either) get the failed
+    fits' probabilities, 0 / 0 as the oracle's, and leave their neighbours'
+    as they are."""
+    st = brownian_stack(8, 6, 6000, seed=21, density=2.0, cps=3e4)
+    st[:, 2:4, ::2] = 300
+    dead = np.zeros((6, 8), bool)
+    dead[2:4, ::2] = True
+    outs = [engine.run_host(st, engine.FCSConfig(width=8, height=6, frames=6000, background=100, gls=gls, bayes=True,
+                                                 **kw)) for kw in ({}, {"map_y0": 2, "out_h": 2})]
+    full, part = (o["bayes_prob"] for o in outs)
+    assert np.isnan(full[dead.ravel()]).all()
+    assert np.isfinite(full[~dead.ravel()]).all(axis=1).sum() >= 30
+    np.testing.assert_array_equal(full[2 * 8:4 * 8], part)
