@@ -1463,10 +1463,18 @@ cudaError_t launch_monitor_finalize(const Job &j, const LagInfo *li_dev, const f
                                     const float2 *segtot, const float2 *snap_part, const int *segbad,
                                     const int *snap_bad, float4 *mon, float4 *blkmon, cudaStream_t s)
 {
-    const int wpb = 4;
-    size_t smem = (size_t)wpb * (nseg + 1 + 2 * j.nsnap) * (sizeof(double) + sizeof(int));
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(monitor_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // four pixels a block; fewer where a recording's segments leave no room for
+    // their scans (from 1.1 million frames on, to 4.9 million with one)
+    constexpr size_t kMaxSmem = 227 * 1024;
+    const size_t one = (size_t)(nseg + 1 + 2 * j.nsnap) * (sizeof(double) + sizeof(int));
+    int wpb = 4;
+    while (wpb > 1 && wpb * one > kMaxSmem) wpb /= 2;
+    const size_t smem = wpb * one;
+    if (smem > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(monitor_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     monitor_finalize_kernel<<<(j.npix + wpb - 1) / wpb, wpb * 32, smem, s>>>(j, li_dev, bparams, nseg, segtot,
                                                                            snap_part, segbad, snap_bad, mon,
                                                                            blkmon);
