@@ -524,45 +524,46 @@ struct CgArgs {
 };
 
 // Level-k samples (k = 1..3 pairwise, java:9467-9476; above, the level-3
-// samples of a sample added in order) of 2^(Q-1) frames per thread.
+// samples of a sample added in order), 2^(Q-1) frames at a time per thread;
+// the blocks of grid.y stride over a long recording's spans.
 template <bool CCF>
 __global__ void __launch_bounds__(128) cg_levels_kernel(CgArgs a)
 {
     const int pc = blockIdx.x * 128 + threadIdx.x;
     if (pc >= a.np) return;
     const int span = 1 << max(a.q - 1, 3);
-    const int f0 = blockIdx.y * span;
-    for (int tr = 0; tr < (CCF ? 2 : 1); tr++) {
-        const float *in = (tr ? a.s0b : a.s0a) + a.p0 + pc;
-        float *lv = (tr ? a.lvb : a.lva) + pc;
-        float up[kMaxLevels];                 // running sums of levels 4..Q-1
+    for (int f0 = blockIdx.y * span; f0 < a.num; f0 += gridDim.y * span)
+        for (int tr = 0; tr < (CCF ? 2 : 1); tr++) {
+            const float *in = (tr ? a.s0b : a.s0a) + a.p0 + pc;
+            float *lv = (tr ? a.lvb : a.lva) + pc;
+            float up[kMaxLevels];             // running sums of levels 4..Q-1
 #pragma unroll
-        for (int k = 4; k < 8; k++) up[k] = 0.f;
-        for (int f = f0; f < f0 + span && f < a.num; f += 8) {
-            float v[8];
+            for (int k = 4; k < 8; k++) up[k] = 0.f;
+            for (int f = f0; f < f0 + span && f < a.num; f += 8) {
+                float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = f + i < a.num ? __ldg(&in[(size_t)(f + i) * a.npix]) : 0.f;
+                for (int i = 0; i < 8; i++) v[i] = f + i < a.num ? __ldg(&in[(size_t)(f + i) * a.npix]) : 0.f;
 #pragma unroll
-            for (int k = 1; k <= 3; k++) {
+                for (int k = 1; k <= 3; k++) {
 #pragma unroll
-                for (int i = 0; i < (8 >> k); i++) {
-                    v[i] = v[2 * i] + v[2 * i + 1];
-                    const int n = (f >> k) + i;
-                    if (k < a.q && n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = v[i];
+                    for (int i = 0; i < (8 >> k); i++) {
+                        v[i] = v[2 * i] + v[2 * i + 1];
+                        const int n = (f >> k) + i;
+                        if (k < a.q && n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = v[i];
+                    }
                 }
-            }
 #pragma unroll
-            for (int k = 4; k < 8; k++) {
-                if (k >= a.q) break;
-                up[k] += v[0];
-                if (((f + 8) & ((1 << k) - 1)) == 0) {
-                    const int n = f >> k;
-                    if (n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = up[k];
-                    up[k] = 0.f;
+                for (int k = 4; k < 8; k++) {
+                    if (k >= a.q) break;
+                    up[k] += v[0];
+                    if (((f + 8) & ((1 << k) - 1)) == 0) {
+                        const int n = f >> k;
+                        if (n < a.numbin[k]) lv[a.lv_off[k] + (size_t)n * a.cs] = up[k];
+                        up[k] = 0.f;
+                    }
                 }
             }
         }
-    }
 }
 
 // One level's samples of one pixel.
@@ -1039,7 +1040,7 @@ cudaError_t launch_corrg(const Job &j, const LagInfo *li, const float *s0, const
     const int span = 1 << max(j.q - 1, 3);
     for (a.p0 = 0; a.p0 < j.npix; a.p0 += p.chunk) {
         a.np = min(p.chunk, j.npix - a.p0);
-        const dim3 gl((a.np + 127) / 128, (j.num + span - 1) / span);
+        const dim3 gl((a.np + 127) / 128, min((j.num + span - 1) / span, 65535));
         const dim3 gb((a.np + kCgThreads - 1) / kCgThreads, j.q + 1, p.nseg);
         if (j.is_ccf) {
             cg_levels_kernel<true><<<gl, 128, 0, stream>>>(a);
