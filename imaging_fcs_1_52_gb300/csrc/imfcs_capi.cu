@@ -244,7 +244,6 @@ struct imfcs_plan {
     size_t bytes = 0;
     // scratch
     float *trace = nullptr, *bparams = nullptr, *basis = nullptr, *grid = nullptr;
-    unsigned *trace_sums = nullptr;   // only where s0 is too small to hold the trace's raw sums
     double *proj = nullptr;
     int *snap_pos = nullptr;
     float2 *segtot = nullptr, *snap_part = nullptr;
@@ -492,7 +491,6 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     AS(pl->stats, corr_stats_floats(j));
     AS(pl->streams, corr_stream_floats(j));
     AS(pl->s0, level0_stream_floats(j));
-    if (trace_sums_elems(j) > level0_stream_floats(j)) AS(pl->trace_sums, trace_sums_elems(j));
     AS(pl->acf_int, np * chanum);
     AS(pl->var_int, np * chanum);
     AL(pl->lagtime, chanum);
@@ -741,13 +739,13 @@ int plan_execute_any(imfcs_plan *pl, const void *dev_stack, const imfcs_outputs 
     for (int i = 0; i <= imfcs_plan::kStages; i++) pl->ev_used[i] = false;
     pl->launches = 0;
     pl->mark(0, s);
-    // the trace's raw sums are read before the streaming pass writes s0
-    CK(launch_trace(j, dev_stack, pl->trace_sums ? pl->trace_sums : (unsigned *)pl->s0, pl->trace, s));
-    if (trace_sums_elems(j)) pl->launches += 1;
+    // the trace's raw sums take s0's place: they are read before the streaming
+    // pass writes it
+    CK(launch_trace(j, dev_stack, pl->s0, pl->trace, s));
     if (pl->given_bleach) CK(launch_center_given(j, pl->trace, pl->bparams, s));
     else CK(launch_bleach(j, pl->trace, pl->proj, (float)pl->uscale, (float)pl->uoff, pl->grid, pl->bparams, s));
     if (!pl->given_bleach && j.bleach == IMFCS_BLEACH_SINGLE_EXP) pl->launches += 1;
-    pl->launches += 2;
+    pl->launches += trace_kernel_count(j) + 1;
     pl->mark(1, s);
     // one streaming pass over the raw stack: the corrected, centred level-0
     // stream and the monitor partial sums

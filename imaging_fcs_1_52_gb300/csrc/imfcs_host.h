@@ -37,9 +37,9 @@ struct GlsArgs;
 cudaError_t launch_gls(const GlsArgs &g, cudaStream_t stream);
 
 // prep launchers (imfcs_prep_launch.cu)
-// sums: trace_sums_elems scratch values (0 of them: the one-pass kernel runs)
-cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float *trace, cudaStream_t s);
-size_t trace_sums_elems(const Job &j);
+// scratch: level0_stream_floats floats (free until the streaming pass writes them)
+cudaError_t launch_trace(const Job &j, const void *stack, float *scratch, float *trace, cudaStream_t s);
+int trace_kernel_count(const Job &j);
 // grid: launch_bleach_grid_table's table (single exponential), else unused
 cudaError_t launch_bleach(const Job &j, const float *trace, const double *proj, float uscale,
                           float uoff, const float *grid, float *bparams, cudaStream_t s);

@@ -54,19 +54,25 @@ __global__ void __launch_bounds__(256) trace_kernel(Job j, const void *stack, fl
 }
 
 // The same in two passes where the traces read most of the frames' columns:
-// the sums of `ave` frames of every raw pixel of the rows read, once and with
-// wide loads (sums[x][pixel], bound by HBM), then the windows of the sums.
-// VEC raw pixels per thread: 8 (16-byte loads), 2 or 1 by the frames' length
-// and alignment.  One pass with a guarded 2-byte load per raw value was bound
-// by issue: 0.67 -> 0.28 ms at 128x128x50,000 (read once at 6.8 TB/s: 0.24),
-// 0.73 -> 0.09 for overlapping 5 x 5 windows at 101x67x12,345.
-template <int VEC>
-__global__ void __launch_bounds__(128) trace_sums_kernel(const uint16_t *base, size_t fsz, int nelem, int ave,
+// the sums of `ave` frames (and, where the windows' rows do not overlap, of a
+// window's rows: ROWS) of every raw pixel of the rows read, once and with wide
+// loads, bound by HBM, then the windows of the sums.
+struct TraceSums {
+    int lines, len, lstride;      // lines of sums (ROWS: one per output row), their length, raw elements between them
+    int rows, in_w;               // raw rows added up
+};
+// sums[x][line][i], VEC raw pixels per thread: 8 (16-byte loads), 2 or 1 by the
+// lines' length and alignment.  One pass with a guarded 2-byte load per raw value
+// was bound by issue: 0.67 -> 0.28 ms at 128x128x50,000 (read once at 6.8
+// TB/s: 0.24), 0.73 -> 0.09 for overlapping 5 x 5 windows at 101x67x12,345.
+template <int VEC, bool ROWS>
+__global__ void __launch_bounds__(128) trace_sums_kernel(const uint16_t *base, size_t fsz, TraceSums g, int ave,
                                                          unsigned *sums)
 {
-    const int i = (blockIdx.x * 128 + threadIdx.x) * VEC;
-    if (i >= nelem) return;
-    const uint16_t *p = base + (size_t)blockIdx.y * ave * fsz + i;
+    const int i = blockIdx.x * 128 + threadIdx.x, per = g.len / VEC;
+    if (i >= g.lines * per) return;
+    const int line = ROWS ? i / per : 0, x = (i - line * per) * VEC;
+    const uint16_t *p = base + (size_t)blockIdx.y * ave * fsz + (size_t)line * g.lstride + x;
     unsigned acc[VEC];
 #pragma unroll
     for (int e = 0; e < VEC; e++) acc[e] = 0;
@@ -74,13 +80,31 @@ __global__ void __launch_bounds__(128) trace_sums_kernel(const uint16_t *base, s
         a[0] = __dp2a_lo(w, 0x0001u, a[0]);
         a[1] = __dp2a_lo(w, 0x0100u, a[1]);
     };
+    // a window's rows, then the next frame
+    const int n = ROWS ? ave * g.rows : ave;
+    const size_t back = fsz - (size_t)(g.rows - 1) * g.in_w;
+    int row = 0;
+    auto next = [&] {
+        if (ROWS && ++row < g.rows) {
+            p += g.in_w;
+        } else {
+            p += ROWS ? back : fsz;
+            row = 0;
+        }
+    };
     constexpr int U = VEC == 8 ? 4 : 8;
-    int f = 0;
-    for (; f + U <= ave; f += U, p += (size_t)U * fsz) {
+    // U values (the last time: those left), all loads before their sums
+    auto batch = [&](int left) {
         if constexpr (VEC == 8) {
             uint4 v[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) v[u] = __ldcs((const uint4 *)(p + (size_t)u * fsz));
+            for (int u = 0; u < U; u++) {
+                v[u] = make_uint4(0, 0, 0, 0);
+                if (u < left) {
+                    v[u] = __ldcs((const uint4 *)p);
+                    next();
+                }
+            }
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 add2(v[u].x, acc);
@@ -91,29 +115,43 @@ __global__ void __launch_bounds__(128) trace_sums_kernel(const uint16_t *base, s
         } else if constexpr (VEC == 2) {
             unsigned v[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) v[u] = __ldcs((const unsigned *)(p + (size_t)u * fsz));
+            for (int u = 0; u < U; u++) {
+                v[u] = 0;
+                if (u < left) {
+                    v[u] = __ldcs((const unsigned *)p);
+                    next();
+                }
+            }
 #pragma unroll
             for (int u = 0; u < U; u++) add2(v[u], acc);
         } else {
             uint16_t v[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) v[u] = __ldcs(p + (size_t)u * fsz);
+            for (int u = 0; u < U; u++) {
+                v[u] = 0;
+                if (u < left) {
+                    v[u] = __ldcs(p);
+                    next();
+                }
+            }
 #pragma unroll
             for (int u = 0; u < U; u++) acc[0] += v[u];
         }
-    }
-    for (; f < ave; f++, p += fsz)
-#pragma unroll
-        for (int e = 0; e < VEC; e++) acc[e] += p[e];
-    unsigned *o = sums + (size_t)blockIdx.y * nelem + i;
+    };
+    int f = 0;
+    for (; f + U <= n; f += U) batch(U);
+    if (f < n) batch(n - f);
+    unsigned *o = sums + ((size_t)blockIdx.y * g.lines + line) * g.len + x;
 #pragma unroll
     for (int e = 0; e < VEC; e++) o[e] = acc[e];
 }
 
 // Block (32 traces) x (8 rows), 4 points per thread, transposed through a
-// shared tile like trace_kernel.  row0: the first raw row of the sums.
-__global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigned *sums, int row0, int nelem,
-                                                            float *trace_out)
+// shared tile like trace_kernel.  row0: the first raw row of the sums; they
+// are those of points p0 .. p0 + np - 1, nelem to a point.
+template <bool ROWS>
+__global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigned *sums, int row0, int nelem, int p0,
+                                                            int np, float *trace_out)
 {
     __shared__ float tile[32][33];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -123,15 +161,15 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
         int x0, y0;
         trace_origin(j, trace, x0, y0);
         const int bg = trace_bg_avg(j, trace) * j.ave;
-        const unsigned *w = sums + (size_t)(y0 - row0) * j.in_w + x0;
+        const unsigned *w = sums + (size_t)(ROWS ? y0 / j.pixbiny - j.map_y0 : y0 - row0) * j.in_w + x0;
         int acc[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) acc[r] = 0;
-        for (int k = 0; k < j.biny; k++)
+        for (int k = 0; k < (ROWS ? 1 : j.biny); k++)
             for (int i = 0; i < j.binx; i++)
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
-                    const int x = min(xbase + ty * 4 + r, j.nopit - 1);
+                    const int x = min(xbase + ty * 4 + r, np - 1);
                     acc[r] += (int)__ldg(&w[(size_t)x * nelem + k * j.in_w + i]);
                 }
 #pragma unroll
@@ -140,7 +178,7 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
     __syncthreads();
     for (int r = 0; r < 4; r++) {
         const int tl = ty * 4 + r, tr = blockIdx.x * 32 + tl, x = xbase + tx;
-        if (tr < j.ntrace && x < j.nopit) trace_out[(size_t)tr * j.nopit + x] = tile[tl][tx];
+        if (tr < j.ntrace && x < np) trace_out[(size_t)tr * j.nopit + p0 + x] = tile[tl][tx];
     }
 }
 
@@ -1371,46 +1409,90 @@ template __global__ void bleach_exp_kernel<5>(Job, const float *, float *);
 
 namespace imfcs {
 
-// Raw rows the traces read: the first one, and the elements per frame of
-// trace_sums_kernel's output (0: the one-pass kernel).  A region narrower
-// than half the frame would have the two-pass form read columns nobody wants.
-static void trace_rows(const Job &j, int &row0, size_t &nelem)
+// How the averaged trace is taken: the raw rows read, from row0 on, the lines
+// of sums, and the points whose sums s0 holds at a time (0: the one-pass
+// kernel, which needs no scratch).  Times of the stage in us, one pass / two:
+//   regions narrower than half the frame, or using a third of its values or
+//     less (every second pixel of every second row at 128x128x20,000: 99 /
+//     132, the left half of the frame at 12,345: 130 / 107): one pass;
+//   single pixels: two (64x64x1,999 46 / 38, 128x128x10,000 241 / 130,
+//     256x256x4,500 576 / 391), but in parts 79 / 89 (half the frame, 1,500);
+//   windows: two from two frames a point on (128x128, 3 x 3: 36 / 52 at one
+//     frame, 54 / 50 at two, 89 / 50 at four; 512x512, 5 x 5: 189 / 237, 316 /
+//     294, 573 / 417), from three on where s0 holds less than a third of the sums
+//     (128x128, 16 x 16: 128 / 153 at two, 236 / 131 at four); those that use
+//     a value twice or more always (101x67, overlapping 5 x 5: 95 / 87 at one
+//     frame, 738 / 105 at twelve).
+struct TracePlan {
+    TraceSums g;
+    int row0, points;
+    bool rows;
+};
+static TracePlan trace_plan(const Job &j)
 {
-    row0 = j.map_y0 * j.pixbiny + (j.cfy < 0 ? j.cfy : 0);
+    TracePlan p;
+    p.row0 = j.map_y0 * j.pixbiny + (j.cfy < 0 ? j.cfy : 0);
     const int row1 = (j.map_y0 + j.out_h - 1) * j.pixbiny + j.biny + (j.cfy > 0 ? j.cfy : 0);
     const int cols = (j.out_w - 1) * j.pixbinx + j.binx + (j.cfx < 0 ? -j.cfx : j.cfx);
-    nelem = j.input_float || 2 * cols < j.in_w ? 0 : (size_t)(row1 - row0) * j.in_w;
-    if (nelem > (1u << 30)) nelem = 0;
+    const size_t raw = (size_t)(row1 - p.row0) * j.in_w;
+    p.points = 0;
+    if (j.input_float || 2 * cols < j.in_w || raw > (1u << 30)) return p;
+    p.rows = j.biny > 1 && j.pixbiny >= j.biny && !j.cfy;
+    p.g.lines = p.rows ? j.out_h : 1;
+    p.g.len = p.rows ? j.in_w : (int)raw;
+    p.g.lstride = j.pixbiny * j.in_w;
+    p.g.rows = p.rows ? j.biny : 1;
+    p.g.in_w = j.in_w;
+    const size_t area = (size_t)j.binx * j.biny, values = (size_t)j.ntrace * area;
+    if (3 * values <= raw) return p;
+    const size_t points = level0_stream_floats(j) / ((size_t)p.g.lines * p.g.len), all = j.nopit;
+    if (area == 1 ? points < all
+                  : values < 2 * raw && (j.ave < 2 || (j.ave < 3 && 3 * points < all)))
+        return p;
+    p.points = points < (size_t)j.nopit ? (int)points : j.nopit;
+    return p;
 }
 
-size_t trace_sums_elems(const Job &j)
+int trace_kernel_count(const Job &j)
 {
-    int row0;
-    size_t nelem;
-    trace_rows(j, row0, nelem);
-    return nelem * j.nopit;
+    const TracePlan p = trace_plan(j);
+    return p.points ? 2 * ((j.nopit + p.points - 1) / p.points) : 1;
 }
 
-cudaError_t launch_trace(const Job &j, const void *stack, unsigned *sums, float *trace, cudaStream_t s)
+cudaError_t launch_trace(const Job &j, const void *stack, float *scratch, float *trace, cudaStream_t s)
 {
-    dim3 grid((j.ntrace + 31) / 32, (j.nopit + 31) / 32), block(32, 8);
-    int row0;
-    size_t nelem;
-    trace_rows(j, row0, nelem);
-    if (nelem) {
-        const size_t fsz = (size_t)j.in_w * j.in_h;
-        const uint16_t *base = (const uint16_t *)stack + (size_t)j.first * fsz + (size_t)row0 * j.in_w;
-        const int n = (int)nelem;
-        auto grid1 = [&](int vec) { return dim3((n / vec + 127) / 128, j.nopit); };
-        if ((uintptr_t)base % 16 == 0 && fsz % 8 == 0 && n % 8 == 0)
-            trace_sums_kernel<8><<<grid1(8), 128, 0, s>>>(base, fsz, n, j.ave, sums);
-        else if ((uintptr_t)base % 4 == 0 && fsz % 2 == 0 && n % 2 == 0)
-            trace_sums_kernel<2><<<grid1(2), 128, 0, s>>>(base, fsz, n, j.ave, sums);
-        else trace_sums_kernel<1><<<grid1(1), 128, 0, s>>>(base, fsz, n, j.ave, sums);
-        trace_windows_kernel<<<grid, block, 0, s>>>(j, sums, row0, n, trace);
+    const dim3 block(32, 8);
+    const unsigned gx = (j.ntrace + 31) / 32;
+    const TracePlan p = trace_plan(j);
+    if (!p.points) {
+        trace_kernel<<<dim3(gx, (j.nopit + 31) / 32), block, 0, s>>>(j, stack, trace);
         return cudaGetLastError();
     }
-    trace_kernel<<<grid, block, 0, s>>>(j, stack, trace);
+    unsigned *sums = (unsigned *)scratch;
+    const size_t fsz = (size_t)j.in_w * j.in_h;
+    const int n = p.g.lines * p.g.len;
+    for (int p0 = 0; p0 < j.nopit; p0 += p.points) {
+        const int np = p.points < j.nopit - p0 ? p.points : j.nopit - p0;
+        const uint16_t *base =
+            (const uint16_t *)stack + ((size_t)j.first + (size_t)p0 * j.ave) * fsz + (size_t)p.row0 * j.in_w;
+        // whole vectors of a line, aligned in every row (ROWS: of in_w elements) and frame
+        auto fits = [&](int vec) { return (uintptr_t)base % (2 * vec) == 0 && fsz % vec == 0 && p.g.len % vec == 0; };
+#define SUMS(vec, rows) \
+    trace_sums_kernel<vec, rows><<<dim3((n / vec + 127) / 128, np), 128, 0, s>>>(base, fsz, p.g, j.ave, sums)
+        if (p.rows) {
+            if (fits(8)) SUMS(8, true);
+            else if (fits(2)) SUMS(2, true);
+            else SUMS(1, true);
+        } else {
+            if (fits(8)) SUMS(8, false);
+            else if (fits(2)) SUMS(2, false);
+            else SUMS(1, false);
+        }
+#undef SUMS
+        const dim3 grid(gx, (np + 31) / 32);
+        if (p.rows) trace_windows_kernel<true><<<grid, block, 0, s>>>(j, sums, p.row0, n, p0, np, trace);
+        else trace_windows_kernel<false><<<grid, block, 0, s>>>(j, sums, p.row0, n, p0, np, trace);
+    }
     return cudaGetLastError();
 }
 
