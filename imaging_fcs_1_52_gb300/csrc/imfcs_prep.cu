@@ -160,9 +160,11 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
     if (trace < j.ntrace) {
         int x0, y0;
         trace_origin(j, trace, x0, y0);
-        const int bg = trace_bg_avg(j, trace) * j.ave;
+        // the raw sums may pass 2^31 (bright windows, many frames a point) where
+        // the sum above the background does not: modulo 2^32
+        const unsigned bg = (unsigned)trace_bg_avg(j, trace) * (unsigned)j.ave;
         const unsigned *w = sums + (size_t)(ROWS ? y0 / j.pixbiny - j.map_y0 : y0 - row0) * j.in_w + x0;
-        int acc[4];
+        unsigned acc[4];
 #pragma unroll
         for (int r = 0; r < 4; r++) acc[r] = 0;
         for (int k = 0; k < (ROWS ? 1 : j.biny); k++)
@@ -170,10 +172,10 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     const int x = min(xbase + ty * 4 + r, np - 1);
-                    acc[r] += (int)__ldg(&w[(size_t)x * nelem + k * j.in_w + i]);
+                    acc[r] += __ldg(&w[(size_t)x * nelem + k * j.in_w + i]);
                 }
 #pragma unroll
-        for (int r = 0; r < 4; r++) tile[tx][ty * 4 + r] = (float)((acc[r] - bg) / j.ave);
+        for (int r = 0; r < 4; r++) tile[tx][ty * 4 + r] = (float)((int)(acc[r] - bg) / j.ave);
     }
     __syncthreads();
     for (int r = 0; r < 4; r++) {

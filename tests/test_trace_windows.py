@@ -55,6 +55,17 @@ def test_centre_is_the_mean_of_the_trace(w, h, frames, kw):
     assert np.abs(got / ref - 1).max() <= 2.2e-6
 
 
+def test_bright_windows_above_a_high_background():
+    """The raw values of a point's frames add up to more than 2^31, those above
+    the background do not."""
+    rng = np.random.default_rng(82)
+    st = rng.integers(58900, 59200, (600_000, 8, 16), dtype=np.uint16)
+    cfg = engine.FCSConfig(width=16, height=8, frames=600_000, background=59000, binx=8, biny=8, do_fit=False)
+    plan = engine.Plan(cfg)
+    plan.execute_host(st)
+    assert np.abs(plan.bleach_params()[:, 12] / traces(st, cfg).mean(axis=1) - 1).max() <= 2.2e-6
+
+
 def test_scratch_follows_the_output_pixels():
     one = engine.Plan(engine.FCSConfig(width=16, height=16, frames=3000, do_fit=False))
     for b in (2, 16):
