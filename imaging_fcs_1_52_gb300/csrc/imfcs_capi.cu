@@ -113,7 +113,8 @@ bool build_lag_info(int p, int q, int num, LagInfo &li, int &chanum, int &blockn
         li.inv_pnum1[ind] = 1.0 / (li.pnum_by_ind[ind] - 1);
         const double n = ind < 31 ? (double)((num - 1) >> ind) : 0.0;
         li.blk_inv_n[ind] = 1.0 / n;
-        li.blk_err[ind] = 1.0 / sqrt(2.0 * (n - 1.0));
+        li.blk_root[ind] = sqrt(2.0 * (n - 1.0));
+        li.blk_inv_root[ind] = 1.0 / li.blk_root[ind];
     }
     return true;
 }

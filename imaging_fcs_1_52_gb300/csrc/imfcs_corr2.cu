@@ -738,16 +738,22 @@ __device__ __forceinline__ void write_lag(const CorrOut &o, const float4 *mon, c
                                           int lag, int ind, double A, double S1, double S2, double r)
 {
     const float4 m = mon[(size_t)pix * chanum + lag];
-    const double n = li->prodnum[lag], ip = li->inv_pnum[ind];
-    const double idm = newton_rcp(f2d(m.z) * f2d(m.w));
-    const double cov = fma(-(n * f2d(m.x)), f2d(m.y), A) * li->inv_prodnum[lag];    // mean of the centred products
-    const double mean = S1 * ip;
-    const double bv = fma(S2, ip, -mean * mean) * li->inv_pnum1[ind] * idm * idm;
-    double acf = cov * idm;
-    if (o.gls) acf = (lag == 0) ? 0.0 : (mean + r) * idm;   // mcov (java:9526-9531)
+    // a non-finite frame in the lag's windows: NaN, whatever the sums
+    double acf = __longlong_as_double(0x7ff8000000000000ll), bv = acf, cov = acf;
+    if (m.x == m.x && m.y == m.y) {
+        const double n = f2d((float)li->prodnum[lag]), pn = f2d((float)li->pnum_by_ind[ind]), ip = li->inv_pnum[ind];
+        const double dmDm = f2d(m.z) * f2d(m.w), idm = newton_rcp(dmDm);
+        const double sumprod = fma(-(n * f2d(m.x)), f2d(m.y), A), in = li->inv_prodnum[lag];   // centred products
+        const double mean = div_by(S1, pn, ip);
+        cov = div_by(sumprod, n, in);
+        bv = div_near(fma(-mean, mean, div_by(S2, pn, ip)), (pn - 1.0) * dmDm * dmDm, li->inv_pnum1[ind] * idm * idm);
+        if (o.gls) acf = div_near(fma(pn, r, S1), pn * dmDm, ip * idm);    // mcov (java:9526-9531)
+        else acf = div_near(sumprod, n * dmDm, in * idm);
+    }
+    if (o.gls && lag == 0) acf = 0.0;
     if (o.acf) o.acf[(size_t)pix * chanum + lag] = acf;
     if (o.var) o.var[(size_t)pix * chanum + lag] = bv;
-    if (o.sd) o.sd[(size_t)pix * chanum + lag] = newton_sqrt(bv);
+    if (o.sd) o.sd[(size_t)pix * chanum + lag] = bv == bv ? newton_sqrt(bv) : bv;
     if (lag == 1) {
         if (o.nb_mean) o.nb_mean[pix] = m.z;
         if (o.nb_cov) o.nb_cov[pix] = cov;
@@ -771,10 +777,10 @@ static __device__ __noinline__ void plain_segments(const float *st, size_t np, s
 }
 
 // Grid (pixel blocks, lags).  Bound by FP64 issue (1/64 of the FP32 rate):
-// plain sums of FP32 values run as compensated FP32 sums (their error, below
-// 1e-14, is FP64's own of a dozen terms), only the products with the segments'
-// shifts are FP64, conversions go to the integer pipe.  0.56 -> 0.19 ms at
-// 16,384 pixels x 50,000 frames.  Float-float for those products too was
+// plain sums of FP32 values run in three FP32 terms, no less precise than FP64,
+// the products with the segments' shifts are FP64, conversions go to the
+// integer pipe, quotients are corrected products with reciprocals.  0.56 -> 0.21
+// ms at 16,384 pixels x 50,000 frames.  Float-float for those products too was
 // no faster and moved results by 1e-13, enough to round some of the fits' FP32
 // data and weights the other way.
 __global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
@@ -789,7 +795,7 @@ __global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
     const float *st = &stat_ref(a.o.stats, a.npix, lag, 0, pix);
     const size_t np = a.npix;
     const double r0 = f2d(__ldg(&st[4 * np]));      // segment 0 always has a counted block
-    ff A = {0.f, 0.f}, s1 = {0.f, 0.f}, s2 = {0.f, 0.f};
+    ff3 A = {0.f, 0.f, 0.f}, s1 = A, s2 = A;
     double S1 = 0.0, S2 = 0.0;
     const float4 m = a.mon[(size_t)pix * a.chanum + lag];
     const bool bad = m.x != m.x || m.y != m.y;      // a non-finite frame in the lag's windows: NaN, whatever the sums
@@ -797,23 +803,23 @@ __global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
     for (int sg = 0; sg < nseg && !bad; sg++, st += a.stat_stride) {
         const float hi = __ldg(&st[0]), lo = __ldg(&st[np]), s1f = __ldg(&st[2 * np]), s2f = __ldg(&st[3 * np]),
                     rf = __ldg(&st[4 * np]);
-        ff_add(A, hi);
-        A.lo = __fadd_rn(A.lo, lo);
+        ff3_add(A, hi);
+        ff3_add_low(A, lo);
         // the segment's blocks that count
         const int f0 = sg << sl, f1 = min(f0 + (1 << sl), a.num);
         const int cnt = min(pnum, (f1 + (1 << ind) - 1) >> ind) - (f0 >> ind);
         if (cnt <= 0) continue;
         // sums of P - r0 from those of P - r: with dr = r - r0,
         // S1 += s1 + cnt dr and S2 += s2 + dr (2 s1 + cnt dr)
-        ff_add(s1, s1f);
-        ff_add(s2, s2f);
+        ff3_add(s1, s1f);
+        ff3_add(s2, s2f);
         const double dr = f2d(rf) - r0, c = f2d((float)cnt);
         S1 = fma(c, dr, S1);
         S2 = fma(dr, fma(c, dr, f2d(2.f * s1f)), S2);
     }
-    S1 += f2d(s1.hi) + f2d(s1.lo);
-    S2 += f2d(s2.hi) + f2d(s2.lo);
-    double Ad = f2d(A.hi) + f2d(A.lo);
+    S1 += ff3_val(s1);
+    S2 += ff3_val(s2);
+    double Ad = ff3_val(A);
     if (!(isfinite(A.hi) && isfinite(s1.hi) && isfinite(s2.hi)) && !bad)
         plain_segments(&stat_ref(a.o.stats, a.npix, lag, 0, pix), np, a.stat_stride, nseg, sl, a.num, ind, pnum, r0, Ad,
                        S1, S2);

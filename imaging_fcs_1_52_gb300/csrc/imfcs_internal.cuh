@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "imfcs_gb300.h"
+#include "imfcs_num.cuh"
 
 namespace imfcs {
 
@@ -82,70 +83,15 @@ struct LagInfo {
     int pnum_by_ind[kMaxBlockLevels];  // pnum for each possible block index
     int nsnap;
     // reciprocals (an FP64 division is a dozen FP64 operations, and GB300
-    // issues those at 1/64 of the FP32 rate)
+    // issues those at 1/64 of the FP32 rate); with div_by the quotients are those
+    // of the division
     double inv_prodnum[kMaxChan];          // 1 / prodnum
     double inv_pnum[kMaxBlockLevels];      // 1 / pnum, 1 / (pnum - 1) per block index
     double inv_pnum1[kMaxBlockLevels];
     double blk_inv_n[kMaxBlockLevels];     // blocking level y: 1 / n, n = (num - 1) >> y,
-    double blk_err[kMaxBlockLevels];       // and 1 / sqrt(2 (n - 1))
+    double blk_root[kMaxBlockLevels];      // sqrt(2 (n - 1)) and its reciprocal
+    double blk_inv_root[kMaxBlockLevels];
 };
-
-// ---------------------------------------------------------------------------
-// Float-float (double-single) accumulation: exact two-sum (Knuth).
-// ---------------------------------------------------------------------------
-struct ff {
-    float hi, lo;
-};
-__device__ __forceinline__ void ff_add(ff &a, float b)
-{
-    float s = __fadd_rn(a.hi, b);
-    float bb = __fsub_rn(s, a.hi);
-    float err = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    a.hi = s;
-    a.lo = __fadd_rn(a.lo, err);
-}
-__device__ __forceinline__ double ff_val(const ff &a) { return (double)a.hi + (double)a.lo; }
-
-// float -> double off the FP64 pipe, where the conversion instruction runs at
-// 1/64 of the FP32 rate (exact): the exponent rebiased, the fraction moved.
-// Subnormal values are scaled by 2^64 first; selects, no branch, so that the
-// instruction is never issued beside them.
-__device__ __forceinline__ double f2d(float x)
-{
-    unsigned m = __float_as_uint(x) & 0x7fffffffu;
-    unsigned bias = m >= 0x7f800000u ? 0x70000000u : 0x38000000u;
-    const unsigned scaled = __float_as_uint(fabsf(x) * 18446744073709551616.f);
-    if (m < 0x00800000u) {
-        m = scaled;
-        bias = m ? 0x34000000u : 0u;
-    }
-    const unsigned hi = ((m >> 3) + bias) | (__float_as_uint(x) & 0x80000000u);
-    return __hiloint2double((int)hi, (int)(m << 29));
-}
-
-// 1/x and sqrt(x) by Newton's iteration from an FP32 start, 24 -> 48 -> 53
-// bits: six and nine FP64 operations.  Arguments outside [1e-30, 1e30] (and
-// non-finite, zero, negative ones) take the plain operation.
-static __device__ __noinline__ double plain_rcp(double x) { return 1.0 / x; }
-static __device__ __noinline__ double plain_sqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double newton_rcp(double x)
-{
-    const float f = fabsf((float)x);
-    if (!(f > 1e-30f && f < 1e30f)) return plain_rcp(x);
-    double r = f2d(copysignf(1.f / f, (float)x));
-    r = fma(fma(-x, r, 1.0), r, r);
-    return fma(fma(-x, r, 1.0), r, r);
-}
-__device__ __forceinline__ double newton_sqrt(double x)
-{
-    const float f = (float)x;
-    if (!(f > 1e-30f && f < 1e30f)) return plain_sqrt(x);
-    const double y = f2d(rsqrtf(f)), h = f2d(0.5f * rsqrtf(f));
-    double s = x * y;
-    const double e = fma(-s, h, 0.5);      // s = sqrt(x) (1 - e)^..., h = 1 / (2 sqrt(x))
-    s = fma(s, e, s);
-    return fma(fma(-s, s, x), fma(h, e, h), s);
-}
 
 // ---------------------------------------------------------------------------
 // Window value of one trace at frame t (0-based, relative to job.first).

@@ -195,17 +195,6 @@ __global__ void __launch_bounds__(256) trace_windows_kernel(Job j, const unsigne
 // issue is 87).
 // ---------------------------------------------------------------------------
 
-// x / d for d = 2 .. 8, the bits of the division (checked for every mantissa):
-// the quotient's remainder corrects it.
-template <int D>
-__device__ __forceinline__ float div_small(float x)
-{
-    if constexpr ((D & (D - 1)) == 0) return x * (1.f / D);
-    constexpr float inv = 1.f / D;
-    const float q = __fmul_rn(x, inv);
-    return fmaf(fmaf(-q, (float)D, x), inv, q);
-}
-
 // legendre() with its roundings.
 template <int K, int N = 1>
 __device__ __forceinline__ void legendre_k(float u, float (&out)[K])
@@ -976,16 +965,6 @@ __global__ void __launch_bounds__(128, 4) bleach_exp_kernel(Job j, const float *
 // pipe, the divisions by the product counts from their reciprocals in the lag
 // table, the counts of non-finite frames as integers (0.31 -> 0.13 ms at
 // 16,384 pixels x 50,000 frames).
-
-// x / n, correctly rounded, from inv = 1 / n correctly rounded (n a small
-// whole number): the quotient's remainder corrects it (Markstein).  The means
-// of unbleached recordings are ratios of short numbers that sit on FP32
-// rounding ties, so x * inv alone would round some of them the other way.
-__device__ __forceinline__ double div_by(double x, double n, double inv)
-{
-    const double q = x * inv;
-    return fma(fma(-q, n, x), inv, q);
-}
 __global__ void __launch_bounds__(128) monitor_finalize_kernel(Job j, const LagInfo *li, const float *bparams,
                                         int nseg, const float2 *segtot, const float2 *snap_part,
                                         const int *segbad, const int *snap_bad, float4 *mon, float4 *blkmon)
@@ -1189,16 +1168,16 @@ __global__ void __launch_bounds__(128) block_kernel(Job j, const float *s0a, con
 }
 
 // Blocking decision.  A CTA serves 32 pixels with 16 threads each: thread
-// (pixel, y) sums the segments' statistics of level y (and y + 16) in
-// float-float (coalesced across pixels, in segment order), the levels above
-// the segment size from segment sums, and takes the level's standard deviation
-// in FP64; then one thread per pixel applies the overlap / monotonic-increase
+// (pixel, y) sums the segments' statistics of level y (and y + 16) in three
+// FP32 terms, no less precise than FP64 (coalesced across pixels, in segment
+// order), the levels above the segment size from segment sums, and takes the
+// level's standard deviation in FP64; then one thread per pixel applies the overlap / monotonic-increase
 // criteria of java:9339-9380.  FP64 sums by 8 threads a pixel: 0.39 ms at
-// 16,384 pixels x 50,000 frames, this 0.06.
+// 16,384 pixels x 50,000 frames, this 0.07.
 constexpr int kBlkFinPix = 32, kBlkFinLev = 16;
 
 // f(value, value) over n pairs `stride` apart, the loads of U at a time.
-template <int U, bool TWO, class F>
+template <int U, class F>
 __device__ __forceinline__ void blk_walk(const float *p1, const float *p2, size_t stride, int n, F f)
 {
     int i = 0;
@@ -1207,7 +1186,7 @@ __device__ __forceinline__ void blk_walk(const float *p1, const float *p2, size_
 #pragma unroll
         for (int u = 0; u < U; u++) {
             v[u] = __ldg(&p1[u * stride]);
-            w[u] = TWO ? __ldg(&p2[u * stride]) : 0.f;
+            w[u] = __ldg(&p2[u * stride]);
         }
         p1 += U * stride;
         p2 += U * stride;
@@ -1215,41 +1194,38 @@ __device__ __forceinline__ void blk_walk(const float *p1, const float *p2, size_
         for (int u = 0; u < U; u++) f(v[u], w[u]);
     }
     for (; i < n; i++) {
-        f(__ldg(p1), TWO ? __ldg(p2) : 0.f);
+        f(__ldg(p1), __ldg(p2));
         p1 += stride;
         p2 += stride;
     }
 }
 
 // Sums a1, a2 of the means and squared means of nb blocks of S * parts segment
-// sums each (inv: 1 / products of a block), loads of 16 at a time: whole
-// blocks where S < 16.
+// sums each (inv: 1 / products of a block, a power of two), loads of 16 at a
+// time: whole blocks where S < 16.
 template <int S>
-__device__ __forceinline__ void blk_upper(const float *p, size_t stride, int nb, int parts, float inv, ff &a1, ff &a2)
+__device__ __forceinline__ void blk_upper(const float *p, size_t stride, int nb, int parts, float inv, ff3 &a1,
+                                          ff3 &a2)
 {
     constexpr int G = 16 / S;             // blocks per batch
-    auto block = [&](const ff &sb) {
-        // the block's mean m (exact scaling) and its square
-        const f2 m = f2_quick(sb.hi * inv, sb.lo * inv), m2 = f2_mul(m, m);
-        ff_add(a1, m.hi);
-        ff_add(a2, m2.hi);
-        a1.lo = __fadd_rn(a1.lo, m.lo);
-        a2.lo = __fadd_rn(a2.lo, m2.lo);
-    };
     for (int b = 0; b < nb; b += G) {
-        ff sb[G];
+        ff3 sb[G];
 #pragma unroll
-        for (int g = 0; g < G; g++) sb[g] = {0.f, 0.f};
+        for (int g = 0; g < G; g++) sb[g] = {0.f, 0.f, 0.f};
         for (int q = 0; q < parts; q++, p += 16 * stride) {
             float v[16];
 #pragma unroll
             for (int u = 0; u < 16; u++) v[u] = b + u / S < nb ? __ldg(&p[u * stride]) : 0.f;
 #pragma unroll
-            for (int u = 0; u < 16; u++) ff_add(sb[u / S], v[u]);
+            for (int u = 0; u < 16; u++) ff3_add(sb[u / S], v[u] * inv);
         }
 #pragma unroll
-        for (int g = 0; g < G; g++)
-            if (b + g < nb) block(sb[g]);
+        for (int g = 0; g < G; g++) {     // (past the last block: zeros)
+            ff3_add(a1, sb[g].hi);
+            ff3_add_low(a1, sb[g].mid);
+            a1.lo = __fadd_rn(a1.lo, sb[g].lo);
+            ff3_add_square(a2, sb[g]);
+        }
     }
 }
 
@@ -1287,19 +1263,18 @@ block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s
     const int full_segs = (j.num - 1) / kBlkSeg;   // segments holding kBlkSeg products
     if (pix < j.npix && ty < blocknum) {
         const float4 bm = blkmon[pix];
-        const double iq = newton_rcp(f2d(bm.z) * f2d(bm.w));
-        const double iq2 = iq * iq;
+        const double dmDm = f2d(bm.z) * f2d(bm.w), idm = newton_rcp(dmDm);
         for (int y = ty; y < blocknum; y += kBlkFinLev) {
             if (bm.x != bm.x || bm.y != bm.y) {     // a non-finite frame: every product is non-finite
                 vb[y][pl] = __longlong_as_double(0x7ff8000000000000ll);
                 continue;
             }
-            ff a1 = {0.f, 0.f}, a2 = {0.f, 0.f};
+            ff3 a1 = {0.f, 0.f, 0.f}, a2 = a1;
             if (y <= kBlkSegLog) {
                 const size_t o = (size_t)y * nbseg * j.npix + pix;
-                blk_walk<16, true>(s1 + o, s2 + o, j.npix, nbseg, [&](float v, float w) {
-                    ff_add(a1, v);
-                    ff_add(a2, w);
+                blk_walk<16>(s1 + o, s2 + o, j.npix, nbseg, [&](float v, float w) {
+                    ff3_add(a1, v);
+                    ff3_add(a2, w);
                 });
             } else {
                 // levels above the segment: block y spans 2^(y-8) consecutive
@@ -1313,12 +1288,12 @@ block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s
                 else if (span == 8) blk_upper<8>(p, j.npix, nb, 1, inv, a1, a2);
                 else blk_upper<16>(p, j.npix, nb, span / 16, inv, a1, a2);
             }
-            double A1 = f2d(a1.hi) + f2d(a1.lo), A2 = f2d(a2.hi) + f2d(a2.lo);
+            double A1 = ff3_val(a1), A2 = ff3_val(a2);
             if (!(isfinite(a1.hi) && isfinite(a2.hi)))
                 blk_plain_sums(s1, s2, segsum, y, nbseg, full_segs, j.npix, pix, A1, A2);
-            const double in = li->blk_inv_n[y];
-            const double m1 = A1 * in, m2 = A2 * in;
-            vb[y][pl] = newton_sqrt((m2 - m1 * m1) * in * iq2);
+            const double n = f2d((float)((j.num - 1) >> y)), in = li->blk_inv_n[y];
+            const double m1 = div_by(A1, n, in), m2 = div_by(A2, n, in);
+            vb[y][pl] = newton_sqrt(div_near(fma(-m1, m1, m2), n * dmDm * dmDm, in * idm * idm));
         }
     }
     __syncthreads();
@@ -1326,9 +1301,9 @@ block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s
     // criteria as bit masks over the levels: error bars of neighbours overlap
     // (crt), the deviation grows (pos)
     unsigned crt = 0, pos = 0;
-    double v0 = vb[0][pl], e0 = v0 * li->blk_err[0];
+    double v0 = vb[0][pl], e0 = div_by(v0, li->blk_root[0], li->blk_inv_root[0]);
     for (int x = 0; x + 1 < blocknum; x++) {
-        const double v1 = vb[x + 1][pl], e1 = v1 * li->blk_err[x + 1];
+        const double v1 = vb[x + 1][pl], e1 = div_by(v1, li->blk_root[x + 1], li->blk_inv_root[x + 1]);
         if (v0 + e0 > v1 - e1 && v1 + e1 > v0 - e0) crt |= 1u << x;
         if (v1 - v0 > 0) pos |= 1u << x;
         v0 = v1;
