@@ -177,9 +177,21 @@ static bool acf_config_from(const imfcs_acf_parameters *p, imfcs_config &c, std:
     return true;
 }
 
+// Device buffers of a calcACF call besides its plan: input, outputs and (not in
+// N&B mode) the lag-major copies.
+static size_t acf_call_bytes(const imfcs_acf_parameters *p, size_t npix, size_t chanum, size_t frames)
+{
+    return (size_t)p->w_temp * p->h_temp * frames * sizeof(float) +
+           npix * (chanum * (p->isNBcalculation ? 2 : 4) * sizeof(double) + 3 * sizeof(double) + 2 * sizeof(int));
+}
+
+// What the call will allocate: its buffers and the plan's tables and scratch (a
+// trial plan without scratch, as the bands size theirs).  A configuration the
+// call refuses is estimated from its input and outputs.
 extern "C" int imfcs_is_acf_memory_sufficient(const imfcs_acf_parameters *p)
 {
     if (!p) return 0;
+    const double free_bytes = (double)free_device_bytes();
     const int frames = p->lastframe - p->firstframe + 1;
     const double npix = (double)p->width * p->height;
     const double ch = p->chanum;
@@ -187,7 +199,16 @@ extern "C" int imfcs_is_acf_memory_sufficient(const imfcs_acf_parameters *p)
                   + npix * ch * (8.0 * 3 + 16 + 20)                    // outputs, monitors, stats
                   + npix * 2 * 1000 * 4.0                              // averaged traces
                   + npix * 2 * ((frames + 255) / 256) * 8.0 * 12;      // segment scratch
-    return need < 0.9 * (double)free_device_bytes() ? 1 : 0;
+    std::string err;
+    imfcs_config c;
+    imfcs_plan *pl = nullptr;
+    if (need < 0.9 * free_bytes && acf_config_from(p, c, err) &&
+        plan_create_ex(&c, 1, p->w_temp, p->h_temp, c.bleach == IMFCS_BLEACH_POLYNOMIAL, &pl, true) == 0) {
+        need = (double)plan_scratch_need(pl) + (double)imfcs_plan_scratch_bytes(pl) +
+               (double)acf_call_bytes(p, (size_t)npix, (size_t)p->chanum, (size_t)frames);
+        imfcs_plan_destroy(pl);
+    }
+    return need < 0.9 * free_bytes ? 1 : 0;
 }
 
 // Monomial coefficients in t (seconds) -> Legendre coefficients in
