@@ -152,13 +152,14 @@ extern "C" int imfcs_band_window(const imfcs_config *cfg, int band_rows, int ban
 
 // Device bytes of a band job of `rows` output rows: the plan (scratch and
 // tables), two band buffers, the band's outputs.  The trial plan binds no
-// scratch, so sizing allocates only the plan's small tables.
-static int bands_need(const imfcs_config &c, int rows, size_t *total)
+// scratch, so sizing allocates only the plan's small tables.  cg_bytes: scratch
+// of the P = 32 correlator's pixel chunk (0: its own choice).
+static int bands_need(const imfcs_config &c, int rows, size_t cg_bytes, size_t *total)
 {
     const BandGeom g = band_geom(c, rows);
     const imfcs_config bc = band_config(c, g);
     imfcs_plan *pl = nullptr;
-    if (plan_create_ex(&bc, 0, bc.width, bc.height, false, &pl, true)) return 1;
+    if (plan_create_ex(&bc, 0, bc.width, bc.height, false, &pl, true, cg_bytes)) return 1;
     *total = plan_scratch_need(pl) + imfcs_plan_scratch_bytes(pl) +
              2 * (size_t)g.in_rows * c.width * c.num * sizeof(uint16_t) +
              (size_t)g.rows * c.out_w * output_bytes_per_pixel(c);
@@ -175,6 +176,7 @@ extern "C" int imfcs_bands_create(const imfcs_config *cfg, int band_rows, size_t
     if (!config_valid(cfg, err)) { set_error(err); return 1; }
     const imfcs_config &c = *cfg;
     int rows = band_rows > 0 ? std::min(band_rows, c.out_h) : 0;
+    size_t cg_bytes = 0;
     if (rows == 0) {
         size_t budget = max_device_bytes;
         if (budget == 0) {
@@ -182,24 +184,28 @@ extern "C" int imfcs_bands_create(const imfcs_config *cfg, int band_rows, size_t
             CK(cudaMemGetInfo(&fr, &tot));
             budget = fr / 10 * 9;
         }
-        // the footprint is linear in the rows: measure it at one and two
-        // rows, then shrink the estimate until it fits (alignment padding)
-        size_t t1 = 0, t2 = 0, total = 0;
-        if (bands_need(c, 1, &t1)) return 1;
-        if (t1 > budget) { set_error("device budget below one band of one output row"); return 1; }
-        if (c.out_h > 1 && bands_need(c, 2, &t2)) return 1;
-        const size_t per_row = t2 > t1 ? t2 - t1 : t1;
-        rows = (int)std::min<size_t>((size_t)c.out_h, 1 + (budget - t1) / per_row);
-        while (rows > 1) {   // rows falls every pass: ends at one row at the latest
-            if (bands_need(c, rows, &total)) return 1;
-            if (total <= budget) break;
-            rows = std::max(1, std::min(rows - 1, rows - rows / 16));
+        size_t total = 0;
+        if (bands_need(c, 1, 0, &total)) return 1;
+        if (total > budget && c.p == 32) {
+            // a row with the smallest chunk, then with the chunk that is left
+            if (bands_need(c, 1, 1, &total)) return 1;
+            if (total <= budget) cg_bytes = std::max<size_t>(budget - total, 1);
+        }
+        if (total > budget) { set_error("device budget below one band of one output row"); return 1; }
+        // the most rows that fit: the footprint grows with them (linearly but
+        // for the P = 32 chunk, whose scratch is bounded, and alignment)
+        rows = 1;
+        for (int hi = cg_bytes ? 1 : c.out_h; rows < hi;) {
+            const int mid = rows + (hi - rows + 1) / 2;
+            if (bands_need(c, mid, 0, &total)) return 1;
+            if (total <= budget) rows = mid;
+            else hi = mid - 1;
         }
     }
     const BandGeom g = band_geom(c, rows);
     const imfcs_config bc = band_config(c, g);
     imfcs_plan *pl = nullptr;
-    if (imfcs_plan_create(&bc, &pl)) return 1;
+    if (plan_create_ex(&bc, 0, bc.width, bc.height, false, &pl, false, cg_bytes)) return 1;
     imfcs_bands *b = new imfcs_bands();
     b->cfg = c;
     b->g = g;

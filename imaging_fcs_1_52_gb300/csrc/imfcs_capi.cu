@@ -421,7 +421,7 @@ namespace imfcs {
 bool config_valid(const imfcs_config *c, std::string &err) { return validate_config(c, err); }
 
 int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h, bool given_bleach,
-                   imfcs_plan **plan_out, bool external_scratch)
+                   imfcs_plan **plan_out, bool external_scratch, size_t cg_bytes)
 {
     std::string err;
     if (!plan_out) { set_error("null plan pointer"); return 1; }
@@ -439,6 +439,7 @@ int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h,
     Job &j = pl->job;
     memset(&j, 0, sizeof(j));
     j.in_w = in_w; j.in_h = in_h; j.input_float = input_float;
+    j.cg_bytes = cg_bytes;
     pl->given_bleach = given_bleach;
     j.first = cfg->first; j.num = cfg->num;
     j.out_w = cfg->out_w; j.out_h = cfg->out_h; j.map_x0 = cfg->map_x0; j.map_y0 = cfg->map_y0;

@@ -933,8 +933,10 @@ static CgPlan cg_plan(const Job &j)
     p.lv *= j.is_ccf ? 2 : 1;
     p.pz = (size_t)j.chanum * p.pnum_max;
     p.tot = (size_t)2 * j.chanum * p.nseg;
-    size_t c = kCgChunkBytes / ((p.lv + p.pz + p.tot) * sizeof(float));
+    const size_t pixel = (p.lv + p.pz + p.tot) * sizeof(float);
+    size_t c = kCgChunkBytes / pixel;
     c = c < 64 ? 64 : c & ~(size_t)63;
+    if (j.cg_bytes) c = j.cg_bytes / pixel > 1 ? j.cg_bytes / pixel : 1;
     p.chunk = (int)(c < (size_t)j.npix ? c : (size_t)j.npix);
     return p;
 }

@@ -96,9 +96,10 @@ void legendre_basis_table(int order, int num, double frametime, double uscale, d
 bool config_valid(const imfcs_config *c, std::string &err);
 
 // external_scratch: the plan's per-execution scratch is not allocated; a
-// batch binds an arena of plan_scratch_need bytes before each execution
+// batch binds an arena of plan_scratch_need bytes before each execution;
+// cg_bytes: Job::cg_bytes
 int plan_create_ex(const imfcs_config *cfg, int input_float, int in_w, int in_h, bool given_bleach,
-                   imfcs_plan **plan_out, bool external_scratch = false);
+                   imfcs_plan **plan_out, bool external_scratch = false, size_t cg_bytes = 0);
 int plan_execute_any(imfcs_plan *pl, const void *dev_stack, const imfcs_outputs *dev_out, void *stream);
 bool corr2_supported(const Job &j);          // the level chain runs (P = 16, Q >= 5)
 

@@ -63,6 +63,8 @@ struct Job {
     // of the tail kernel, 2^c2_seg_extra and 2^c2_tail_extra times the
     // shortest legal segment
     int c2_cta, c2_seg_extra, c2_tail_extra;
+    // scratch bytes of a pixel chunk of the P = 32 correlator (0: its own choice)
+    size_t cg_bytes;
 };
 
 // Lag tables, snapshot positions and per-lag snapshot indices, stored in a

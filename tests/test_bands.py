@@ -119,6 +119,27 @@ def test_bands_sized_from_a_device_budget():
 
 
 @pytest.mark.gpu
+def test_p32_bands_under_tight_budgets():
+    """The P = 32 correlator's chunk scratch gives way to the budget: down to
+    0.65 of what a row takes with the chunk of its own choice (the level-0
+    stream and the band buffers, without any chunk, are some 0.55) a row is
+    accepted; larger budgets take the most rows that fit."""
+    from tests.synth import brownian_stack
+    st = brownian_stack(40, 6, 9000, seed=5, density=2.0, cps=3e4)
+    cfg = engine.FCSConfig(width=40, height=6, frames=9000, background=100, p=32, do_fit=False)
+    ref = engine.run_host(st, cfg)
+    row_b = engine.Bands(cfg, band_rows=1)
+    row = row_b.geometry()["device_bytes"]
+    row_b.close()
+    for part, rows in ((0.65, 1), (0.8, 1), (1.05, 1), (3.2, 3)):
+        bands = engine.Bands(cfg, max_device_bytes=int(part * row))
+        g = bands.geometry()
+        assert g["band_rows"] == rows and g["device_bytes"] <= part * row
+        _compare(ref, bands.execute_host(st), engine.output_names(cfg))
+        bands.close()
+
+
+@pytest.mark.gpu
 def test_bands_refuse_a_background_image():
     """A background image on the band plan would cover one band's rows only:
     execution is refused."""
