@@ -741,12 +741,14 @@ __device__ __forceinline__ void write_lag(const CorrOut &o, const float4 *mon, c
     // a non-finite frame in the lag's windows: NaN, whatever the sums
     double acf = __longlong_as_double(0x7ff8000000000000ll), bv = acf, cov = acf;
     if (m.x == m.x && m.y == m.y) {
-        const double n = f2d((float)li->prodnum[lag]), pn = f2d((float)li->pnum_by_ind[ind]), ip = li->inv_pnum[ind];
-        const double dmDm = f2d(m.z) * f2d(m.w), idm = newton_rcp(dmDm);
+        const int pnum = li->pnum_by_ind[ind];
+        const double n = f2d((float)li->prodnum[lag]), pn = f2d((float)pnum), ip = li->inv_pnum[ind];
+        const double dmDm = f2d(m.z) * f2d(m.w), idm = rcp_near(dmDm, m.z * m.w);
         const double sumprod = fma(-(n * f2d(m.x)), f2d(m.y), A), in = li->inv_prodnum[lag];   // centred products
         const double mean = div_by(S1, pn, ip);
-        cov = div_by(sumprod, n, in);
-        bv = div_near(fma(-mean, mean, div_by(S2, pn, ip)), (pn - 1.0) * dmDm * dmDm, li->inv_pnum1[ind] * idm * idm);
+        if (lag == 1) cov = div_by(sumprod, n, in);
+        bv = div_near(fma(-mean, mean, div_by(S2, pn, ip)), f2d((float)(pnum - 1)) * dmDm * dmDm,
+                      li->inv_pnum1[ind] * idm * idm);
         if (o.gls) acf = div_near(fma(pn, r, S1), pn * dmDm, ip * idm);    // mcov (java:9526-9531)
         else acf = div_near(sumprod, n * dmDm, in * idm);
     }
@@ -779,7 +781,7 @@ static __device__ __noinline__ void plain_segments(const float *st, size_t np, s
 // Grid (pixel blocks, lags).  Bound by FP64 issue (1/64 of the FP32 rate):
 // plain sums of FP32 values run in three FP32 terms, no less precise than FP64,
 // the products with the segments' shifts are FP64, conversions go to the
-// integer pipe, quotients are corrected products with reciprocals.  0.56 -> 0.21
+// integer pipe, quotients are corrected products with reciprocals.  0.56 -> 0.19
 // ms at 16,384 pixels x 50,000 frames.  Float-float for those products too was
 // no faster and moved results by 1e-13, enough to round some of the fits' FP32
 // data and weights the other way.
@@ -799,23 +801,33 @@ __global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
     double S1 = 0.0, S2 = 0.0;
     const float4 m = a.mon[(size_t)pix * a.chanum + lag];
     const bool bad = m.x != m.x || m.y != m.y;      // a non-finite frame in the lag's windows: NaN, whatever the sums
-#pragma unroll 2
-    for (int sg = 0; sg < nseg && !bad; sg++, st += a.stat_stride) {
-        const float hi = __ldg(&st[0]), lo = __ldg(&st[np]), s1f = __ldg(&st[2 * np]), s2f = __ldg(&st[3 * np]),
-                    rf = __ldg(&st[4 * np]);
-        ff3_add(A, hi);
-        ff3_add_low(A, lo);
-        // the segment's blocks that count
-        const int f0 = sg << sl, f1 = min(f0 + (1 << sl), a.num);
-        const int cnt = min(pnum, (f1 + (1 << ind) - 1) >> ind) - (f0 >> ind);
-        if (cnt <= 0) continue;
-        // sums of P - r0 from those of P - r: with dr = r - r0,
-        // S1 += s1 + cnt dr and S2 += s2 + dr (2 s1 + cnt dr)
-        ff3_add(s1, s1f);
-        ff3_add(s2, s2f);
-        const double dr = f2d(rf) - r0, c = f2d((float)cnt);
-        S1 = fma(c, dr, S1);
-        S2 = fma(dr, fma(c, dr, f2d(2.f * s1f)), S2);
+    constexpr int U = 4;                            // segments whose statistics load together
+    for (int sb = 0; sb < nseg && !bad; sb += U) {
+        float v[U][kStatN];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int f = 0; f < kStatN; f++)
+                v[u][f] = sb + u < nseg ? __ldg(&st[(size_t)u * a.stat_stride + f * np]) : 0.f;
+        st += U * a.stat_stride;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int sg = sb + u;
+            if (sg >= nseg) break;
+            ff3_add(A, v[u][0]);
+            ff3_add_low(A, v[u][1]);
+            // the segment's blocks that count
+            const int f0 = sg << sl, f1 = min(f0 + (1 << sl), a.num);
+            const int cnt = min(pnum, (f1 + (1 << ind) - 1) >> ind) - (f0 >> ind);
+            if (cnt <= 0) continue;
+            // sums of P - r0 from those of P - r: with dr = r - r0,
+            // S1 += s1 + cnt dr and S2 += s2 + dr (2 s1 + cnt dr)
+            ff3_add(s1, v[u][2]);
+            ff3_add(s2, v[u][3]);
+            const double dr = f2d(v[u][4]) - r0, c = f2d((float)cnt);
+            S1 = fma(c, dr, S1);
+            S2 = fma(dr, fma(c, dr, f2d(2.f * v[u][2])), S2);
+        }
     }
     S1 += ff3_val(s1);
     S2 += ff3_val(s2);

@@ -78,28 +78,29 @@ __device__ __forceinline__ double f2d(float x)
 
 __device__ __forceinline__ double ff3_val(const ff3 &a) { return f2d(a.hi) + (f2d(a.mid) + f2d(a.lo)); }
 
-// 1/x and sqrt(x) by Newton's iteration from an FP32 start, 24 -> 48 -> 53
-// bits: six and nine FP64 operations.  Arguments outside [1e-30, 1e30] (and
-// non-finite, zero, negative ones) take the plain operation.
+// 1/x to 46 bits (for div_near) and sqrt(x) within 0.5 ulp and 1e-15, by
+// Newton's iteration from an FP32 start: two and six FP64 operations.  xf: x
+// within a few FP32 ulps, from a caller that has it without a conversion.
+// Arguments outside [1e-30, 1e30] (and non-finite, zero, negative ones) take
+// the plain operation.
 static __device__ __noinline__ double plain_div(double x, double y) { return x / y; }
 static __device__ __noinline__ double plain_sqrt(double x) { return sqrt(x); }
-__device__ __forceinline__ double newton_rcp(double x)
+__device__ __forceinline__ double rcp_near(double x, float xf)
 {
-    const float f = fabsf((float)x);
+    const float f = fabsf(xf);
     if (!(f > 1e-30f && f < 1e30f)) return plain_div(1.0, x);
-    double r = f2d(copysignf(1.f / f, (float)x));
-    r = fma(fma(-x, r, 1.0), r, r);
+    const double r = f2d(1.f / xf);
     return fma(fma(-x, r, 1.0), r, r);
 }
 __device__ __forceinline__ double newton_sqrt(double x)
 {
     const float f = (float)x;
     if (!(f > 1e-30f && f < 1e30f)) return plain_sqrt(x);
-    const double y = f2d(rsqrtf(f)), h = f2d(0.5f * rsqrtf(f));
-    double s = x * y;
-    const double e = fma(-s, h, 0.5);      // s = sqrt(x) (1 - e)^..., h = 1 / (2 sqrt(x))
-    s = fma(s, e, s);
-    return fma(fma(-s, s, x), fma(h, e, h), s);
+    const float yf = rsqrtf(f);
+    const double y = f2d(yf), h = f2d(0.5f * yf);
+    double s = x * y;                      // sqrt(x) (1 - e), h = 1 / (2 sqrt(x))
+    s = fma(s, fma(-s, h, 0.5), s);
+    return fma(fma(-s, s, x), h, s);
 }
 
 // x / n, correctly rounded, from inv = 1 / n correctly rounded (n a small
@@ -112,9 +113,10 @@ __device__ __forceinline__ double div_by(double x, double n, double inv)
     return fma(fma(-q, n, x), inv, q);
 }
 
-// x / y the same way from any reciprocal `inv` of y within a few ulps: within
-// 0.5 ulp and 1e-15.  The plain division where the quotient is zero,
-// non-finite or tiny (y outside the range of its reciprocal among them).
+// x / y the same way from a reciprocal `inv` of y good to 40 bits (its error
+// enters squared): within 0.5 ulp and 1e-9.  The plain division where the
+// quotient is zero, non-finite or tiny (y outside the range of its reciprocal
+// among them).
 __device__ __forceinline__ double div_near(double x, double y, double inv)
 {
     const double q = x * inv;

@@ -1256,17 +1256,18 @@ __global__ void __launch_bounds__(kBlkFinPix * kBlkFinLev)
 block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s1, const float *s2, const float *segsum,
                       const float4 *blkmon, int *ind_out, int *ok_out)
 {
-    __shared__ double vb[kMaxBlockLevels][kBlkFinPix];
+    // the levels' standard deviations and their error bars' ends
+    __shared__ double vb[kMaxBlockLevels][kBlkFinPix], up[kMaxBlockLevels][kBlkFinPix], lo[kMaxBlockLevels][kBlkFinPix];
     const int pl = threadIdx.x % kBlkFinPix, ty = threadIdx.x / kBlkFinPix;
     const int pix = blockIdx.x * kBlkFinPix + pl;
     const int blocknum = j.blocknum;
     const int full_segs = (j.num - 1) / kBlkSeg;   // segments holding kBlkSeg products
     if (pix < j.npix && ty < blocknum) {
         const float4 bm = blkmon[pix];
-        const double dmDm = f2d(bm.z) * f2d(bm.w), idm = newton_rcp(dmDm);
+        const double dmDm = f2d(bm.z) * f2d(bm.w), idm = rcp_near(dmDm, bm.z * bm.w);
         for (int y = ty; y < blocknum; y += kBlkFinLev) {
             if (bm.x != bm.x || bm.y != bm.y) {     // a non-finite frame: every product is non-finite
-                vb[y][pl] = __longlong_as_double(0x7ff8000000000000ll);
+                vb[y][pl] = up[y][pl] = lo[y][pl] = __longlong_as_double(0x7ff8000000000000ll);
                 continue;
             }
             ff3 a1 = {0.f, 0.f, 0.f}, a2 = a1;
@@ -1293,7 +1294,11 @@ block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s
                 blk_plain_sums(s1, s2, segsum, y, nbseg, full_segs, j.npix, pix, A1, A2);
             const double n = f2d((float)((j.num - 1) >> y)), in = li->blk_inv_n[y];
             const double m1 = div_by(A1, n, in), m2 = div_by(A2, n, in);
-            vb[y][pl] = newton_sqrt(div_near(fma(-m1, m1, m2), n * dmDm * dmDm, in * idm * idm));
+            const double v = newton_sqrt(div_near(fma(-m1, m1, m2), n * dmDm * dmDm, in * idm * idm));
+            const double e = div_by(v, li->blk_root[y], li->blk_inv_root[y]);
+            vb[y][pl] = v;
+            up[y][pl] = v + e;
+            lo[y][pl] = v - e;
         }
     }
     __syncthreads();
@@ -1301,13 +1306,9 @@ block_finalize_kernel(Job j, const LagInfo *li, int q, int nbseg, const float *s
     // criteria as bit masks over the levels: error bars of neighbours overlap
     // (crt), the deviation grows (pos)
     unsigned crt = 0, pos = 0;
-    double v0 = vb[0][pl], e0 = div_by(v0, li->blk_root[0], li->blk_inv_root[0]);
     for (int x = 0; x + 1 < blocknum; x++) {
-        const double v1 = vb[x + 1][pl], e1 = div_by(v1, li->blk_root[x + 1], li->blk_inv_root[x + 1]);
-        if (v0 + e0 > v1 - e1 && v1 + e1 > v0 - e0) crt |= 1u << x;
-        if (v1 - v0 > 0) pos |= 1u << x;
-        v0 = v1;
-        e0 = e1;
+        if (up[x][pl] > lo[x + 1][pl] && up[x + 1][pl] > lo[x][pl]) crt |= 1u << x;
+        if (vb[x + 1][pl] > vb[x][pl]) pos |= 1u << x;
     }
     const unsigned below = (1u << (blocknum - 2)) - 1;
     unsigned cr12 = crt & (crt >> 1) & below;

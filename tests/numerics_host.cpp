@@ -69,15 +69,15 @@ double num_sum3_squares(const float *x, int n, int k)
     }
     return imfcs::ff3_val(s);
 }
-// the reciprocal a few ulps off
-double num_div(double x, double y, int ulps)
+// the FP32 start of the reciprocal a few ulps off
+double num_rcp(double x, int ulps)
 {
-    double inv = imfcs::newton_rcp(y);
-    for (int i = 0; i < ulps; i++) inv = nextafter(inv, INFINITY);
-    for (int i = 0; i > ulps; i--) inv = nextafter(inv, -INFINITY);
-    return imfcs::div_near(x, y, inv);
+    float f = (float)x;
+    for (int i = 0; i < ulps; i++) f = nextafterf(f, INFINITY);
+    for (int i = 0; i > ulps; i--) f = nextafterf(f, -INFINITY);
+    return imfcs::rcp_near(x, f);
 }
-double num_rcp(double x) { return imfcs::newton_rcp(x); }
+double num_div(double x, double y, int ulps) { return imfcs::div_near(x, y, num_rcp(y, ulps)); }
 double num_div_by(double x, double n) { return imfcs::div_by(x, n, 1.0 / n); }
 double num_sqrt(double x, int ulps)
 {

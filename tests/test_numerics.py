@@ -24,7 +24,7 @@ def lib(tmp_path_factory):
     for name, args in (("num_sum2", [C.c_void_p, C.c_int]), ("num_sum3", [C.c_void_p, C.c_int]),
                        ("num_sum3_low", [C.c_void_p, C.c_void_p, C.c_int]), ("num_f2d", [C.c_float]),
                        ("num_sum3_squares", [C.c_void_p, C.c_int, C.c_int]),
-                       ("num_div", [d, d, C.c_int]), ("num_rcp", [d]), ("num_div_by", [d, d]),
+                       ("num_div", [d, d, C.c_int]), ("num_rcp", [d, C.c_int]), ("num_div_by", [d, d]),
                        ("num_sqrt", [d, C.c_int])):
         getattr(L, name).argtypes, getattr(L, name).restype = args, d
     L.num_div_small_misses.restype = C.c_int
@@ -74,8 +74,8 @@ def test_quotients_and_roots_are_those_of_fp64(lib):
     for _ in range(4000):
         x = float(rng.choice([-1, 1]) * rng.lognormal(0, 15))
         y = float(rng.choice([-1, 1]) * rng.lognormal(0, 15))
-        assert ulps(lib.num_rcp(y), 1 / Fraction(y)) <= 0.5 + 1e-9
         for off in (-3, 0, 3):
+            assert abs(Fraction(lib.num_rcp(y, off)) * Fraction(y) - 1) <= Fraction(1, 2 ** 40)
             assert ulps(lib.num_div(x, y, off), Fraction(x) / Fraction(y)) <= 0.5 + 1e-9
         n = float(rng.integers(1, 5_000_000))
         assert lib.num_div_by(x, n) == x / n
