@@ -839,7 +839,7 @@ __global__ void __launch_bounds__(128) c2_finalize_kernel(C2Args a)
 }
 
 // P = 32: the block statistics of one (pixel, lag) over its blocks in order
-// (FP32, shifted by the first block), the segments' totals in FP64.
+// (FP32, shifted by the first block), the segments' totals in three FP32 terms.
 __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
 {
     const int pc = blockIdx.x * 128 + threadIdx.x, lag = blockIdx.y;
@@ -868,10 +868,21 @@ __global__ void __launch_bounds__(128) cg_finalize_kernel(CgArgs a)
     }
     const int sl = a.seg_log[lag <= a.p ? 0 : 1 + (lag - (a.p + 1)) / (a.p / 2)];
     const int nseg = (a.num + (1 << sl) - 1) >> sl;
-    double A = 0.0;
+    const float2 *tot = a.tot + (size_t)lag * a.cs + pc;
+    const size_t tstride = (size_t)a.chanum * a.cs;
+    ff3 At = {0.f, 0.f, 0.f};
     for (int sg = 0; sg < nseg; sg++) {
-        const float2 t = a.tot[((size_t)sg * a.chanum + lag) * a.cs + pc];
-        A += f2d(t.x) + f2d(t.y);
+        const float2 t = tot[sg * tstride];
+        ff3_add(At, t.x);
+        ff3_add_low(At, t.y);
+    }
+    double A = ff3_val(At);
+    if (!isfinite(At.hi)) {                         // beyond the FP32 range
+        A = 0.0;
+        for (int sg = 0; sg < nseg; sg++) {
+            const float2 t = tot[sg * tstride];
+            A += f2d(t.x) + f2d(t.y);
+        }
     }
     write_lag(a.o, a.mon, a.li, a.chanum, pix, lag, ind, A, f2d(S1), f2d(S2), f2d(r));
 }
