@@ -9,14 +9,14 @@
 //             frame-major ([t][pixel]): the level-0 sample stream s0;
 //   pair k    one thread per (pixel, frame segment) streams the level-k
 //             samples and correlates levels k and k+1 (lags 0..16 at level 0,
-//             delays 9..16 above) in registers: rings of the last 32 samples
-//             whose positions are compile-time constants inside a 64-sample
-//             unrolled step; it writes the level-(k+2) samples (pair sums of
-//             its level-(k+1) samples) for the next kernel;
+//             delays 9..16 above) in registers: a window of 32 samples that
+//             moves by register copies every 16, so that one step's code
+//             serves every step; it writes the level-(k+2) samples (pair sums
+//             of its level-(k+1) samples) for the next kernel;
 //   tail      levels k0..Q-1 (blocks possibly one sample long): one level per
 //             thread, samples built from the level-k0 stream, block
 //             statistics in registers;
-//   finalise  per (pixel, lag): segments combined in FP64, outputs.
+//   finalise  per (pixel, lag): segments combined at FP64 precision, outputs.
 //
 // Products are grouped by their direct sample y (processed when the delayed
 // samples y..y+16 are present), so the blocks of the blocked variance
@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) c2_tail_kernel(C2Args a, const f
 // 8 delays) over the whole recording -- two warps an SM at work, each summing
 // its samples from s0 again -- to 0.56 ms (blocks) + 0.06 (levels) + 0.08
 // (finalise).  A chunk's scratch (level streams and products, some 400 KB a
-// pixel at 50,000 frames) stays below 512 MB, less than the level-0 stream.
+// pixel at 50,000 frames and Q = 8) stays below 512 MB, with 64 pixels at
+// least; bands under a tight budget grant it what is left.
 // ---------------------------------------------------------------------------
 constexpr int kCgDelays = 17;                 // delays per thread: 0..16 and 17..32
 constexpr int kCgStep = 16;                   // samples per step of a thread

@@ -36,7 +36,7 @@ cudaError_t launch_bayes_combine(int npix, const double *lp1, const double *lp2,
 struct GlsArgs;
 cudaError_t launch_gls(const GlsArgs &g, cudaStream_t stream);
 
-// prep launchers (imfcs_prep_launch.cu)
+// prep launchers (imfcs_prep.cu)
 // scratch: level0_stream_floats floats (free until the streaming pass writes them)
 cudaError_t launch_trace(const Job &j, const void *stack, float *scratch, float *trace, cudaStream_t s);
 int trace_kernel_count(const Job &j);

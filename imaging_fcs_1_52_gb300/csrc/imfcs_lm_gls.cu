@@ -11,9 +11,10 @@
 // the code stays near the instruction caches, and chi^2 comes first: a rejected
 // step (about half of them) ends there, on the FP64 model without the FP32
 // model and its products.  Bound by FP64 issue where fits end in many FP64
-// steps (weak correlations), else by latency.  4,096 fits of 72 points: 0.54
-// -> 0.41 ms; 9,120 with an offset 5.47 -> 4.67 ms.  (The same machine gave
-// the OLS fits nothing: they take few steps and no products.)
+// steps (weak correlations), else by latency.  4,096 fits of 72 points: 0.67
+// ms with one row of a lane at a time, 0.54 with three side by side, 0.40 in
+// this form; 9,120 with an offset 5.47 -> 4.6 ms.  (The same machine gave the
+// OLS fits nothing: they take few steps and no products.)
 #include "imfcs_tirf.cuh"
 
 namespace imfcs {

@@ -303,7 +303,7 @@ __global__ void center_kernel(Job j, const float *trace, float *bp_out)
 //            variable projection (the oracle scans the same grid); double
 //            exponential: the reference's initial guesses;
 //   phase 1: FP32 Levenberg-Marquardt until the Gauss-Newton step is below
-//            1e-4 sigma + 1e-6 |p| (or no step lowers chi^2);
+//            1e-3 sigma + 1e-6 |p| (or no step lowers chi^2);
 //   phase 2: Newton with the full Hessian of chi^2/2 (J^T J - sum r d2f; the
 //            Gauss-Newton matrix alone does not contract on these
 //            large-residual problems), residuals and gradient in float-float

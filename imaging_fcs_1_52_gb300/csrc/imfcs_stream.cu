@@ -319,10 +319,10 @@ __device__ __forceinline__ void window_sums(const Job &j, const BoxGeo<TMA> &g, 
 }
 
 // Staged stream pass: grid (output tiles, ceil(nseg / segs)).  Bound by HBM
-// and issue about equally (2 B in, 4 B out a frame-pixel: 0.72 ms at
-// 128x128x50,000): eight frames at a time with the tests of the curve's form,
-// of non-finite values and of snapshots taken out of the frame loop 1.76 ->
-// 1.09 ms there; whole-row tiles of up to 128 threads with short boxes, and
+// and issue about equally: 2 B in and 4 B out a frame-pixel take 0.72 ms at the
+// copy rate for 128x128x50,000, the kernel 1.09 ms (1.76 before eight frames
+// went at a time, with the tests of the curve's form, of non-finite values and
+// of snapshots out of the frame loop); whole-row tiles of up to 128 threads with short boxes, and
 // the polynomial's coefficients in registers, 7.6 -> 0.59 ms for 2 x 2 binned
 // cross-correlation at 128x128x20,000 (32-thread CTAs with 83 KB each before)
 // and 1.50 -> 0.76 ms for overlapping 5 x 5 windows of rows of 101 (25 plain
