@@ -1395,12 +1395,18 @@ namespace imfcs {
 //     132, the left half of the frame at 12,345: 130 / 107): one pass;
 //   single pixels: two (64x64x1,999 46 / 38, 128x128x10,000 241 / 130,
 //     256x256x4,500 576 / 391), but in parts 79 / 89 (half the frame, 1,500);
-//   windows: two from two frames a point on (128x128, 3 x 3: 36 / 52 at one
-//     frame, 54 / 50 at two, 89 / 50 at four; 512x512, 5 x 5: 189 / 237, 316 /
-//     294, 573 / 417), from three on where s0 holds less than a third of the sums
-//     (128x128, 16 x 16: 128 / 153 at two, 236 / 131 at four); those that use
-//     a value twice or more always (101x67, overlapping 5 x 5: 95 / 87 at one
-//     frame, 738 / 105 at twelve).
+//   windows whose rows do not overlap: two from two frames a point on (128x128,
+//     3 x 3: 36 / 52 at one frame, 54 / 50 at two, 89 / 50 at four; 512x512, 5 x
+//     5: 189 / 237, 316 / 294, 573 / 417), from three on where s0 holds less than
+//     a third of the sums (128x128, 16 x 16: 128 / 153 at two, 236 / 131 at four),
+//     from one on where a value is used twice (2 x 2 cross-correlation at
+//     128x128x1,500: 74 / 59);
+//   other windows, whose sums are as many as the raw values: where s0 holds them
+//     (overlapping 5 x 5 windows at 101x67: 95 / 87 at one frame, 738 / 105 at
+//     twelve), else with half as many frames again a point as parts, each of
+//     which adds up its windows anew (128x128, 8 x 8 in steps of 4: 113 / 152 at
+//     four frames and four parts, 183 / 135 at seven and three; 16 x 16 in steps
+//     of 8: 419 / 617 at seven and eleven, 1,160 / 327 at twenty and four).
 struct TracePlan {
     TraceSums g;
     int row0, points;
@@ -1424,9 +1430,12 @@ static TracePlan trace_plan(const Job &j)
     const size_t area = (size_t)j.binx * j.biny, values = (size_t)j.ntrace * area;
     if (3 * values <= raw) return p;
     const size_t points = level0_stream_floats(j) / ((size_t)p.g.lines * p.g.len), all = j.nopit;
-    if (area == 1 ? points < all
-                  : values < 2 * raw && (j.ave < 2 || (j.ave < 3 && 3 * points < all)))
-        return p;
+    bool one;
+    if (area == 1) one = points < all;
+    else if (j.ave < 2 && values < 2 * raw) one = true;
+    else if (p.rows) one = j.ave < 3 && 3 * points < all;
+    else one = points < all && 2 * j.ave * points <= 3 * all;
+    if (one) return p;
     p.points = points < (size_t)j.nopit ? (int)points : j.nopit;
     return p;
 }

@@ -42,8 +42,11 @@ def traces(st, cfg):
     (24, 16, 4100, {"binx": 2, "biny": 3, "cfy": 2}),
     (32, 32, 20000, {"pixbinx": 2, "pixbiny": 2, "out_w": 16, "out_h": 16}),
     (32, 8, 1900, {"out_w": 16, "q": 6}),
+    (40, 40, 10500, {"binx": 8, "biny": 8, "pixbinx": 4, "pixbiny": 4}),
+    (40, 40, 2500, {"binx": 8, "biny": 8, "pixbinx": 4, "pixbiny": 4}),
 ], ids=["rows8", "rows2", "rows1", "rows-gaps-range-cfx", "rows-parts", "rows-two-frames", "one-pass-parts",
-        "one-pass-short", "overlap", "cfy", "one-pass-sparse", "one-pass-half"])
+        "one-pass-short", "overlap", "cfy", "one-pass-sparse", "one-pass-half",
+        "overlap-parts", "one-pass-overlap"])
 def test_centre_is_the_mean_of_the_trace(w, h, frames, kw):
     rng = np.random.default_rng(81)
     st = rng.integers(100, 60000, (frames, h, w), dtype=np.uint16)
