@@ -13,8 +13,9 @@
 // completing on its own mbarrier) where the frames' rows are 16-byte aligned,
 // by 4-byte cp.async otherwise (any row length; each row is copied from its
 // start rounded down to a word).  The threads walk the staged frames in order,
-// eight at a time.  Float input, or a stack that is not 4-byte aligned, is
-// read with plain loads instead.
+// eight at a time.  Float input, a stack that is not 4-byte aligned and shapes
+// for which cp.async does not pay (stream_plan) are read with plain loads
+// instead.
 //
 // The exponential bleach curve is advanced by a recurrence e <- e q within
 // each 64-frame stage (reseeded with exp() per stage: at most 64 FP32
@@ -494,7 +495,8 @@ __global__ void __launch_bounds__(kStMaxThreads) stream_box_kernel(StreamArgs a,
     }
 }
 
-// Plain-load stream pass (float input, or a stack at an odd address): grid
+// Plain-load stream pass (float input, a stack at an odd address, or by
+// stream_plan's rule): grid
 // (ceil(npix/128), nseg), one thread per (pixel, segment).
 template <int MODE, bool CCF>
 __global__ void __launch_bounds__(128) stream_plain_kernel(StreamArgs a)
@@ -548,6 +550,17 @@ struct StreamPlan {
 // idle).  Boxes are as long as fits 56 KB for the ring (four CTAs per SM),
 // shorter for tiles that read many raw pixels; what does not fit at 8 frames
 // gets a smaller tile.
+//
+// The cp.async boxes cost a warp's turn per row and frame (per frame where the
+// tile is as wide as the frame), whatever the row's length.  Windows of several
+// pixels are worth up to four such rows a warp (plain / boxes, us: overlapping 5
+// x 5 at 11x6x15,253 404 / 58, 2 x 2 steps at 439x4x37,510 345 / 136; narrow
+// outputs of many rows, 1x158 of 3 x 1 windows at 4,242 frames 218 / 1,680, 6x47
+// of 2 x 1 at 6,441 130 / 295).  Single pixels gain where all four warps share
+// one copy a frame and the plain kernel's blocks leave the SMs part-empty,
+// from 100 pixels up to 600 blocks (123x8x18,566 71 / 57); else the plain kernel is faster
+// (13x1x2,627 36 / 67, a third of 25x44x7,172 52 / 218, 85x75x39,755 966 /
+// 1,605).
 static StreamPlan stream_plan(const Job &j, const void *stack, int nseg)
 {
     StreamPlan sp;
@@ -585,6 +598,16 @@ static StreamPlan stream_plan(const Job &j, const void *stack, int nseg)
             sp.col_rows = col_rows;
             sp.col_w = need;
             sp.smem = smem;
+            if (!sp.tma) {
+                const int warps = sp.threads / 32, copies = run ? 1 : rows;
+                const bool boxes = j.binx * j.biny > 1
+                                       ? run || rows <= 4 * warps
+                                       : 4 * copies <= warps && j.npix >= 100 && (j.npix + 127) / 128 * nseg <= 600;
+                if (!boxes) {
+                    sp.ok = 0;
+                    return sp;
+                }
+            }
             // several monitor segments per CTA keep its ring busy; one each
             // where that would leave SMs without a CTA
             sp.segs = 4;

@@ -34,3 +34,29 @@ def test_stack_addresses_give_the_same_bits(w, h, kw):
     for o in outs[1:]:
         for k in o:
             np.testing.assert_array_equal(o[k], outs[0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("w,h,kw", [
+    (33, 3, {"bleach": _lib.BLEACH_POLYNOMIAL}), (25, 4, {"bleach": _lib.BLEACH_POLYNOMIAL}),
+    (101, 1, {"cfx": 1, "bleach": _lib.BLEACH_SINGLE_EXP}), (25, 44, {"out_w": 8}), (43, 9, {"out_w": 14}),
+    (5, 16, {"binx": 3, "biny": 1}), (5, 17, {"binx": 3, "biny": 1}), (11, 64, {"binx": 5, "biny": 5, "pixbiny": 1}),
+    (21, 20, {"binx": 2, "biny": 3, "pixbinx": 1, "pixbiny": 1, "cfy": 1}),
+], ids=["99-pixels", "100-pixels", "one-row-ccf", "third-of-rows", "third-of-rows-2", "16-rows", "17-rows", "narrow-overlap",
+        "run-ccf"])
+def test_either_side_of_the_staging_rule(w, h, kw):
+    """Frames whose rows are not 16-byte aligned are staged by cp.async or read
+    with plain loads, by their shape; a stack at an odd address always takes
+    the plain loads.  Same bits."""
+    import torch
+    frames = 2900
+    st = engine.simulate(w, h, frames, steps_per_frame=1, density=4.0, cps=1e5, tau_bleach=20.0, seed=9)
+    plan = engine.Plan(engine.FCSConfig(width=w, height=h, frames=frames, background=100, do_fit=False, **kw))
+    buf = torch.zeros(st.numel() + 1, dtype=torch.int16, device="cuda")
+    buf[1:].copy_(st.view(torch.int16).flatten())
+    outs = []
+    for stack in (st, buf[1:].view(torch.uint16).view(frames, h, w)):
+        o = plan.alloc_device_outputs()
+        plan.execute(stack, o)
+        outs.append({k: v.cpu().numpy() for k, v in o.items()})
+    for k in outs[0]:
+        np.testing.assert_array_equal(outs[1][k], outs[0][k], err_msg=k)
