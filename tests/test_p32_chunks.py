@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 from imaging_fcs_1_52_gb300 import engine
-from tests.helpers import ACF_TOL, acf_deviation, run_both
+from tests.helpers import run_both
+from tests.helpers import ACF_TOL, acf_deviation
 from tests.synth import brownian_stack
 from tests.test_gpu_correlator import check_acf
 
